@@ -25,6 +25,9 @@
 #include <cfloat>
 #include <cstdint>
 
+#include <type_traits>
+
+#include "pair2.cuh"
 #include "sph_math.cuh"
 
 namespace ag {
@@ -55,6 +58,7 @@ struct DevGrid {
     int reach;       // stencil half-width in cells: cell size (2 max(h) + skin) / reach
     float half_skin2;  // (skin / 2)^2: a particle this far from its binned position forces a sort
     float skin;        // sort skin (length): neighbour lists hold pairs within h_i + h_j + skin
+    int huni;          // every particle has the same h (the passes' per-pair h terms are constants)
 };
 
 // A unit of work of the persistent passes: slots [s0, s1) of one instance.
@@ -265,6 +269,7 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__
     const int* __restrict__ resort = nullptr) {
     if (sort_skipped(resort)) return;
     float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, mh = 0.f;
+    float lh = FLT_MAX;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         float4 a = xh[i];
         mn[0] = fminf(mn[0], a.x);
@@ -276,6 +281,7 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__
             mx[2] = fmaxf(mx[2], a.z);
         }
         mh = fmaxf(mh, a.w);
+        lh = fminf(lh, a.w);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -285,8 +291,9 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__
             mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
         mh = fmaxf(mh, __shfl_xor_sync(0xffffffffu, mh, o));
+        lh = fminf(lh, __shfl_xor_sync(0xffffffffu, lh, o));
     }
-    __shared__ float s[8][7];
+    __shared__ float s[8][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         for (int d = 0; d < 3; ++d) {
@@ -294,13 +301,14 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__
             s[warp][3 + d] = mx[d];
         }
         s[warp][6] = mh;
+        s[warp][7] = lh;
     }
     __syncthreads();
-    if (threadIdx.x < 7) {
+    if (threadIdx.x < 8) {
         int k = threadIdx.x;
         float v = s[0][k];
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            v = (k < 3) ? fminf(v, s[w][k]) : fmaxf(v, s[w][k]);
+            v = (k < 3 || k == 7) ? fminf(v, s[w][k]) : fmaxf(v, s[w][k]);
         part[blockIdx.x * 8 + k] = v;
     }
 }
@@ -314,22 +322,22 @@ __global__ void __launch_bounds__(256) k_bbox_final(const float* __restrict__ pa
                                                     unsigned* __restrict__ flags,
     const int* __restrict__ resort = nullptr) {
     if (sort_skipped(resort)) return;
-    __shared__ float s[7][256];
-    float v[7] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f};
+    __shared__ float s[8][256];
+    float v[8] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f, FLT_MAX};
     for (int b = threadIdx.x; b < nparts; b += blockDim.x)
-        for (int k = 0; k < 7; ++k)
-            v[k] = (k < 3) ? fminf(v[k], part[b * 8 + k]) : fmaxf(v[k], part[b * 8 + k]);
-    for (int k = 0; k < 7; ++k) s[k][threadIdx.x] = v[k];
+        for (int k = 0; k < 8; ++k)
+            v[k] = (k < 3 || k == 7) ? fminf(v[k], part[b * 8 + k]) : fmaxf(v[k], part[b * 8 + k]);
+    for (int k = 0; k < 8; ++k) s[k][threadIdx.x] = v[k];
     __syncthreads();
     for (int st = blockDim.x / 2; st > 0; st >>= 1) {
         if ((int)threadIdx.x < st)
-            for (int k = 0; k < 7; ++k)
-                s[k][threadIdx.x] = (k < 3) ? fminf(s[k][threadIdx.x], s[k][threadIdx.x + st])
+            for (int k = 0; k < 8; ++k)
+                s[k][threadIdx.x] = (k < 3 || k == 7) ? fminf(s[k][threadIdx.x], s[k][threadIdx.x + st])
                                             : fmaxf(s[k][threadIdx.x], s[k][threadIdx.x + st]);
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    const float mm[7] = {s[0][0], s[1][0], s[2][0], s[3][0], s[4][0], s[5][0], s[6][0]};
+    const float mm[8] = {s[0][0], s[1][0], s[2][0], s[3][0], s[4][0], s[5][0], s[6][0], s[7][0]};
     unsigned fl = 0;
     DevGrid g = grid_from_bbox(mm, P, capacity, fl);
     *grid = g;
@@ -337,7 +345,7 @@ __global__ void __launch_bounds__(256) k_bbox_final(const float* __restrict__ pa
 }
 
 // The link_list grid (CERNsource/link_list.f:39-67) of a bbox mm = {min[3],
-// max[3], max h}, in FP32; periodic axes split their box into >= 3 cells.
+// max[3], max h, min h}, in FP32; periodic axes split their box into >= 3 cells.
 // With P.reach = f the cells are (2 mh + skin) / f wide, skin = P.skin * mh,
 // and the passes search (2f + 1)^dim cells. Unless f = 1 and skin = 0 (which
 // keep link_list's cell exactly) the cells are widened by a margin larger
@@ -401,6 +409,7 @@ __device__ __forceinline__ DevGrid grid_from_bbox(const float* mm, const DevPara
     g.reach = f;
     g.half_skin2 = 0.25f * skin * skin;
     g.skin = skin;
+    g.huni = mm[7] == mh ? 1 : 0;
     if (ncells > capacity || (fl & FLAG_GRID_OVERFLOW) || (fl & FLAG_PERIODIC_SMALL)) {
         fl |= (ncells > capacity) ? FLAG_GRID_OVERFLOW : 0u;
         g.ok = 0;
@@ -455,7 +464,8 @@ template <int DIM>
 __global__ void __launch_bounds__(256) k_bbox_partial_raw(const float* __restrict__ x,
                                                           const float* __restrict__ h, int n,
                                                           float* __restrict__ part) {
-    float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, mh = 0.f;
+    float mn[3] = {FLT_MAX, FLT_MAX, FLT_MAX}, mx[3] = {-FLT_MAX, -FLT_MAX, -FLT_MAX}, mh = 0.f,
+          lh = FLT_MAX;
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
 #pragma unroll
         for (int d = 0; d < DIM; ++d) {
@@ -464,6 +474,7 @@ __global__ void __launch_bounds__(256) k_bbox_partial_raw(const float* __restric
             mx[d] = fmaxf(mx[d], v);
         }
         mh = fmaxf(mh, h[i]);
+        lh = fminf(lh, h[i]);
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) {
@@ -473,8 +484,9 @@ __global__ void __launch_bounds__(256) k_bbox_partial_raw(const float* __restric
             mx[d] = fmaxf(mx[d], __shfl_xor_sync(0xffffffffu, mx[d], o));
         }
         mh = fmaxf(mh, __shfl_xor_sync(0xffffffffu, mh, o));
+        lh = fminf(lh, __shfl_xor_sync(0xffffffffu, lh, o));
     }
-    __shared__ float s[8][7];
+    __shared__ float s[8][8];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     if (lane == 0) {
         for (int d = 0; d < 3; ++d) {
@@ -482,13 +494,14 @@ __global__ void __launch_bounds__(256) k_bbox_partial_raw(const float* __restric
             s[warp][3 + d] = mx[d];
         }
         s[warp][6] = mh;
+        s[warp][7] = lh;
     }
     __syncthreads();
-    if (threadIdx.x < 7) {
+    if (threadIdx.x < 8) {
         int k = threadIdx.x;
         float v = s[0][k];
         for (int w = 1; w < (int)(blockDim.x >> 5); ++w)
-            v = (k < 3) ? fminf(v, s[w][k]) : fmaxf(v, s[w][k]);
+            v = (k < 3 || k == 7) ? fminf(v, s[w][k]) : fmaxf(v, s[w][k]);
         part[blockIdx.x * 8 + k] = v;
     }
 }
@@ -951,29 +964,29 @@ __global__ void __launch_bounds__(kPassThreads)
                  float* __restrict__ part) {
     const WorkItem w = items[blockIdx.x];
     const int s = w.s0 + threadIdx.x;
-    float v[7] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f};
+    float v[8] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f, FLT_MAX};
     if (s < w.s1) {
         const float4 a = xh[s];
         v[0] = v[3] = a.x;
         v[1] = v[4] = a.y;
         if (dim == 3) v[2] = v[5] = a.z;
-        v[6] = a.w;
+        v[6] = v[7] = a.w;
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int k = 0; k < 7; ++k) {
+        for (int k = 0; k < 8; ++k) {
             const float t = __shfl_xor_sync(0xffffffffu, v[k], o);
-            v[k] = (k < 3) ? fminf(v[k], t) : fmaxf(v[k], t);
+            v[k] = (k < 3 || k == 7) ? fminf(v[k], t) : fmaxf(v[k], t);
         }
-    __shared__ float sw[kPassThreads / 32][7];
+    __shared__ float sw[kPassThreads / 32][8];
     if ((threadIdx.x & 31) == 0)
-        for (int k = 0; k < 7; ++k) sw[threadIdx.x >> 5][k] = v[k];
+        for (int k = 0; k < 8; ++k) sw[threadIdx.x >> 5][k] = v[k];
     __syncthreads();
-    if (threadIdx.x < 7) {
+    if (threadIdx.x < 8) {
         const int k = threadIdx.x;
         float r = sw[0][k];
-        for (int w2 = 1; w2 < kPassThreads / 32; ++w2) r = (k < 3) ? fminf(r, sw[w2][k]) : fmaxf(r, sw[w2][k]);
+        for (int w2 = 1; w2 < kPassThreads / 32; ++w2) r = (k < 3 || k == 7) ? fminf(r, sw[w2][k]) : fmaxf(r, sw[w2][k]);
         part[blockIdx.x * 8 + k] = r;
     }
 }
@@ -983,23 +996,24 @@ __global__ void __launch_bounds__(256)
     k_bbox_final_batch(const float* __restrict__ part, const int* __restrict__ inst_items,
                        const DevParams* __restrict__ params, DevGrid* __restrict__ grids,
                        int* __restrict__ ncells_inst, unsigned* __restrict__ flags) {
-    __shared__ float sv[7][256];
+    __shared__ float sv[8][256];
     const int k = blockIdx.x;
-    float v[7] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f};
+    float v[8] = {FLT_MAX, FLT_MAX, FLT_MAX, -FLT_MAX, -FLT_MAX, -FLT_MAX, 0.f, FLT_MAX};
     for (int b = inst_items[k] + threadIdx.x; b < inst_items[k + 1]; b += blockDim.x)
-        for (int q = 0; q < 7; ++q)
-            v[q] = (q < 3) ? fminf(v[q], part[b * 8 + q]) : fmaxf(v[q], part[b * 8 + q]);
-    for (int q = 0; q < 7; ++q) sv[q][threadIdx.x] = v[q];
+        for (int q = 0; q < 8; ++q)
+            v[q] = (q < 3 || q == 7) ? fminf(v[q], part[b * 8 + q]) : fmaxf(v[q], part[b * 8 + q]);
+    for (int q = 0; q < 8; ++q) sv[q][threadIdx.x] = v[q];
     __syncthreads();
     for (int st = blockDim.x / 2; st > 0; st >>= 1) {
         if ((int)threadIdx.x < st)
-            for (int q = 0; q < 7; ++q)
-                sv[q][threadIdx.x] = (q < 3) ? fminf(sv[q][threadIdx.x], sv[q][threadIdx.x + st])
+            for (int q = 0; q < 8; ++q)
+                sv[q][threadIdx.x] = (q < 3 || q == 7) ? fminf(sv[q][threadIdx.x], sv[q][threadIdx.x + st])
                                              : fmaxf(sv[q][threadIdx.x], sv[q][threadIdx.x + st]);
         __syncthreads();
     }
     if (threadIdx.x != 0) return;
-    const float mm[7] = {sv[0][0], sv[1][0], sv[2][0], sv[3][0], sv[4][0], sv[5][0], sv[6][0]};
+    const float mm[8] = {sv[0][0], sv[1][0], sv[2][0], sv[3][0],
+                         sv[4][0], sv[5][0], sv[6][0], sv[7][0]};
     unsigned fl = 0;
     DevGrid g = grid_from_bbox(mm, params[k], (long long)1 << 30, fl);
     grids[k] = g;
@@ -1171,6 +1185,23 @@ __device__ __forceinline__ void refine_periodic(const float4& xi, const float4& 
     for (int k = 0; k < DIM; ++k)
         if (g.periodic[k]) d[k] = __fadd_rn(dh[k], dl[k]);
     dr2 = sph::dist2_exact<DIM>(d);
+}
+
+// Minimum image of two differences x_i - x_a, x_i - x_b along axis k, for the force
+// passes: a difference that wraps is the exact one rounded once (exact_delta); one
+// that does not is already.
+__device__ __forceinline__ f2 min_image2(f2 d, float xi, float xa, float xb, const DevGrid& g, int k) {
+    if (fabsf(d.x) > g.half[k]) {
+        const sph::ff s = sph::two_diff(xi, xa);
+        const sph::ff u = sph::two_sum(s.hi, s.hi > 0.f ? -g.L[k] : g.L[k]);
+        d.x = __fadd_rn(u.hi, __fadd_rn(s.lo, u.lo));
+    }
+    if (fabsf(d.y) > g.half[k]) {
+        const sph::ff s = sph::two_diff(xi, xb);
+        const sph::ff u = sph::two_sum(s.hi, s.hi > 0.f ? -g.L[k] : g.L[k]);
+        d.y = __fadd_rn(u.hi, __fadd_rn(s.lo, u.lo));
+    }
+    return d;
 }
 
 template <int DIM>
@@ -1974,9 +2005,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         }
     }
     const bool work = valid && it > 0 && g.ok;
-    CellCoord cc = {{0, 0, 0}};
-    if (work) cc = decode_key<DIM>(keys[s], g);
-    const float ihf = __fdividef(1.0f, xi.w);
+    const float ihf = __frcp_rn(xi.w);
     const float kgih_i = P.kg * pow_grad<DIM>(ihf);
     float4 ti = make_float4(0.f, 0.f, 0.f, 0.f), ti2 = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool visc = !LEAN && P.visc, heat_art = !LEAN && P.heat_art;
@@ -1985,199 +2014,210 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         if (DIM == 3) ti2 = B.tau2[s];
     }
     const float ulo_i = (work && heat_art) ? B.ulo[s] : 0.f;
-    float a0 = 0.f, a1 = 0.f, a2 = 0.f, he_sum = 0.f, av_du = 0.f, ah_du = 0.f;
+    // Pair sums in the order of the walk (an entry beyond the support adds a zero,
+    // so lists and cell walks in the same order sum alike): acceleration, twice
+    // the pressure and art_visc energy rate, art_heat's.
+    const f2 zero2 = bc2(0.f);
+    float a0 = 0.f, a1 = 0.f, a2 = 0.f, e_sum = 0.f, ah_du = 0.f;
     // single_step options: continuity drho/dt, XSPH velocity, div v for h
     const bool cont = OPT && P.density_form == 1, xsph = OPT && P.xsph, sle2 = OPT && P.sle == 2;
     float drho_s = 0.f, divh = 0.f, x0s = 0.f, x1s = 0.f, x2s = 0.f;
-    constexpr int W = mask_words<DIM>() / TPP;  // mask words of this lane
-    const size_t mlane = (size_t)s * TPP + sub;
-    Cursor cu = cursor_begin<DIM>(g);
     bool done = !work;
-    // The density pass left the neighbour bits of the candidates (word-major).
-    constexpr int CW = mask_chunk<W>();
-    bool from_mask = false;
-    uint4 ch = make_uint4(0u, 0u, 0u, 0u);  // mask chunk being decoded
-    unsigned wbits = 0u;                    // bits left of word wi
-    // A listed particle walks its neighbour list (coalesced rows of entries)
-    // and re-tests each entry; the others decode the density pass's bits.
+    // A listed particle walks its neighbour list (coalesced rows of entries);
+    // the others decode the density pass's bits.
     const int lpk = (LST && work) ? __ldg(B.ncount + s) : -1;
     const int lc = lpk >= 0 ? list_near(lpk) + list_far(lpk) : -1;  // entries (-1: no list)
     if (LST) prefetch_list_rows(B.nlist, B.lstride, s, lc);
-    if (work && !(LST && lc >= 0)) {
+    // The place of an absent entry (the odd end of a list, a lane without
+    // entries): the particle itself, whose terms vanish with d = 0 and dv = 0.
+    int kself = valid ? s : 0;
+    if (STG) kself = work ? s + SV.shift[DIM == 2 ? g.reach : g.reach * (2 * g.reach + 2)] : 0;
+    const float k_alpha = P.visc_art ? P.av_alpha * P.c0 : 0.f;        // times h_i + h_j
+    const float k_beta = P.visc_art ? 0.5f * P.av_beta : 0.f;          // times (h_i + h_j)^2
+    // Push between particles of different type (ArmandoThrust/armando.cu:507-513
+    // for wall_model 1, acpu.c:424-429 for 2) along (x_i - x_j)/r, c = c0; with
+    // wall_model 1 the pair's only interaction (its mass is zeroed).
+    auto push = [&](const int k, const float4& xj, float rhoj, float e0, float e1, float e2, float dr2,
+                    float tt, float t, float ih, float& mj, float& p0, float& p1, float& p2) {
+        if (__ldg(B.itype + k) == it) return;
+        const float r = fast_sqrt_pos(dr2);
+        if (dr2 > 2.0f * kTinyDr2) {
+            const float w = 0.0625f * tt * tt * fmaf(2.0f, t, 5.0f);  // W / W(0)
+            const float c2 = P.c0 * P.c0;
+            float f;
+            if (P.wall_model == 1) {
+                const float alpha = P.kw_hi * (DIM == 2 ? ih * ih : ih * ih * ih);
+                f = 0.5f * alpha * w * mj / (rhoj * xj.w) * c2;
+            } else {
+                f = 0.02f * w * c2 / r * mj / (mass_of<DIM>(xi, vi) + mj);
+            }
+            f /= r;
+            p0 = fmaf(f, e0, p0);
+            p1 = fmaf(f, e1, p1);
+            if (DIM == 3) p2 = fmaf(f, e2, p2);
+        }
+        if (P.wall_model == 1) mj = 0.f;
+    };
+    // Terms of two entries (pressure, viscosity, art_visc, art_heat, options).
+    // va, vb: the neighbours' 2D {vx, vy, rho, P} (ra, rb unused) or 3D v and
+    // {rho, P, u, psi}. No pair test: the kernel's gradient is zero beyond its
+    // support, so the entries in the skin margin add nothing.
+    //
+    // Pressure, art_visc and their energy rates share one factor per pair: with
+    // s = m_j G (grad W = G d), T = P_i + P_j + Pi_ij and dv = v_j - v_i,
+    //   a_i -= s T d,   du_i -= s T (dv.d) / 2
+    // (internal_force.f:179-428 and art_visc.f:71-100 summed), G = kg (q - 2)^3.
+    // art_visc: Pi_ij = alpha c0 A + beta rho_bar A^2, A = mh (dv.d)+ / (rho_bar
+    // (r^2 + (eta mh)^2)): one reciprocal, of rho_bar's and the distance's product,
+    // serves both of its divisions, and (dv.d)+ = max(dv.d, 0) its condition.
+    // The pass was bound by issue (62% of cycles) and its neighbours' loads: about 80
+    // instructions an entry, 50 now. Measured: 2D lists (2.03 M dam break) 0.213 ->
+    // 0.160 ms, 3D lists (8.78 M channel) 6.77 -> 4.41 ms, 2D cells (42 k) 17.6 -> 16.1 us.
+    // UNI: every particle has the same h (g.huni), whose factors are constants.
+    // PH: the physics beyond pressure and art_visc compiled in, bits 1 art_heat,
+    // 2 physical viscosity, 4 repulsive walls and the single_step options.
+    auto pair2 = [&](auto uni, auto ph, const int ka, const int kb, const float4& xa, const float4& xb,
+                     const float4& va, const float4& vb, const float4& ra, const float4& rb) {
+        constexpr bool UNI = decltype(uni)::value;
+        constexpr int PH = decltype(ph)::value;
+        f2 d0 = make_float2(xi.x - xa.x, xi.x - xb.x), d1 = make_float2(xi.y - xa.y, xi.y - xb.y);
+        f2 d2 = DIM == 3 ? make_float2(xi.z - xa.z, xi.z - xb.z) : zero2;
+        if (g.periodic[0]) d0 = min_image2(d0, xi.x, xa.x, xb.x, g, 0);
+        if (g.periodic[1]) d1 = min_image2(d1, xi.y, xa.y, xb.y, g, 1);
+        if (DIM == 3 && g.periodic[2]) d2 = min_image2(d2, xi.z, xa.z, xb.z, g, 2);
+        f2 dr2 = fma2(d1, d1, fma2(d0, d0, bc2(kTinyDr2)));
+        if (DIM == 3) dr2 = fma2(d2, d2, dr2);
+        f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
+        f2 ih = bc2(ihf), kg = bc2(kgih_i), hs = bc2(2.0f * xi.w);
+        if (!UNI) {
+            hs = make_float2(xi.w + xa.w, xi.w + xb.w);
+            ih = mul2(bc2(2.0f), rcp2(hs));
+            const f2 ih2 = mul2(ih, ih);
+            kg = mul2(bc2(P.kg), mul2(ih2, ih2));
+            if (DIM == 3) kg = mul2(kg, ih);
+        }
+        const f2 r = mul2(dr2, rsqrt2(dr2));
+        const f2 t = min2(fma2(r, ih, bc2(-2.0f)), 0.0f);  // q - 2, 0 beyond the support
+        const f2 tt = mul2(t, t);
+        const f2 rhoj = DIM == 2 ? make_float2(va.z, vb.z) : make_float2(ra.x, rb.x);
+        if ((PH & 4) && repulsive_walls(P)) {
+            push(ka, xa, rhoj.x, d0.x, d1.x, d2.x, dr2.x, tt.x, t.x, ih.x, mj.x, a0, a1, a2);
+            push(kb, xb, rhoj.y, d0.y, d1.y, d2.y, dr2.y, tt.y, t.y, ih.y, mj.y, a0, a1, a2);
+        }
+        const f2 sm = mul2(mul2(tt, t), mul2(mj, kg));
+        const f2 vx = make_float2(va.x - vi.x, vb.x - vi.x), vy = make_float2(va.y - vi.y, vb.y - vi.y);
+        const f2 vz = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : zero2;
+        f2 vr = fma2(vy, d1, mul2(vx, d0));
+        if (DIM == 3) vr = fma2(vz, d2, vr);
+        const f2 rs = make_float2(rpi.x + rhoj.x, rpi.x + rhoj.y);
+        f2 T = DIM == 2 ? make_float2(rpi.y + va.w, rpi.y + vb.w) : make_float2(rpi.y + ra.y, rpi.y + rb.y);
+        f2 sv = sm;  // the viscous terms' factor
+        if (P.pa_sph != 1) {
+            const f2 irr = rcp2(mul2(bc2(rpi.x), rhoj));
+            T = mul2(T, irr);
+            sv = mul2(sv, irr);
+        }
+        const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
+        const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
+                         : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);
+        const f2 rc = rcp2(mul2(D, rs));
+        const f2 A = mul2(max2(vr, 0.0f), rc);
+        T = fma2(A, UNI ? bc2(k_alpha * (2.0f * xi.w)) : mul2(bc2(k_alpha), hs), T);
+        if (k_beta != 0.f) T = fma2(mul2(mul2(A, A), rs), mul2(bc2(k_beta), hs2), T);
+        const f2 c = neg2(mul2(sm, T));
+        a0 = dot2(c, d0, a0);
+        a1 = dot2(c, d1, a1);
+        if (DIM == 3) a2 = dot2(c, d2, a2);
+        e_sum = dot2(c, vr, e_sum);
+        if (cont) drho_s = dot2(neg2(sm), vr, drho_s);  // con_density, density.f:203-216
+        if (sle2) {                                   // hsml.f:75-90
+            divh = fmaf(__fdiv_rn(sm.x, rhoj.x), vr.x, divh);
+            divh = fmaf(__fdiv_rn(sm.y, rhoj.y), vr.y, divh);
+        }
+        if (xsph) {  // av_vel.f:47-58: -eps m_j / rho_ij (v_i - v_j) W_ij, eps = 0.3
+            const f2 ih2 = mul2(ih, ih);
+            // W = kw ih^dim (q - 2)^4 (2 (q - 2) + 5) / 16; 1 / rho_bar = 2 D rc
+            f2 wv = mul2(mul2(mul2(tt, tt), fma2(bc2(2.0f), t, bc2(5.0f))), mul2(bc2(0.0625f * P.kw_hi), ih2));
+            if (DIM == 3) wv = mul2(wv, ih);
+            const f2 cx = mul2(mul2(mul2(bc2(0.6f), mj), wv), mul2(D, rc));
+            x0s = dot2(cx, vx, x0s);
+            x1s = dot2(cx, vy, x1s);
+            if (DIM == 3) x2s = dot2(cx, vz, x2s);
+        }
+        if ((PH & 2) && visc) {
+            const float4 qa = __ldg(B.tau + ka), qb = __ldg(B.tau + kb);
+            const f2 sxx = make_float2(ti.x + qa.x, ti.x + qb.x), syy = make_float2(ti.y + qa.y, ti.y + qb.y);
+            const f2 sxy = make_float2(ti.z + qa.z, ti.z + qb.z);
+            f2 h0 = fma2(sxy, d1, mul2(sxx, d0)), h1 = fma2(syy, d1, mul2(sxy, d0));
+            if (DIM == 3) {
+                const float4 ua = __ldg(B.tau2 + ka), ub = __ldg(B.tau2 + kb);
+                const f2 szz = make_float2(ti.w + qa.w, ti.w + qb.w);
+                const f2 sxz = make_float2(ti2.x + ua.x, ti2.x + ub.x), syz = make_float2(ti2.y + ua.y, ti2.y + ub.y);
+                h0 = fma2(sxz, d2, h0);
+                h1 = fma2(syz, d2, h1);
+                a2 = dot2(sv, fma2(szz, d2, fma2(syz, d1, mul2(sxz, d0))), a2);
+            }
+            a0 = dot2(sv, h0, a0);
+            a1 = dot2(sv, h1, a1);
+        }
+        if ((PH & 1) && heat_art) {  // art_heat.f:69-97: grad W . d = G r^2
+            f2 rh = rc;
+            if (P.ah_eta2 != P.av_eta2)
+                rh = rcp2(mul2(fma2(hs2, bc2(0.25f * P.ah_eta2), dr2), rs));
+            float4 qa = ra, qb = rb;
+            if (DIM == 2) {  // u and psi are not in the 2D record
+                qa = __ldg(B.rp + ka);
+                qb = __ldg(B.rp + kb);
+            }
+            const f2 ps = make_float2(rpi.w + qa.w, rpi.w + qb.w);
+            const f2 lo = make_float2(ulo_i - __ldg(B.ulo + ka), ulo_i - __ldg(B.ulo + kb));
+            const f2 du2 = add2(make_float2(rpi.z - qa.z, rpi.z - qb.z), lo);
+            ah_du = dot2(mul2(mul2(mul2(sm, dr2), mul2(ps, rh)), bc2(2.0f)), du2, ah_du);
+        }
+    };
+    // The entries, two at a time, with every particle's h alike or not.
+    auto walk = [&](auto uni, auto ph) {
+    // A listed particle takes each entry's terms as the entry is read, without
+    // a candidate list; the mask decoding and cell walk below serve the others.
+    if (LST) {
+        constexpr int NB = list_batch<DIM>();
+        const int lcm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
+        for (int t0 = 0; t0 < lcm; t0 += NB) {
+            int kb[NB];
+            float4 xb[NB], va[NB], rb[NB];
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                kb[u] = t0 + u < lc ? __ldg(B.nlist + (size_t)(t0 + u) * B.lstride + s) : kself;
+#pragma unroll
+            for (int u = 0; u < NB; ++u) {
+                xb[u] = __ldg(xsrc + kb[u]);
+                va[u] = __ldg((DIM == 2 ? B.vr : B.vm) + kb[u]);
+                rb[u] = DIM == 3 ? __ldg(B.rp + kb[u]) : va[u];
+            }
+#pragma unroll
+            for (int u = 0; u < NB; u += 2)
+                pair2(uni, ph, kb[u], kb[u + 1], xb[u], xb[u + 1], va[u], va[u + 1], rb[u], rb[u + 1]);
+        }
+        if (lc >= 0) done = true;
+    }
+    if (!__any_sync(0xffffffffu, !done)) return;
+    constexpr int W = mask_words<DIM>() / TPP;  // mask words of this lane
+    constexpr int CW = mask_chunk<W>();
+    const size_t mlane = (size_t)s * TPP + sub;
+    CellCoord cc = {{0, 0, 0}};
+    Cursor cu = cursor_begin<DIM>(g);
+    // The density pass left the neighbour bits of the candidates (word-major).
+    bool from_mask = false;
+    uint4 ch = make_uint4(0u, 0u, 0u, 0u);  // mask chunk being decoded
+    unsigned wbits = 0u;                    // bits left of word wi
+    if (!done) {
+        cc = decode_key<DIM>(keys[s], g);
         ch = mask_load_chunk<W>(B.nmask, B.mstride, mlane, 0);
         wbits = ch.x;
         from_mask = !(ch.x == ~0u && (W == 1 || ch.y == ~0u));
     }
     int wi = 0, rbase = 0;  // index of wbits; ordinal of the cursor row's first slot
     int shift = 0;          // staged index - slot in the cursor's row
-    // One pair's terms (pressure, viscosity, art_visc, art_heat, options).
-    // va, vb: the neighbour's 2D {vx, vy, rho, P} (vb unused) or 3D v and
-    // {rho, P, u, psi}; d, dr2 from the pair test.
-    auto pair_terms = [&](const int k, const float4& xj, const float4& va, const float4& vb,
-                          float* d, float dr2) {
-            float4 vj, rpj;
-            if (DIM == 2) {  // u and psi only for art_heat
-                vj = make_float4(va.x, va.y, 0.f, 0.f);
-                rpj = make_float4(va.z, va.w, 0.f, 0.f);
-                if (heat_art) {
-                    const float4 r = __ldg(B.rp + k);
-                    rpj.z = r.z;
-                    rpj.w = r.w;
-                }
-            } else {
-                vj = va;
-                rpj = vb;
-            }
-            refine_periodic<DIM>(xi, xj, g, d, dr2);
-            const float mj = mass_of<DIM>(xj, vj);
-            float ih = ihf, kgih = kgih_i;
-            if (xj.w != xi.w) {
-                ih = __fdividef(2.0f, xi.w + xj.w);
-                kgih = P.kg * pow_grad<DIM>(ih);
-            }
-            const float q = __fmul_rn(fast_sqrt_pos(dr2), ih);
-            if (!LEAN && repulsive_walls(P) && __ldg(B.itype + k) != it) {
-                // Push between particles of different type (ArmandoThrust/armando.cu:507-513
-                // for wall_model 1, acpu.c:424-429 for 2) along (x_i - x_j)/r, c = c0.
-                const float r = fast_sqrt_pos(dr2);
-                if (r > 0.f) {
-                    float tt = fmaf(-0.5f, q, 1.0f);
-                    tt = tt * tt;
-                    tt = tt * tt;
-                    tt *= fmaf(2.0f, q, 1.0f);  // W / W(0)
-                    const float c2 = P.c0 * P.c0;
-                    float f;
-                    if (P.wall_model == 1) {
-                        const float alpha = P.kw_hi * (DIM == 2 ? ih * ih : ih * ih * ih);
-                        f = 0.5f * alpha * tt * mj / (rpj.x * xj.w) * c2;
-                    } else {
-                        f = 0.02f * tt * c2 / r * mj / (mass_of<DIM>(xi, vi) + mj);
-                    }
-                    f /= r;
-                    a0 = fmaf(f, d[0], a0);
-                    a1 = fmaf(f, d[1], a1);
-                    if (DIM == 3) a2 = fmaf(f, d[2], a2);
-                }
-                if (P.wall_model == 1) return;  // no other interaction
-            }
-            const float t3 = q - 2.0f;
-            const float gw = kgih * t3 * t3 * t3;
-            const float w0 = gw * d[0], w1 = gw * d[1], w2 = (DIM == 3) ? gw * d[2] : 0.f;
-            const float vx = vj.x - vi.x, vy = vj.y - vi.y, vz = (DIM == 3) ? vj.z - vi.z : 0.f;
-            if (cont || sle2) {  // (v_j - v_i) . grad_i W
-                float vdw = fmaf(vy, w1, __fmul_rn(vx, w0));
-                if (DIM == 3) vdw = fmaf(vz, w2, vdw);
-                if (cont) drho_s = fmaf(-mj, vdw, drho_s);  // con_density, density.f:203-216
-                if (sle2) divh = fmaf(__fdiv_rn(mj, rpj.x), vdw, divh);  // hsml.f:75-90
-            }
-            if (xsph) {  // av_vel.f:47-58: -eps m_j / rho_ij (v_i - v_j) W_ij, eps = 0.3
-                float tt = fmaf(-0.5f, q, 1.0f);
-                tt = tt * tt;
-                tt = tt * tt;
-                const float wv = P.kw_hi * (DIM == 2 ? ih * ih : ih * ih * ih) * tt * fmaf(2.0f, q, 1.0f);
-                const float c = __fdiv_rn(0.3f * mj * wv, 0.5f * (rpi.x + rpj.x));
-                x0s = fmaf(c, vx, x0s);
-                x1s = fmaf(c, vy, x1s);
-                if (DIM == 3) x2s = fmaf(c, vz, x2s);
-            }
-            // Pressure (internal_force.f:309-428 for pa_sph 1, 179-306 for pa_sph 0).
-            const float fs = -(rpi.y + rpj.y);
-            // Products that feed a sum are written out (fmaf / __fmul_rn) so that
-            // every instantiation of this body rounds alike (no free contraction).
-            float h0 = fs * w0, h1 = fs * w1, h2 = fs * w2;
-            float he = fmaf(vy, h1, __fmul_rn(vx, h0));
-            if (DIM == 3) he = fmaf(vz, h2, he);
-            if (visc) {
-                const float4 tj = __ldg(B.tau + k);
-                float4 tj2 = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (DIM == 3) tj2 = __ldg(B.tau2 + k);
-                const float sxx = ti.x + tj.x, syy = ti.y + tj.y, sxy = ti.z + tj.z;
-                if (DIM == 2) {
-                    h0 = fmaf(sxy, w1, fmaf(sxx, w0, h0));
-                    h1 = fmaf(syy, w1, fmaf(sxy, w0, h1));
-                } else {
-                    const float szz = ti.w + tj.w, sxz = ti2.x + tj2.x, syz = ti2.y + tj2.y;
-                    h0 = fmaf(sxz, w2, fmaf(sxy, w1, fmaf(sxx, w0, h0)));
-                    h1 = fmaf(syz, w2, fmaf(syy, w1, fmaf(sxy, w0, h1)));
-                    h2 = fmaf(szz, w2, fmaf(syz, w1, fmaf(sxz, w0, h2)));
-                }
-            }
-            if (P.pa_sph != 1) {
-                const float inv_rr = __fdividef(1.0f, rpi.x * rpj.x);
-                h0 *= inv_rr;
-                h1 *= inv_rr;
-                h2 *= inv_rr;
-                he *= inv_rr;
-            }
-            a0 = fmaf(mj, h0, a0);
-            a1 = fmaf(mj, h1, a1);
-            if (DIM == 3) a2 = fmaf(mj, h2, a2);
-            he_sum = fmaf(mj, he, he_sum);
-            const float mh = 0.5f * (xi.w + xj.w);
-            const float rho_bar = 0.5f * (rpi.x + rpj.x);
-            // art_visc.f:71-100.
-            if (P.visc_art) {
-                float vr = fmaf(vy, d[1], __fmul_rn(vx, d[0]));
-                if (DIM == 3) vr = fmaf(vz, d[2], vr);
-                if (vr > 0.f) {  // (v_i - v_j) . (x_i - x_j) = -vr < 0
-                    const float phi = __fdividef(-mh * vr, fmaf(__fmul_rn(mh, mh), P.av_eta2, dr2));
-                    const float piv = __fdividef(
-                        fmaf(P.av_beta, phi, -__fmul_rn(P.av_alpha, P.c0)) * phi, rho_bar);
-                    const float mp = mj * piv;
-                    a0 = fmaf(-mp, w0, a0);
-                    a1 = fmaf(-mp, w1, a1);
-                    if (DIM == 3) a2 = fmaf(-mp, w2, a2);
-                    float vdw = fmaf(vy, w1, __fmul_rn(vx, w0));
-                    if (DIM == 3) vdw = fmaf(vz, w2, vdw);
-                    av_du = fmaf(-0.5f * mp, vdw, av_du);
-                }
-            }
-            // art_heat.f:69-97.
-            if (heat_art) {
-                float rdw = fmaf(d[1], w1, __fmul_rn(d[0], w0));
-                if (DIM == 3) rdw = fmaf(d[2], w2, rdw);
-                const float psi = __fdividef(
-                    rpi.w + rpj.w, rho_bar * fmaf(__fmul_rn(mh, mh), P.ah_eta2, dr2)) * rdw;
-                const float du_ij = (rpi.z - rpj.z) + (ulo_i - __ldg(B.ulo + k));
-                ah_du = fmaf(mj * psi, du_ij, ah_du);
-            }
-    };
-    // A listed particle takes each entry's terms as the entry is read and
-    // passes the pair test, without a candidate list; the mask decoding and
-    // cell walk below serve the others.
-    if (LST) {
-        constexpr int NB = list_batch<DIM>();
-        const int lcm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
-        // (a lane past the last slot reads slot 0: its loads stay in bounds)
-        auto entry = [&](int t) {
-            return lc > 0 ? __ldg(B.nlist + (size_t)min(t, lc - 1) * B.lstride + s) : (valid ? s : 0);
-        };
-        for (int t0 = 0; t0 < lcm; t0 += NB) {
-            int kb[NB];
-            float4 xb[NB];
-#pragma unroll
-            for (int u = 0; u < NB; ++u) kb[u] = entry(t0 + u);
-            // 2D: the neighbours' {vx, vy, rho, P} load with their positions; 3D
-            // loads v and {rho, P} once the pair test passed (registers).
-            float4 vr[NB];
-#pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                xb[u] = __ldg(xsrc + kb[u]);
-                if (DIM == 2) vr[u] = __ldg(B.vr + kb[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                float d[3], dr2;
-                if (t0 + u < lc && kb[u] != s && pair_delta<DIM>(xi, xb[u], g, d, dr2)) {
-                    if (DIM == 2)
-                        pair_terms(kb[u], xb[u], vr[u], vr[u], d, dr2);
-                    else
-                        pair_terms(kb[u], xb[u], __ldg(B.vm + kb[u]), __ldg(B.rp + kb[u]), d, dr2);
-                }
-            }
-        }
-        if (lc >= 0) done = true;
-    }
     while (__any_sync(0xffffffffu, !done)) {
         int nl = 0;
         while (!done && from_mask) {
@@ -2243,28 +2283,36 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             }
         }
         const int ml = __reduce_max_sync(0xffffffffu, nl);
-        for (int t = 0; t < ml; ++t) {
-            if (t >= nl) continue;
-            const int k = (int)s_list[t][tid];
-            const float4 xj = STG ? SV.x[k] : __ldg(xsrc + k);
-            float4 va, vb = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (DIM == 2) {
-                va = STG ? SV.v[k] : __ldg(B.vr + k);
-            } else {
-                va = STG ? SV.v[k] : __ldg(B.vm + k);
-                vb = STG ? SV.r[k] : __ldg(B.rp + k);
+        for (int t = 0; t < ml; t += 2) {
+            int kb[2];
+            float4 xb[2], va[2], rb[2];
+#pragma unroll
+            for (int u = 0; u < 2; ++u) {
+                const int k = kb[u] = t + u < nl ? (int)s_list[t + u][tid] : kself;
+                xb[u] = STG ? SV.x[k] : __ldg(xsrc + k);
+                va[u] = STG ? SV.v[k] : __ldg((DIM == 2 ? B.vr : B.vm) + k);
+                rb[u] = DIM == 2 ? va[u] : STG ? SV.r[k] : __ldg(B.rp + k);
             }
-            float d[3], dr2;
-            pair_delta<DIM>(xi, xj, g, d, dr2);
-            pair_terms(k, xj, va, vb, d, dr2);
+            pair2(uni, ph, kb[0], kb[1], xb[0], xb[1], va[0], va[1], rb[0], rb[1]);
         }
+    }
+    };
+    using std::integral_constant;
+    if constexpr (LEAN) {
+        if (TPP == 1 && g.huni) walk(std::true_type{}, integral_constant<int, 0>{});
+        else walk(std::false_type{}, integral_constant<int, 0>{});
+    } else if constexpr (TPP == 1 && !OPT) {
+        if (g.huni && !repulsive_walls(P) && !P.visc) walk(std::true_type{}, integral_constant<int, 1>{});
+        else if (g.huni && !repulsive_walls(P) && !P.heat_art) walk(std::true_type{}, integral_constant<int, 2>{});
+        else walk(std::false_type{}, integral_constant<int, 7>{});
+    } else {
+        walk(std::false_type{}, integral_constant<int, 7>{});
     }
     if (TPP > 1) {  // the particle's lanes reach this point together
         a0 = group_sum<TPP>(a0);
         a1 = group_sum<TPP>(a1);
         if (DIM == 3) a2 = group_sum<TPP>(a2);
-        he_sum = group_sum<TPP>(he_sum);
-        av_du = group_sum<TPP>(av_du);
+        e_sum = group_sum<TPP>(e_sum);
         ah_du = group_sum<TPP>(ah_du);
         if (cont) drho_s = group_sum<TPP>(drho_s);
         if (sle2) divh = group_sum<TPP>(divh);
@@ -2275,7 +2323,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         }
     }
     if (!work || sub != 0) return;
-    float du = __fadd_rn(fmaf(0.5f, he_sum, av_du), ah_du);  // internal_force.f:433-435
+    float du = fmaf(0.5f, e_sum, ah_du);  // internal_force.f:433-435
     if (visc) du += B.tds[s];
     if (S.heat_on) {
         float e0 = xi.x - P.heat_center[0], e1 = xi.y - P.heat_center[1];
@@ -2447,7 +2495,10 @@ __global__ void __launch_bounds__(kPassThreads)
 
 template <int DIM, int TPP, int BS, bool PER, bool LEAN, bool OPT = false, bool LST = false,
           bool FUS = false>
-__global__ void __launch_bounds__(BS, 1024 / BS)
+__global__ void
+    // 64 registers for the lean physics; the others spill there: 80 (six CTAs of 128)
+    // take the 3D channel from 4.82 to 4.41 ms, XSPH + normalised density 61 to 40 us
+    __launch_bounds__(BS, (LEAN ? 1024 : 768) / BS)
     k_force(StateB B, StateA A, const unsigned* __restrict__ keys, const int* __restrict__ start,
             const DevGrid* __restrict__ gp, DevParams P, StepArgs S, unsigned* __restrict__ flags,
             int n, FusedSrc F) {
