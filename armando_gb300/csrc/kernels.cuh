@@ -58,6 +58,7 @@ struct DevGrid {
     int reach;       // stencil half-width in cells: cell size (2 max(h) + skin) / reach
     float half_skin2;  // (skin / 2)^2: a particle this far from its binned position forces a sort
     float skin;        // sort skin (length): neighbour lists hold pairs within h_i + h_j + skin
+    float hmax;        // largest h
     int huni;          // every particle has the same h (the passes' per-pair h terms are constants)
 };
 
@@ -409,6 +410,7 @@ __device__ __forceinline__ DevGrid grid_from_bbox(const float* mm, const DevPara
     g.reach = f;
     g.half_skin2 = 0.25f * skin * skin;
     g.skin = skin;
+    g.hmax = mh;
     g.huni = mm[7] == mh ? 1 : 0;
     if (ncells > capacity || (fl & FLAG_GRID_OVERFLOW) || (fl & FLAG_PERIODIC_SMALL)) {
         fl |= (ncells > capacity) ? FLAG_GRID_OVERFLOW : 0u;
@@ -1167,6 +1169,7 @@ __device__ __forceinline__ void exact_delta(const float4& xi, const float4& xj, 
                 s.hi = u.hi;
                 s.lo = __fadd_rn(s.lo, u.lo);
             }
+            s = sph::two_sum(s.hi, s.lo);  // a wrapped difference's residual may exceed an ulp
         }
         dh[k] = s.hi;
         dl[k] = s.lo;
@@ -1510,176 +1513,215 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
         vi = B.vm[s];
     }
     const bool work = valid && g.ok && (fluid || need_div);
-    CellCoord cc = {{0, 0, 0}};
-    if (work) cc = decode_key<DIM>(keys[s], g);
     const sph::ff kw = {P.kw_hi, P.kw_lo};
     const sph::ff ih_i = sph::ff_recip(xi.w);
     const sph::ff al_i = sph::ff_mul(kw, ff_pow_dim<DIM>(ih_i));
     const float mi = mass_of<DIM>(xi, vi);
-    // Self density m_i W(0, h_i) (density.f:39-42), on the particle's first lane.
-    sph::ff S = sph::ff_mul_f(al_i, mi);
+    const float kgih_i = __fmul_rn(P.kg, pow_grad<DIM>(ih_i.hi));
     // Normalised summation (nor_density, density.f:65-158): the denominator
     // m_i W(0)/rho_i + sum_j m_j/rho_j W_ij on the start densities, float-float.
     const bool nor = OPT && P.density_form == 2 && fluid;
-    sph::ff Wn = sph::ff{0.f, 0.f};
-    if (nor) Wn = sph::ff_mul(S, sph::ff_recip(B.q[s]));
-    if (sub != 0) S = Wn = sph::ff{0.f, 0.f};
-    const float ihf = ih_i.hi;
-    const float kgih_i = __fmul_rn(P.kg, pow_grad<DIM>(ihf));
+    // Density sums of the even (.x) and odd (.y) entries, float-float: of m_j W_ij,
+    // or with every h alike (UNI) of m_j W_ij h^dim / K, the factor applied once to
+    // the sum. The self term (density.f:39-42) opens the first lane's even one.
+    f2 Sh = bc2(0.f), Sl = bc2(0.f);
+    f2 Wh = bc2(0.f), Wl = bc2(0.f);  // the normalised summation's denominator, alike
     float divs = 0.f;
-    constexpr int W = mask_words<DIM>() / TPP;  // mask words of this lane
-    const size_t mlane = (size_t)s * TPP + sub;
-    Cursor cu = cursor_begin<DIM>(g);
     bool done = !work;
-    // (listed particles, LST, need no bits: the force pass re-tests their list)
-    bool mask_on = work && fluid;
-    int ord = 0;  // candidate ordinal (cursor order, self included)
-    int wb = 0;   // the accumulator holds the bits of ordinals 32 wb .. 32 wb + 63
-    unsigned long long cur = 0ull;
-    int shift = 0;  // staged index - slot in the cursor's row
+    // Differences x_i - x_j of near pairs are exact in FP32 unless the coordinates
+    // differ by more than a factor of two (near a coordinate's zero) or wrap: a
+    // particle farther than that from both skips the residuals. rmax: farther than
+    // any entry of a list (h_i + h_j + skin when built, each moved skin/2 since).
+    bool plain = true;
+    {
+        const float rmax = 1.01f * (xi.w + g.hmax + 2.0f * g.skin);
+        const float c[3] = {xi.x, xi.y, xi.z};
+#pragma unroll
+        for (int k = 0; k < DIM; ++k) {
+            plain = plain && fabsf(c[k]) >= 2.0f * rmax;
+            if (g.periodic[k]) plain = plain && c[k] - g.o[k] > rmax && g.o[k] + g.L[k] - c[k] > rmax;
+        }
+    }
+    // (listed particles, LST, need no bits: the force pass walks their list)
     const int lpk = (LST && work) ? __ldg(B.ncount + s) : -1;
     const int lc = list_near(lpk);  // near list entries (-1: walk the cells)
     const int lf = list_far(lpk);   // far list entries (2D)
-    if (LST && lc >= 0) mask_on = false;
     if (LST) prefetch_list_rows(B.nlist, B.lstride, s, lc + lf);
-    // A listed particle evaluates each list entry as it is read, the near
-    // ones in float-float, the far ones (2D) like the cell walk's far pairs;
-    // the kernel is zero beyond its support, so the entries need no pair
-    // test: no candidate lists in shared memory, no second load. The cell
-    // walk below serves the others.
+    // The place of an absent entry: the particle itself, with no mass.
+    int kself = valid ? s : 0;
+    if (STG) kself = work ? s + SV.shift[DIM == 2 ? g.reach : g.reach * (2 * g.reach + 2)] : 0;
+    // Two entries. NEAR: float-float weights on the exact pair difference, else
+    // (2D) FP32 weights, the pair's r and q rounded once. The kernel is zero beyond
+    // its support, so entries in a list's skin margin need no pair test.
+    // ka, kb: the entries; ina, inb: whether they are there; x, v: their {x, h} and
+    // v (3D: the mass; artificial heat).
+    // Issue-bound (72-89% of cycles): the packed forms take half the slots, and
+    // K/h^dim once per sum, Fast2Sum where the larger term is known and no residuals
+    // for `plain` particles save about 30 of 85 operations a near pair. Measured: 3D
+    // lists (8.78 M channel) 5.24 -> 3.45 ms, 2D lists (2.03 M dam break) 0.179 ->
+    // 0.154 ms, 2D cells (42 k) 21.6 -> 19.8 us.
+    auto pair2 = [&](auto uni, auto ph, auto near, const int ka, const int kb, const bool ina,
+                     const bool inb, const float4& xa, const float4& xb, const float4& va,
+                     const float4& vb) {
+        constexpr bool UNI = decltype(uni)::value, NEAR = decltype(near)::value;
+        constexpr int PH = decltype(ph)::value;
+        f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
+        if (!ina) mj.x = 0.f;
+        if (!inb) mj.y = 0.f;
+        if ((PH & 4) && P.wall_model == 1) {  // push only
+            if (__ldg(B.itype + ka) != it_i) mj.x = 0.f;
+            if (__ldg(B.itype + kb) != it_i) mj.y = 0.f;
+        }
+        f2 d0 = make_float2(xi.x - xa.x, xi.x - xb.x), d1 = make_float2(xi.y - xa.y, xi.y - xb.y);
+        f2 d2 = DIM == 3 ? make_float2(xi.z - xa.z, xi.z - xb.z) : bc2(0.f);
+        f2 ddl = bc2(0.f);  // 2 dh . dl of the residuals dl
+        if (!plain) {
+            float ha[3], la[3], hb[3], lb[3];
+            exact_delta<DIM>(xi, xa, g, ha, la);
+            exact_delta<DIM>(xi, xb, g, hb, lb);
+            d0 = make_float2(ha[0], hb[0]);
+            d1 = make_float2(ha[1], hb[1]);
+            ddl = fma2(d1, make_float2(la[1], lb[1]), mul2(d0, make_float2(la[0], lb[0])));
+            if (DIM == 3) {
+                d2 = make_float2(ha[2], hb[2]);
+                ddl = fma2(d2, make_float2(la[2], lb[2]), ddl);
+            }
+            ddl = add2(ddl, ddl);
+        }
+        ff2 ih = {bc2(ih_i.hi), bc2(ih_i.lo)}, cm = {mj, bc2(0.f)};  // 1/h; the term's factor
+        if (!UNI) {
+            ih = recip_ff2(mul2(bc2(0.5f), make_float2(xi.w + xa.w, xi.w + xb.w)));
+            ff2 al = sqr_ff2(ih);
+            if (DIM == 3) al = mul_ff2(al, ih);
+            cm = mul_ff2_f(mul_ff2(ff2{bc2(kw.hi), bc2(kw.lo)}, al), mj);
+        }
+        f2 t;  // 1 - q/2, 0 beyond the support
+        if (NEAR) {
+            ff2 dr2 = two_prod2(d0, d0);
+            {
+                const ff2 p1 = two_prod2(d1, d1), w = two_sum2(dr2.hi, p1.hi);
+                dr2.lo = add2(add2(add2(dr2.lo, p1.lo), w.lo), ddl);
+                dr2.hi = w.hi;
+            }
+            if (DIM == 3) {
+                const ff2 p2 = two_prod2(d2, d2), w = two_sum2(dr2.hi, p2.hi);
+                dr2.lo = add2(add2(dr2.lo, p2.lo), w.lo);
+                dr2.hi = w.hi;
+            }
+            const ff2 q = mul_ff2(sqrt_ff2(dr2), ih);
+            ff2 T = fast_affine2(q, -0.5f, 1.0f);
+            T.hi = max2(T.hi, 0.0f);
+            t = T.hi;
+            if (fluid) {
+                const ff2 f = mul_ff2(sqr_ff2(sqr_ff2(T)), fast_affine2(T, -4.0f, 5.0f));  // t^4 (1 + 2q)
+                const ff2 m = UNI ? mul_ff2_f(f, mj) : mul_ff2(f, cm);
+                acc_ff2(Sh, Sl, m);
+                if ((PH & 4) && nor)
+                    acc_ff2(Wh, Wl, mul_ff2(m, recip_ff2(make_float2(__ldg(B.q + ka), __ldg(B.q + kb)))));
+            }
+        } else {
+            // With uniform h and m every pair would share the rounding of K m / h^dim
+            // and of 1/h: a bias that adds up over the far pairs. So the prefactor
+            // and 1/h stay float-float, r is the Newton-corrected square root, and
+            // q = r (ih.hi + ih.lo) is rounded once.
+            f2 dr2 = fma2(d1, d1, fma2(d0, d0, bc2(kTinyDr2)));
+            if (DIM == 3) dr2 = fma2(d2, d2, dr2);
+            const f2 rs = rsqrt2(dr2);
+            f2 r = mul2(dr2, rs);
+            r = fma2(fma2(neg2(r), r, dr2), mul2(rs, bc2(0.5f)), r);
+            const f2 q = fma2(r, ih.hi, mul2(r, ih.lo));
+            t = max2(fma2(q, bc2(-0.5f), bc2(1.0f)), 0.0f);
+            if (fluid) {
+                const f2 t2 = mul2(t, t);
+                const f2 f = mul2(mul2(t2, t2), fma2(q, bc2(2.0f), bc2(1.0f)));
+                const f2 m = UNI ? mul2(mj, f) : fma2(cm.hi, f, mul2(cm.lo, f));
+                acc_ff2(Sh, Sl, m);
+                if ((PH & 4) && nor)
+                    acc_ff2(Wh, Wl, mul2(m, rcp2(make_float2(__ldg(B.q + ka), __ldg(B.q + kb)))));
+            }
+        }
+        if ((PH & 1) && need_div) {  // art_heat.f:46-67: grad W = kg (q - 2)^3 d = -8 kg t^3 d
+            f2 kg = bc2(kgih_i);
+            if (!UNI) {
+                const f2 i2 = mul2(ih.hi, ih.hi);
+                kg = mul2(bc2(P.kg), mul2(i2, i2));
+                if (DIM == 3) kg = mul2(kg, ih.hi);
+            }
+            const f2 gm = mul2(mul2(mul2(t, t), mul2(t, bc2(-8.0f))), mul2(kg, mj));
+            f2 vd = fma2(make_float2(va.y - vi.y, vb.y - vi.y), d1,
+                         mul2(make_float2(va.x - vi.x, vb.x - vi.x), d0));
+            if (DIM == 3) vd = fma2(make_float2(va.z - vi.z, vb.z - vi.z), d2, vd);
+            divs = dot2(gm, vd, divs);
+        }
+    };
+    constexpr int W = mask_words<DIM>() / TPP;  // mask words of this lane
+    const size_t mlane = (size_t)s * TPP + sub;
+    bool mask_on = false;
+    int ord = 0;  // candidate ordinal (cursor order, self included)
+    int wb = 0;   // the accumulator holds the bits of ordinals 32 wb .. 32 wb + 63
+    unsigned long long cur = 0ull;
+    auto walk = [&](auto uni, auto ph) {
+    constexpr bool UNI = decltype(uni)::value;
+    constexpr bool VJ = DIM == 3 || (decltype(ph)::value & 1) != 0;  // the neighbour's v is read
+    const std::true_type kNear{};
+    const std::false_type kFar{};
+    {
+        const sph::ff self = UNI ? sph::ff{mi, 0.f} : sph::ff_mul_f(al_i, mi);
+        if (sub == 0) {
+            Sh.x = self.hi;
+            Sl.x = self.lo;
+            if (nor) {
+                const sph::ff w = sph::ff_mul(self, sph::ff_recip(B.q[s]));
+                Wh.x = w.hi;
+                Wl.x = w.lo;
+            }
+        }
+    }
+    // A listed particle evaluates each list entry as it is read, the near ones in
+    // float-float, the far ones (2D) like the cell walk's far pairs: no candidate
+    // lists in shared memory, no second load. The cell walk below serves the others.
     if (LST) {
         constexpr int NB = density_list_batch<DIM>();
-        const int lcm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
-        // (a lane past the last slot reads slot 0: its loads stay in bounds)
-        auto entry = [&](int t) {
-            return lc > 0 ? __ldg(B.nlist + (size_t)min(t, lc - 1) * B.lstride + s) : (valid ? s : 0);
-        };
-        int kn[NB];  // the next batch's entries, loaded one batch ahead
-#pragma unroll
-        for (int u = 0; u < NB; ++u) kn[u] = entry(u);
-        for (int t0 = 0; t0 < lcm; t0 += NB) {
-            int kb[NB];
-            float4 xb[NB], vb[NB];
-#pragma unroll
-            for (int u = 0; u < NB; ++u) kb[u] = kn[u];
-            if (t0 + NB < lcm) {
-#pragma unroll
-                for (int u = 0; u < NB; ++u) kn[u] = entry(t0 + NB + u);
-            }
-#pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                xb[u] = __ldg(xsrc + kb[u]);
-                vb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (DIM == 3 || need_div) vb[u] = __ldg(vsrc + kb[u]);
-            }
-#pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                const int k = kb[u];
-                const float4 xj = xb[u];
-                // no pair test: the kernel's support (W = 0 for q >= 2) drops the
-                // entries beyond it
-                bool in = t0 + u < lc;
-                if (!LEAN && P.wall_model == 1 && __ldg(B.itype + k) != it_i) in = false;  // push only
-                const float mj = mass_of<DIM>(xj, vb[u]);
-                float dh[3], dl[3];
-                exact_delta<DIM>(xi, xj, g, dh, dl);
-                sph::ff ih = ih_i, al = al_i;
-                if (xj.w != xi.w) {
-                    ih = sph::ff_recip(__fmul_rn(0.5f, __fadd_rn(xi.w, xj.w)));
-                    al = sph::ff_mul(kw, ff_pow_dim<DIM>(ih));
-                }
-                if (fluid) {
-                    const sph::ff wm = sph::wendland_mw_ff<DIM, true>(dh, dl, ih, al, mj);
-                    if (in) {
-                        sph::ff_acc(S, wm);
-                        if (nor) sph::ff_acc(Wn, sph::ff_mul(wm, sph::ff_recip(__ldg(B.q + k))));
-                    }
-                }
-                if (need_div && in) {
-                    const float4 vj = vb[u];
-                    const float r2 = sph::dist2_exact<DIM>(dh);
-                    float gw = sph::wendland_grad_factor<DIM>(
-                        fast_sqrt_pos(r2), ih.hi, __fmul_rn(P.kg, pow_grad<DIM>(ih.hi)));
-                    if (!(fast_sqrt_pos(r2) * ih.hi < 2.0f)) gw = 0.f;  // beyond the support
-                    float vd = fmaf(vj.y - vi.y, dh[1], __fmul_rn(vj.x - vi.x, dh[0]));
-                    if (DIM == 3) vd = fmaf(vj.z - vi.z, dh[2], vd);
-                    divs = fmaf(mj * gw, vd, divs);
-                }
-            }
-        }
-        // 2D far entries (the rows after the near ones): FP32 weights with
-        // the float-float prefactor, zero beyond the support.
-        if constexpr (DIM == 2) {
-            constexpr int NF = density_far_batch();
-            const int lfm = __reduce_max_sync(0xffffffffu, lf);
-            auto fentry = [&](int t) {
-                return lf > 0 ? __ldg(B.nlist + (size_t)(lc + min(t, lf - 1)) * B.lstride + s)
-                              : (valid ? s : 0);
+        auto rows = [&](auto near, const int first, const int cnt) {
+            const int cm = __reduce_max_sync(0xffffffffu, cnt > 0 ? cnt : 0);
+            auto entry = [&](int t) {
+                return t < cnt ? __ldg(B.nlist + (size_t)(first + t) * B.lstride + s) : kself;
             };
-            int kf[NF];
+            int kn[NB];  // the next batch's entries, loaded one batch ahead
 #pragma unroll
-            for (int u = 0; u < NF; ++u) kf[u] = fentry(u);
-            for (int t0 = 0; t0 < lfm; t0 += NF) {
-                int kb[NF];
-                float4 xb[NF], vb[NF];
+            for (int u = 0; u < NB; ++u) kn[u] = entry(u);
+            for (int t0 = 0; t0 < cm; t0 += NB) {
+                int kb[NB];
+                float4 xb[NB], vb[NB];
 #pragma unroll
-                for (int u = 0; u < NF; ++u) kb[u] = kf[u];
-                if (t0 + NF < lfm) {
+                for (int u = 0; u < NB; ++u) kb[u] = kn[u];
+                if (t0 + NB < cm) {
 #pragma unroll
-                    for (int u = 0; u < NF; ++u) kf[u] = fentry(t0 + NF + u);
+                    for (int u = 0; u < NB; ++u) kn[u] = entry(t0 + NB + u);
                 }
 #pragma unroll
-                for (int u = 0; u < NF; ++u) {
+                for (int u = 0; u < NB; ++u) {
                     xb[u] = __ldg(xsrc + kb[u]);
-                    vb[u] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (need_div) vb[u] = __ldg(vsrc + kb[u]);
+                    vb[u] = VJ ? __ldg(vsrc + kb[u]) : xb[u];
                 }
 #pragma unroll
-                for (int u = 0; u < NF; ++u) {
-                    const int k = kb[u];
-                    const float4 xj = xb[u];
-                    bool in = t0 + u < lf;
-                    if (!LEAN && P.wall_model == 1 && __ldg(B.itype + k) != it_i) in = false;  // push only
-                    const float mj = mass_of<DIM>(xj, vb[u]);
-                    float d[3], dr2;
-                    pair_delta<DIM>(xi, xj, g, d, dr2);
-                    refine_periodic<DIM>(xi, xj, g, d, dr2);
-                    sph::ff ih = ih_i, al = al_i;
-                    float kgih = kgih_i;
-                    if (xj.w != xi.w) {
-                        ih = sph::ff_recip(__fmul_rn(0.5f, __fadd_rn(xi.w, xj.w)));
-                        al = sph::ff_mul(kw, ff_pow_dim<DIM>(ih));
-                        kgih = P.kg * pow_grad<DIM>(ih.hi);
-                    }
-                    float r = 0.f;
-                    if (dr2 > 0.f) {
-                        const float rs = rsqrtf(dr2);
-                        r = __fmul_rn(dr2, rs);
-                        r = fmaf(fmaf(-r, r, dr2), 0.5f * rs, r);
-                    }
-                    const float q = fmaf(r, ih.hi, __fmul_rn(r, ih.lo));
-                    if (fluid && in) {
-                        float tt = fmaxf(fmaf(-0.5f, q, 1.0f), 0.0f);  // 0 beyond the support
-                        tt = tt * tt;
-                        tt = tt * tt;
-                        const float f = tt * fmaf(2.0f, q, 1.0f);
-                        const sph::ff c = sph::ff_mul_f(al, mj);
-                        const float wm = fmaf(c.hi, f, __fmul_rn(c.lo, f));
-                        sph::ff_acc(S, sph::ff{wm, 0.f});
-                        if (nor) sph::ff_acc(Wn, sph::ff{__fdiv_rn(wm, __ldg(B.q + k)), 0.f});
-                    }
-                    if (need_div && in && q < 2.0f) {
-                        const float4 vj = vb[u];
-                        const float t3 = q - 2.0f;
-                        const float gw = kgih * t3 * t3 * t3;
-                        float vd = fmaf(vj.y - vi.y, d[1], __fmul_rn(vj.x - vi.x, d[0]));
-                        divs = fmaf(mj * gw, vd, divs);
-                    }
-                }
+                for (int u = 0; u < NB; u += 2)
+                    pair2(uni, ph, near, kb[u], kb[u + 1], t0 + u < cnt, t0 + u + 1 < cnt, xb[u],
+                          xb[u + 1], vb[u], vb[u + 1]);
             }
-        }
+        };
+        rows(kNear, 0, lc);
+        if (DIM == 2) rows(kFar, lc, lf);
         if (lc >= 0) done = true;
     }
+    if (!__any_sync(0xffffffffu, !done)) return;
+    CellCoord cc = {{0, 0, 0}};
+    Cursor cu = cursor_begin<DIM>(g);
+    if (!done) {
+        cc = decode_key<DIM>(keys[s], g);
+        mask_on = fluid;
+    }
+    int shift = 0;  // staged index - slot in the cursor's row
     while (__any_sync(0xffffffffu, !done)) {
         int nn = 0, nf = 0;
         // Test phase: fill the near / far lists, kTestBatch candidate loads in flight.
@@ -1732,86 +1774,42 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
         }
         const int mn = __reduce_max_sync(0xffffffffu, nn);
         const int mf = __reduce_max_sync(0xffffffffu, nf);
-        // Near pairs: float-float weights on the exact pair difference.
-        for (int t = 0; t < mn; ++t) {
-            if (t >= nn) continue;
-            const int k = (int)s_near[t][tid];
-            if (!LEAN && P.wall_model == 1 && __ldg(B.itype + k) != it_i) continue;  // push only
-            const float4 xj = STG ? SV.x[k] : __ldg(xsrc + k);
-            float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (DIM == 3 || need_div) vj = STG ? SV.v[k] : __ldg(vsrc + k);
-            const float mj = mass_of<DIM>(xj, vj);
-            float dh[3], dl[3];
-            exact_delta<DIM>(xi, xj, g, dh, dl);
-            sph::ff ih = ih_i, al = al_i;
-            if (xj.w != xi.w) {
-                ih = sph::ff_recip(__fmul_rn(0.5f, __fadd_rn(xi.w, xj.w)));
-                al = sph::ff_mul(kw, ff_pow_dim<DIM>(ih));
+        auto listed = [&](auto near, LT (*lst)[BS], const int cnt, const int cm) {
+            for (int t = 0; t < cm; t += 2) {
+                int kb[2];
+                float4 xb[2], vb[2];
+#pragma unroll
+                for (int u = 0; u < 2; ++u) {
+                    const int k = kb[u] = t + u < cnt ? (int)lst[t + u][tid] : kself;
+                    xb[u] = STG ? SV.x[k] : __ldg(xsrc + k);
+                    vb[u] = !VJ ? xb[u] : STG ? SV.v[k] : __ldg(vsrc + k);
+                }
+                pair2(uni, ph, near, kb[0], kb[1], t < cnt, t + 1 < cnt, xb[0], xb[1], vb[0], vb[1]);
             }
-            if (fluid) {
-                const sph::ff wm = sph::wendland_mw_ff<DIM>(dh, dl, ih, al, mj);
-                sph::ff_acc(S, wm);
-                if (nor) sph::ff_acc(Wn, sph::ff_mul(wm, sph::ff_recip(__ldg(B.q + k))));
-            }
-            if (need_div) {
-                const float dr2 = sph::dist2_exact<DIM>(dh);
-                const float gw = sph::wendland_grad_factor<DIM>(
-                    fast_sqrt_pos(dr2), ih.hi, __fmul_rn(P.kg, pow_grad<DIM>(ih.hi)));
-                float vd = fmaf(vj.y - vi.y, dh[1], __fmul_rn(vj.x - vi.x, dh[0]));
-                if (DIM == 3) vd = fmaf(vj.z - vi.z, dh[2], vd);
-                divs = fmaf(mj * gw, vd, divs);
-            }
-        }
-        // Far pairs: FP32 weights (each below ~1% of the self term).
-        for (int t = 0; t < mf; ++t) {
-            if (t >= nf) continue;
-            const int k = (int)s_far[t][tid];
-            if (!LEAN && P.wall_model == 1 && __ldg(B.itype + k) != it_i) continue;
-            const float4 xj = STG ? SV.x[k] : __ldg(xsrc + k);
-            float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (DIM == 3 || need_div) vj = STG ? SV.v[k] : __ldg(vsrc + k);
-            const float mj = mass_of<DIM>(xj, vj);
-            float d[3], dr2;
-            pair_delta<DIM>(xi, xj, g, d, dr2);
-            refine_periodic<DIM>(xi, xj, g, d, dr2);
-            // With uniform h and m every pair would share the rounding of
-            // K m / h^dim and of 1/h: a bias that adds up over the far pairs.
-            // So the prefactor and 1/h stay float-float, r is the
-            // Newton-corrected square root, and q is rounded once.
-            sph::ff ih = ih_i, al = al_i;
-            float kgih = kgih_i;
-            if (xj.w != xi.w) {
-                ih = sph::ff_recip(__fmul_rn(0.5f, __fadd_rn(xi.w, xj.w)));
-                al = sph::ff_mul(kw, ff_pow_dim<DIM>(ih));
-                kgih = P.kg * pow_grad<DIM>(ih.hi);
-            }
-            float r = 0.f;
-            if (dr2 > 0.f) {
-                const float rs = rsqrtf(dr2);
-                r = __fmul_rn(dr2, rs);
-                r = fmaf(fmaf(-r, r, dr2), 0.5f * rs, r);
-            }
-            // one rounding of r (ih.hi + ih.lo): rounding r ih.hi first and then
-            // adding r ih.lo would lose the correction, the same way for all pairs
-            const float q = fmaf(r, ih.hi, __fmul_rn(r, ih.lo));
-            if (fluid) {
-                float tt = fmaf(-0.5f, q, 1.0f);
-                tt = tt * tt;
-                tt = tt * tt;
-                const float f = tt * fmaf(2.0f, q, 1.0f);
-                const sph::ff c = sph::ff_mul_f(al, mj);
-                const float wm = fmaf(c.hi, f, __fmul_rn(c.lo, f));
-                sph::ff_acc(S, sph::ff{wm, 0.f});
-                if (nor) sph::ff_acc(Wn, sph::ff{__fdiv_rn(wm, __ldg(B.q + k)), 0.f});
-            }
-            if (need_div) {
-                const float t3 = q - 2.0f;
-                const float gw = kgih * t3 * t3 * t3;
-                float vd = fmaf(vj.y - vi.y, d[1], __fmul_rn(vj.x - vi.x, d[0]));
-                if (DIM == 3) vd = fmaf(vj.z - vi.z, d[2], vd);
-                divs = fmaf(mj * gw, vd, divs);
-            }
-        }
+        };
+        listed(kNear, s_near, nn, mn);
+        if (DIM == 2) listed(kFar, s_far, nf, mf);
+    }
+    };
+    using std::integral_constant;
+    const bool uni = TPP == 1 && g.huni && (LEAN || OPT || P.wall_model != 1);
+    if constexpr (LEAN) {
+        if (uni) walk(std::true_type{}, integral_constant<int, 0>{});
+        else walk(std::false_type{}, integral_constant<int, 0>{});
+    } else if constexpr (TPP == 1 && !OPT) {
+        if (uni && !need_div) walk(std::true_type{}, integral_constant<int, 0>{});
+        else if (uni) walk(std::true_type{}, integral_constant<int, 1>{});
+        else walk(std::false_type{}, integral_constant<int, 7>{});
+    } else {
+        if (uni) walk(std::true_type{}, integral_constant<int, 7>{});
+        else walk(std::false_type{}, integral_constant<int, 7>{});
+    }
+    sph::ff S = {Sh.x, Sl.x}, Wn = {Wh.x, Wl.x};
+    sph::ff_acc(S, sph::ff{Sh.y, Sl.y});
+    if (OPT) sph::ff_acc(Wn, sph::ff{Wh.y, Wl.y});
+    if (uni) {
+        S = sph::ff_mul(al_i, S);
+        if (OPT) Wn = sph::ff_mul(al_i, Wn);
     }
     if (TPP > 1) {  // the particle's lanes reach this point together
         const unsigned gm = group_mask<TPP>();

@@ -38,9 +38,69 @@ __device__ __forceinline__ float rsqrt_fast(float a) {
 __device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp_fast(a.x), rcp_fast(a.y)); }
 __device__ __forceinline__ f2 rsqrt2(f2 a) { return make_float2(rsqrt_fast(a.x), rsqrt_fast(a.y)); }
 
+// ---- float-float on two values at once (hi + lo each; sph_math.cuh's forms) ----
+struct ff2 {
+    f2 hi, lo;
+};
+// Knuth TwoSum: hi + lo == a + b exactly.
+__device__ __forceinline__ ff2 two_sum2(f2 a, f2 b) {
+    const f2 s = add2(a, b), bb = sub2(s, a);
+    return {s, add2(sub2(a, sub2(s, bb)), sub2(b, bb))};
+}
+__device__ __forceinline__ ff2 two_prod2(f2 a, f2 b) {
+    const f2 p = mul2(a, b);
+    return {p, fma2(a, b, neg2(p))};
+}
+__device__ __forceinline__ ff2 mul_ff2(ff2 a, ff2 b) {
+    ff2 p = two_prod2(a.hi, b.hi);
+    p.lo = fma2(a.hi, b.lo, fma2(a.lo, b.hi, p.lo));
+    return p;
+}
+__device__ __forceinline__ ff2 mul_ff2_f(ff2 a, f2 b) {
+    ff2 p = two_prod2(a.hi, b);
+    p.lo = fma2(a.lo, b, p.lo);
+    return p;
+}
+__device__ __forceinline__ ff2 sqr_ff2(ff2 a) {
+    ff2 p = two_prod2(a.hi, a.hi);
+    p.lo = fma2(add2(a.hi, a.hi), a.lo, p.lo);
+    return p;
+}
+// c + k a for |c| >= |k a.hi| and k a power of two (Fast2Sum).
+__device__ __forceinline__ ff2 fast_affine2(ff2 a, float k, float c) {
+    const f2 s = fma2(a.hi, bc2(k), bc2(c));
+    const f2 z = sub2(s, bc2(c));
+    return {s, fma2(a.lo, bc2(k), fma2(a.hi, bc2(k), neg2(z)))};
+}
+// 1/a: the hardware reciprocal and its exact residual (relative error ~2^-44).
+__device__ __forceinline__ ff2 recip_ff2(f2 a) {
+    const f2 r = rcp2(a);
+    return {r, mul2(r, fma2(neg2(r), a, bc2(1.0f)))};
+}
+// acc += x, every rounding error collected in the low part.
+__device__ __forceinline__ void acc_ff2(f2& hi, f2& lo, ff2 x) {
+    const ff2 s = two_sum2(hi, x.hi);
+    hi = s.hi;
+    lo = add2(lo, add2(s.lo, x.lo));
+}
+__device__ __forceinline__ void acc_ff2(f2& hi, f2& lo, f2 x) {
+    const ff2 s = two_sum2(hi, x);
+    hi = s.hi;
+    lo = add2(lo, s.lo);
+}
+
 // Added to squared distances before a reciprocal square root: no effect on any
 // distance above 1e-15 times the unit, and a coincident pair (or a particle
 // with itself) gets r = 0 without a comparison.
 constexpr float kTinyDr2 = 1.0e-37f;
+
+// sqrt: the hardware reciprocal square root and one Newton correction from the exact
+// residual a.hi - r^2 (relative error ~2^-44). 0 for a = 0.
+__device__ __forceinline__ ff2 sqrt_ff2(ff2 a) {
+    const f2 rs = rsqrt2(max2(a.hi, kTinyDr2));
+    const f2 r = mul2(a.hi, rs);
+    const f2 res = add2(fma2(neg2(r), r, a.hi), a.lo);
+    return {r, mul2(res, mul2(rs, bc2(0.5f)))};
+}
 
 }  // namespace ag
