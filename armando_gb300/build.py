@@ -1,17 +1,20 @@
-"""In-tree build of the sm_103a library (nvcc, one translation unit)."""
+"""In-tree build of the sm_103a library: nvcc, one translation unit for the C-ABI and
+one per neighbour pass and dimension, compiled side by side."""
 from __future__ import annotations
 
 import os
 import subprocess
+import tempfile
+from concurrent.futures import ThreadPoolExecutor
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = os.path.join(HERE, "csrc", "armando.cu")
+UNITS = ("armando", "pass_density2d", "pass_density3d", "pass_force2d", "pass_force3d")
 OUT = os.path.join(HERE, "lib", "libarmando_gb300.so")
 
 NVCC_FLAGS = [
     "-std=c++17", "-O3", "-lineinfo",
     "-gencode", "arch=compute_103a,code=sm_103a",
-    "-Xcompiler", "-fPIC", "-shared",
+    "-Xcompiler", "-fPIC",
     # host code rounds like the oracle on x86 and on Arm (no fused multiply-add)
     "-Xcompiler", "-ffp-contract=off",
 ]
@@ -32,15 +35,24 @@ def up_to_date() -> bool:
 
 
 def build_library(force: bool = False, verbose: bool = False, extra_flags=()) -> str:
-    """Compiles csrc/armando.cu into lib/libarmando_gb300.so (skipped when fresh)."""
+    """Compiles csrc/*.cu into lib/libarmando_gb300.so (skipped when fresh)."""
     if not force and up_to_date():
         return OUT
     os.makedirs(os.path.dirname(OUT), exist_ok=True)
     nvcc = os.environ.get("NVCC", "nvcc")
-    cmd = [nvcc, *NVCC_FLAGS, *extra_flags, "-o", OUT, SRC]
-    if verbose:
-        print(" ".join(cmd))
-    subprocess.run(cmd, check=True)
+
+    def run(cmd):
+        if verbose:
+            print(" ".join(cmd))
+        subprocess.run(cmd, check=True)
+
+    with tempfile.TemporaryDirectory(dir=os.path.dirname(OUT)) as tmp:
+        objs = [os.path.join(tmp, u + ".o") for u in UNITS]
+        cmds = [[nvcc, *NVCC_FLAGS, *extra_flags, "-c", "-o", o, os.path.join(HERE, "csrc", u + ".cu")]
+                for u, o in zip(UNITS, objs)]
+        with ThreadPoolExecutor(len(cmds)) as ex:
+            list(ex.map(run, cmds))
+        run([nvcc, *NVCC_FLAGS, "-shared", "-o", OUT, *objs])
     return OUT
 
 

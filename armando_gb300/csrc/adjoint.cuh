@@ -155,7 +155,7 @@ __global__ void k_adj_store(AdjState G, int n, float* __restrict__ xbar, float* 
 
 // Corrector reverse: x' = x + dt v', v' = v + kdt a, u' = max(0, u + kdt du),
 // outputs also carry a and du to the next predictor.
-__global__ void k_adj_out(StateB B, const float* __restrict__ du_out, AdjState G, StepArgs S,
+static __global__ void k_adj_out(StateB B, const float* __restrict__ du_out, AdjState G, StepArgs S,
                           float4* __restrict__ abar, float4* __restrict__ xpart,
                           float4* __restrict__ vpart, int n) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -785,7 +785,7 @@ __global__ void __launch_bounds__(kPassThreads)
 }
 
 // Adds the step's parameter cotangents (block partials, fixed order) to acc.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
     k_adj_params(const double* __restrict__ block_part, int nblocks, double* __restrict__ acc) {
     __shared__ double s[ADJ_NPARAM][256];
     for (int q = 0; q < ADJ_NPARAM; ++q) {

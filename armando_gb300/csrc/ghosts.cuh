@@ -157,7 +157,7 @@ __global__ void k_wall_keys(StateA A, int n, const WallGrid* __restrict__ wgp,
 }
 
 // The walls in cell order: position {x, h} and normal of each, and its index.
-__global__ void k_wall_gather(const int* __restrict__ order, const int* __restrict__ wstart,
+static __global__ void k_wall_gather(const int* __restrict__ order, const int* __restrict__ wstart,
                               const WallGrid* __restrict__ wgp, StateA A, int n,
                               float4* __restrict__ wall_xh, float4* __restrict__ wall_n,
                               int* __restrict__ wall_id) {
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(kGhostThreads)
 }
 
 // Exclusive scan of the tile counts (one block); total = ghosts this iteration.
-__global__ void __launch_bounds__(1024)
+static __global__ void __launch_bounds__(1024)
     k_ghost_scan(const unsigned* __restrict__ tile_count, int tiles, unsigned* __restrict__ tile_off,
                  int* __restrict__ total) {
     __shared__ unsigned s_warp[32];

@@ -497,7 +497,7 @@ __global__ void __launch_bounds__(kGhostThreads)
 }
 
 // The kept particles of A, in order, into D.
-__global__ void __launch_bounds__(kGhostThreads)
+static __global__ void __launch_bounds__(kGhostThreads)
     k_open_compact(StateA A, StateA D, int n, const int* __restrict__ keep,
                    const unsigned* __restrict__ tile_off) {
     __shared__ unsigned s_warp[32];
@@ -523,7 +523,7 @@ __global__ void __launch_bounds__(kGhostThreads)
 }
 
 // Keys of the output order: the particles' serial numbers.
-__global__ void k_open_id_keys(StateA A, int n, unsigned* __restrict__ keys) {
+static __global__ void k_open_id_keys(StateA A, int n, unsigned* __restrict__ keys) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) keys[s] = (unsigned)A.id[s];
 }

@@ -216,14 +216,14 @@ __device__ __forceinline__ unsigned resort_begin(int* resort, int* sorts) {
     return sort;
 }
 
-__global__ void k_resort_begin(int* __restrict__ resort, int* __restrict__ sorts) {
+static __global__ void k_resort_begin(int* __restrict__ resort, int* __restrict__ sorts) {
     if (threadIdx.x == 0 && blockIdx.x == 0) resort_begin(resort, sorts);
 }
 
 // Head of a lazily sorting step graph: starts the iteration; the IF node
 // after it runs the grid, hash, sort and cell-table kernels only when this
 // iteration sorts.
-__global__ void k_resort_cond(cudaGraphConditionalHandle handle, int* __restrict__ resort,
+static __global__ void k_resort_cond(cudaGraphConditionalHandle handle, int* __restrict__ resort,
                               int* __restrict__ sorts) {
     if (threadIdx.x == 0 && blockIdx.x == 0)
         cudaGraphSetConditional(handle, resort_begin(resort, sorts));
@@ -265,7 +265,7 @@ __device__ __forceinline__ unsigned block_excl_scan(unsigned v, unsigned* s_warp
 // ---------------------------------------------------------------------------
 // Grid: bbox of all particles and the link_list grid in FP32.
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__ xh, int n, int dim,
+static __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__ xh, int n, int dim,
                                                       float* __restrict__ part,
     const int* __restrict__ resort = nullptr) {
     if (sort_skipped(resort)) return;
@@ -317,7 +317,7 @@ __global__ void __launch_bounds__(256) k_bbox_partial(const float4* __restrict__
 __device__ __forceinline__ DevGrid grid_from_bbox(const float* mm, const DevParams& P,
                                                   long long capacity, unsigned& fl);
 
-__global__ void __launch_bounds__(256) k_bbox_final(const float* __restrict__ part, int nparts,
+static __global__ void __launch_bounds__(256) k_bbox_final(const float* __restrict__ part, int nparts,
                                                     DevParams P, long long capacity,
                                                     DevGrid* __restrict__ grid,
                                                     unsigned* __restrict__ flags,
@@ -533,7 +533,7 @@ __global__ void k_keys_only(const float4* __restrict__ xh, int n, const DevGrid*
 // ---------------------------------------------------------------------------
 // LSD radix sort, reduce-then-scan (no inter-block waiting).
 // ---------------------------------------------------------------------------
-__global__ void __launch_bounds__(kSortThreads)
+static __global__ void __launch_bounds__(kSortThreads)
     k_radix_hist(const unsigned* __restrict__ keys, int n, int shift, unsigned* __restrict__ hist,
                  int num_tiles,
     const int* __restrict__ resort = nullptr) {
@@ -552,7 +552,7 @@ __global__ void __launch_bounds__(kSortThreads)
 }
 
 // Block d: exclusive scan of the tile counts of digit d; total per digit.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
     k_radix_scan(unsigned* __restrict__ hist, int num_tiles, unsigned* __restrict__ dtotal,
     const int* __restrict__ resort = nullptr) {
     if (sort_skipped(resort)) return;
@@ -575,7 +575,7 @@ __global__ void __launch_bounds__(256)
 
 // Stable scatter of one tile by one 8-bit digit. vals_in == nullptr means
 // the values are the slot indices themselves.
-__global__ void __launch_bounds__(kSortThreads)
+static __global__ void __launch_bounds__(kSortThreads)
     k_radix_scatter(const unsigned* __restrict__ keys_in, const int* __restrict__ vals_in,
                     unsigned* __restrict__ keys_out, int* __restrict__ vals_out, int n, int shift,
                     const unsigned* __restrict__ hist, const unsigned* __restrict__ dtotal,
@@ -660,7 +660,7 @@ __global__ void __launch_bounds__(kSortThreads)
 // time. Entries past `cap` (the table's last index) are never written.
 constexpr int kCellStartThreads = 256;
 
-__global__ void __launch_bounds__(kCellStartThreads)
+static __global__ void __launch_bounds__(kCellStartThreads)
     k_cell_start(const unsigned* __restrict__ keys, int n, const int* __restrict__ ncells_total,
                  int cap, int* __restrict__ start,
     const int* __restrict__ resort = nullptr) {
@@ -781,19 +781,19 @@ __global__ void k_load_xh(const float* __restrict__ x, const float* __restrict__
 
 // inv[id[s]] = s: the cell-order slot of each caller index.
 // dst[id[s]] = src[s]: a slot-order array back to caller order.
-__global__ void k_scatter_by_id(const float* __restrict__ src, const int* __restrict__ id,
+static __global__ void k_scatter_by_id(const float* __restrict__ src, const int* __restrict__ id,
                                 float* __restrict__ dst, int n) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) dst[id[s]] = src[s];
 }
 
 // Smoothing lengths of A in caller order.
-__global__ void k_hsml_out(StateA A, float* __restrict__ h, int n) {
+static __global__ void k_hsml_out(StateA A, float* __restrict__ h, int n) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) h[A.id[s]] = A.xh[s].w;
 }
 
-__global__ void k_invert_ids(const int* __restrict__ id, int* __restrict__ inv, int n) {
+static __global__ void k_invert_ids(const int* __restrict__ id, int* __restrict__ inv, int n) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s < n) inv[id[s]] = s;
 }
@@ -810,7 +810,7 @@ constexpr int kScatterSeq = 256;
 // after the density pass (the force pass copies them): written to the caller's
 // arrays from a few CTAs on a second stream while the force pass runs. inv is
 // the inverse of B.id.
-__global__ void k_scatter_rp(StateB B, const int* __restrict__ inv, int n, float* __restrict__ rho,
+static __global__ void k_scatter_rp(StateB B, const int* __restrict__ inv, int n, float* __restrict__ rho,
                              float* __restrict__ p) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const int s = inv[i];
@@ -940,7 +940,7 @@ __global__ void k_reorder_dim(StateA A, const int* __restrict__ perm, StateB B, 
 
 // Positions in cell order on an iteration that sorts (B.xsort), read by the
 // list build as contiguous candidate ranges.
-__global__ void k_sorted_positions(StateA A, const int* __restrict__ perm, StateB B, int n,
+static __global__ void k_sorted_positions(StateA A, const int* __restrict__ perm, StateB B, int n,
                                    const int* __restrict__ resort) {
     if (sort_skipped(resort)) return;
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
@@ -949,7 +949,7 @@ __global__ void k_sorted_positions(StateA A, const int* __restrict__ perm, State
 }
 
 // Positions only (neighbour entry point).
-__global__ void k_reorder_xh(StateA A, const int* __restrict__ perm, StateB B, int n) {
+static __global__ void k_reorder_xh(StateA A, const int* __restrict__ perm, StateB B, int n) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
     const int j = perm[s];
@@ -961,7 +961,7 @@ __global__ void k_reorder_xh(StateA A, const int* __restrict__ perm, StateB B, i
 // Batched grid, hash and reorder (one cell grid per instance).
 // ---------------------------------------------------------------------------
 // Bbox partial {min[3], max[3], max h} of every work item.
-__global__ void __launch_bounds__(kPassThreads)
+static __global__ void __launch_bounds__(kPassThreads)
     k_bbox_items(const float4* __restrict__ xh, const WorkItem* __restrict__ items, int dim,
                  float* __restrict__ part) {
     const WorkItem w = items[blockIdx.x];
@@ -994,7 +994,7 @@ __global__ void __launch_bounds__(kPassThreads)
 }
 
 // Grid of instance blockIdx.x from the partials of its items.
-__global__ void __launch_bounds__(256)
+static __global__ void __launch_bounds__(256)
     k_bbox_final_batch(const float* __restrict__ part, const int* __restrict__ inst_items,
                        const DevParams* __restrict__ params, DevGrid* __restrict__ grids,
                        int* __restrict__ ncells_inst, unsigned* __restrict__ flags) {
@@ -1025,7 +1025,7 @@ __global__ void __launch_bounds__(256)
 
 // Cell offsets of the instances in the shared table (exclusive scan of their
 // cell counts); a total above the table's capacity disables every grid.
-__global__ void __launch_bounds__(1024)
+static __global__ void __launch_bounds__(1024)
     k_cell_offsets(const int* __restrict__ ncells_inst, int n_inst, long long capacity,
                    DevGrid* __restrict__ grids, int* __restrict__ total_cells,
                    unsigned* __restrict__ flags) {
@@ -1111,7 +1111,7 @@ __global__ void k_reorder_batch(StateA A, const int* __restrict__ perm, StateB B
     B.inst[s] = k;
 }
 
-__global__ void k_advance_its(int* its) { *its += 1; }
+static __global__ void k_advance_its(int* its) { *its += 1; }
 
 // ---------------------------------------------------------------------------
 // Neighbour-cell iteration
