@@ -216,51 +216,59 @@ armando_status force_sort(armando_ctx* ctx) {
 template <int DIM>
 int launch_build_list(armando_ctx* ctx, const int* rs, cudaStream_t st);
 
+// Scan, place and rank of the counting sort; total: the number of cells, gp: the
+// grid (null: batches).
+int launch_cell_order(armando_ctx* ctx, const int* total, const DevGrid* gp, const int* rs,
+                      cudaStream_t st, float4* xsort) {
+    const int n = (int)ctx->n_work, cap = (int)ctx->cell_cap;
+    const int tiles = blocks_for((int64_t)cap + 1, kScanTile);
+    int L = 3;
+    if (tiles > 1) {
+        k_cell_sums<<<tiles, kScanThreads, 0, st>>>(ctx->cell_cnt, total, cap, ctx->cell_sums, rs);
+        ++L;
+    }
+    k_cell_scan<<<tiles, kScanThreads, 0, st>>>(ctx->cell_cnt, total, cap, ctx->cell_sums,
+                                                ctx->start, rs);
+    k_cell_place<<<blocks_for(n, 256), 256, 0, st>>>(ctx->keys[0], ctx->vals[0], ctx->start, gp, n,
+                                                     ctx->placed, ctx->keys[1], rs);
+    k_cell_rank<<<blocks_for(n, 256), 256, 0, st>>>(ctx->placed, ctx->keys[1], ctx->start, gp, n,
+                                                    ctx->vals[1], ctx->A.xh, xsort, ctx->A.inst,
+                                                    ctx->d_grids, rs);
+    return L;
+}
+
+template <int DIM>
+int launch_grid(armando_ctx* ctx, const int* rs, cudaStream_t st) {
+    const int n = (int)ctx->n_work;
+    k_bbox_grid<<<std::max(1, std::min(blocks_for(n, 256), kBBoxBlocks)), 256, 0, st>>>(
+        ctx->A.xh, n, DIM, ctx->bbox_part, ctx->dp, ctx->cell_cap, ctx->grid, ctx->flags,
+        ctx->ticket, rs);
+    k_cell_count<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A.xh, n, ctx->grid, ctx->keys[0],
+                                                         ctx->vals[0], ctx->cell_cnt, rs);
+    return 2;
+}
+
 // lists: also rebuild the neighbour lists (a lazily sorting step).
 template <int DIM>
 int launch_grid_and_sort(armando_ctx* ctx, const int* rs, cudaStream_t st, bool lists = false) {
-    const int n = (int)ctx->n_work;
-    int L = 0;
-    k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(ctx->A.xh, n, DIM, ctx->bbox_part, rs);
-    k_bbox_final<<<1, 256, 0, st>>>(ctx->bbox_part, kBBoxBlocks, ctx->dp, ctx->cell_cap, ctx->grid,
-                                    ctx->flags, rs);
-    k_hash<DIM><<<ctx->num_tiles, kSortThreads, 0, st>>>(ctx->A.xh, n, ctx->grid, ctx->keys[0],
-                                                          ctx->hist, ctx->num_tiles, rs);
-    L += 3;
-    for (int p = 0; p < ctx->passes; ++p) {
-        const int shift = 8 * p;
-        const int a = p & 1, b = (p + 1) & 1;
-        if (p > 0) {
-            k_radix_hist<<<ctx->num_tiles, kSortThreads, 0, st>>>(ctx->keys[a], n, shift,
-                                                                   ctx->hist, ctx->num_tiles, rs);
-            ++L;
-        }
-        k_radix_scan<<<kRadix, 256, 0, st>>>(ctx->hist, ctx->num_tiles, ctx->dtotal, rs);
-        k_radix_scatter<<<ctx->num_tiles, kSortThreads, 0, st>>>(
-            ctx->keys[a], p == 0 ? nullptr : ctx->vals[a], ctx->keys[b], ctx->vals[b], n, shift,
-            ctx->hist, ctx->dtotal, ctx->num_tiles, rs);
-        L += 2;
-    }
-    k_cell_start<<<blocks_for((int64_t)n + 1, kCellStartThreads), kCellStartThreads, 0, st>>>(ctx->keys[ctx->passes & 1], n,
-                                                                   &ctx->grid->ncells, (int)ctx->cell_cap,
-                                                                   ctx->start, rs);
+    int L = launch_grid<DIM>(ctx, rs, st);
+    L += launch_cell_order(ctx, &ctx->grid->ncells, ctx->grid, rs, st,
+                           lists ? ctx->B.xsort : nullptr);
     if (lists) L += launch_build_list<DIM>(ctx, rs, st);
-    return L + 1;
+    return L;
 }
 
 template <int DIM>
 int launch_build_list(armando_ctx* ctx, const int* rs, cudaStream_t st) {
     const int n = (int)ctx->n_work;
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
-    k_sorted_positions<<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, n, rs);
+    const unsigned* skeys = ctx->keys[1];
     if (ctx->dp.periodic[0] || ctx->dp.periodic[1] || ctx->dp.periodic[2])
         k_build_list<DIM, true><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
             ctx->B, skeys, ctx->start, ctx->grid, n, rs);
     else
         k_build_list<DIM, false><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
             ctx->B, skeys, ctx->start, ctx->grid, n, rs);
-    return 2;
+    return 1;
 }
 
 // Start of a lazily sorting iteration launched without the step graph's
@@ -301,8 +309,8 @@ template <int DIM>
 int launch_passes(armando_ctx* ctx, const StepArgs& S, const int* rs, bool reorder = true) {
     cudaStream_t st = ctx->stream;
     const int n = (int)ctx->n_work;
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     int L = 1;
     if (reorder) {
         k_reorder_dim<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, S, n, rs,
@@ -398,7 +406,7 @@ armando_status build_lazy_graph(armando_ctx* ctx, const StepArgs& S, cudaGraphEx
     if (body_reorder) {
         const int n = (int)ctx->n_work;
         k_reorder_dim<DIM><<<blocks_for(n, 256), 256, 0, ctx->stream2>>>(
-            ctx->A, ctx->vals[ctx->passes & 1], ctx->B, S, n);
+            ctx->A, ctx->vals[1], ctx->B, S, n);
         ++body;
     }
     int L = 1 + body;
@@ -432,8 +440,8 @@ int launch_gpuc_passes(armando_ctx* ctx, const StepArgs& S, const int* rs) {
     cudaStream_t st = ctx->stream;
     const int n = (int)ctx->n_work;
     const int nm = ctx->materials.empty() ? ARMANDO_MAX_MATERIALS : (int)ctx->materials.size();
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     ctx->gs.xsort = rs ? ctx->xsort_buf : nullptr;
     k_gpuc_gather<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->gs, ctx->d_mat, nm,
                                                            ctx->flags, n, rs);
@@ -488,24 +496,9 @@ int launch_batch_grid_and_sort(armando_ctx* ctx, long long capacity) {
                                        ctx->d_total_cells, ctx->flags);
     L += 3;
     if (!ctx->start) return L;  // planning: grids only
-    k_hash_batch<DIM><<<ctx->num_tiles, kSortThreads, 0, st>>>(
-        ctx->A.xh, ctx->A.inst, n, ctx->d_grids, ctx->keys[0], ctx->hist, ctx->num_tiles);
-    ++L;
-    for (int p = 0; p < ctx->passes; ++p) {
-        const int shift = 8 * p;
-        const int a = p & 1, b = (p + 1) & 1;
-        if (p > 0) {
-            k_radix_hist<<<ctx->num_tiles, kSortThreads, 0, st>>>(ctx->keys[a], n, shift,
-                                                                   ctx->hist, ctx->num_tiles);
-            ++L;
-        }
-        k_radix_scan<<<kRadix, 256, 0, st>>>(ctx->hist, ctx->num_tiles, ctx->dtotal);
-        k_radix_scatter<<<ctx->num_tiles, kSortThreads, 0, st>>>(
-            ctx->keys[a], p == 0 ? nullptr : ctx->vals[a], ctx->keys[b], ctx->vals[b], n, shift,
-            ctx->hist, ctx->dtotal, ctx->num_tiles);
-        L += 2;
-    }
-    return L;
+    k_cell_count_batch<DIM><<<blocks_for(n, 256), 256, 0, st>>>(
+        ctx->A.xh, ctx->A.inst, n, ctx->d_grids, ctx->keys[0], ctx->vals[0], ctx->cell_cnt);
+    return L + 1 + launch_cell_order(ctx, ctx->d_total_cells, nullptr, nullptr, st, nullptr);
 }
 
 // One leapfrog step of every instance; ev (optional, ARMANDO_N_PHASES + 1
@@ -521,10 +514,8 @@ int launch_batch_step(armando_ctx* ctx, cudaEvent_t* ev) {
         cudaEventRecord(ev[1], st);
         cudaEventRecord(ev[2], st);
     }
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
-    k_cell_start<<<blocks_for((int64_t)n + 1, kCellStartThreads), kCellStartThreads, 0, st>>>(skeys, n, ctx->d_total_cells,
-                                                                   (int)ctx->cell_cap, ctx->start);
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     k_reorder_batch<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, ctx->d_params,
                                                              ctx->d_its, n);
     if (ev) cudaEventRecord(ev[3], st);
@@ -537,7 +528,7 @@ int launch_batch_step(armando_ctx* ctx, cudaEvent_t* ev) {
             ctx->B, skeys, ctx->start, ctx->d_grids, ctx->d_params, ctx->d_items, ctx->n_items,
             ctx->d_queue + 0);
     if (ev) cudaEventRecord(ev[4], st);
-    L += 3;
+    L += 2;
     if (ctx->any_visc) {
         k_shear_batch<DIM><<<ctx->grid_shear, kPassThreads, 0, st>>>(
             ctx->B, skeys, ctx->start, ctx->d_grids, ctx->d_params, ctx->d_items, ctx->n_items,
@@ -572,39 +563,20 @@ int launch_step_phased(armando_ctx* ctx, const StepArgs& S, cudaEvent_t* ev) {
     cudaEventRecord(ev[0], st);
     const int* rs = lazy(ctx) ? resort_flags(ctx) : nullptr;
     if (rs) L += launch_resort_begin(ctx);
-    k_bbox_partial<<<kBBoxBlocks, 256, 0, st>>>(ctx->A.xh, n, DIM, ctx->bbox_part, rs);
-    k_bbox_final<<<1, 256, 0, st>>>(ctx->bbox_part, kBBoxBlocks, ctx->dp, ctx->cell_cap, ctx->grid,
-                                    ctx->flags, rs);
-    k_hash<DIM><<<ctx->num_tiles, kSortThreads, 0, st>>>(ctx->A.xh, n, ctx->grid, ctx->keys[0],
-                                                          ctx->hist, ctx->num_tiles, rs);
-    L += 3;
+    L += launch_grid<DIM>(ctx, rs, st);
     cudaEventRecord(ev[1], st);
-    for (int p = 0; p < ctx->passes; ++p) {
-        const int shift = 8 * p;
-        const int a = p & 1, b = (p + 1) & 1;
-        if (p > 0) {
-            k_radix_hist<<<ctx->num_tiles, kSortThreads, 0, st>>>(ctx->keys[a], n, shift,
-                                                                   ctx->hist, ctx->num_tiles, rs);
-            ++L;
-        }
-        k_radix_scan<<<kRadix, 256, 0, st>>>(ctx->hist, ctx->num_tiles, ctx->dtotal, rs);
-        k_radix_scatter<<<ctx->num_tiles, kSortThreads, 0, st>>>(
-            ctx->keys[a], p == 0 ? nullptr : ctx->vals[a], ctx->keys[b], ctx->vals[b], n, shift,
-            ctx->hist, ctx->dtotal, ctx->num_tiles, rs);
-        L += 2;
-    }
+    L += launch_cell_order(ctx, &ctx->grid->ncells, ctx->grid, rs, st,
+                           use_lists(ctx) ? ctx->B.xsort : nullptr);
     cudaEventRecord(ev[2], st);
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
-    k_cell_start<<<blocks_for((int64_t)n + 1, kCellStartThreads), kCellStartThreads, 0, st>>>(skeys, n, &ctx->grid->ncells,
-                                                                   (int)ctx->cell_cap, ctx->start, rs);
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     if (use_lists(ctx)) L += launch_build_list<DIM>(ctx, rs, st);
     k_reorder_dim<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, S, n, rs,
                                                            fused(ctx));
     cudaEventRecord(ev[3], st);
     launch_density<DIM>(ctx, skeys, S);
     cudaEventRecord(ev[4], st);
-    L += 3;
+    L += 2;
     if (ctx->dp.visc) {
         k_shear<DIM><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
             ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
@@ -695,8 +667,8 @@ int launch_overlapped_step(armando_ctx* ctx, const StepArgs& S, float* rho_out, 
     const int n = (int)ctx->n_work;
     int L = launch_grid_and_sort<DIM>(ctx, nullptr, st);
     cudaStreamWaitEvent(st, ctx->ev_ovl[1], 0);  // the rest of the inputs
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     k_reorder_dim<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, S, n);
     launch_density<DIM>(ctx, skeys, S);
     cudaEventRecord(ctx->ev_ovl[2], st);
@@ -830,6 +802,10 @@ armando_status alloc_state(armando_ctx* ctx) {
         ctx->owned.push_back(ctx->keys[k]);
         ctx->owned.push_back(ctx->vals[k]);
     }
+    ctx->placed = dalloc<int>(n, e);
+    ctx->owned.push_back(ctx->placed);
+    ctx->ticket = dalloc<unsigned>(1, e);
+    ctx->owned.push_back(ctx->ticket);
     ctx->hist = dalloc<unsigned>((size_t)kRadix * std::max(ctx->num_tiles, 1), e);
     ctx->num_tiles = blocks_for(ctx->n, kSortTile);
     ctx->dtotal = dalloc<unsigned>(kRadix, e);
@@ -875,6 +851,7 @@ armando_status alloc_state(armando_ctx* ctx) {
     }
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
     CK(cudaMemset(ctx->flags, 0, kFlagWords * sizeof(unsigned)));
+    CK(cudaMemset(ctx->ticket, 0, sizeof(unsigned)));
     cudaError_t he = cudaMallocHost((void**)&ctx->h_flags, kFlagWords * sizeof(unsigned));
     if (he != cudaSuccess) return cuda_fail(ctx, he, "cudaMallocHost");
     he = cudaMallocHost((void**)&ctx->h_grid, sizeof(DevGrid));
@@ -884,6 +861,38 @@ armando_status alloc_state(armando_ctx* ctx) {
         if (he == cudaSuccess) he = cudaMallocHost((void**)&ctx->h_ng, sizeof(int));
         if (he != cudaSuccess) return cuda_fail(ctx, he, "cudaMallocHost");
     }
+    return ARMANDO_OK;
+}
+
+void release(armando_ctx* c, void* p) {
+    if (!p) return;
+    auto it = std::find(c->owned.begin(), c->owned.end(), p);
+    if (it != c->owned.end()) c->owned.erase(it);
+    cudaFree(p);
+}
+
+// The cell table and the sort's counters (whole scan tiles) for `cap` cells.
+armando_status alloc_cells(armando_ctx* ctx, long long cap) {
+    const size_t tiles = (size_t)((cap + 1 + kScanTile - 1) / kScanTile);
+    release(ctx, ctx->start);
+    release(ctx, ctx->cell_cnt);
+    release(ctx, ctx->cell_sums);
+    cudaError_t e = cudaSuccess;
+    ctx->start = dalloc<int>((size_t)cap + 1, e);
+    ctx->cell_cnt = dalloc<int>(tiles * kScanTile, e);
+    ctx->cell_sums = dalloc<int>(tiles, e);
+    if (e == cudaSuccess)
+        e = cudaMemsetAsync(ctx->cell_cnt, 0, tiles * kScanTile * sizeof(int), ctx->stream);
+    if (e != cudaSuccess) {
+        for (int** q : {&ctx->start, &ctx->cell_cnt, &ctx->cell_sums}) {
+            if (*q) cudaFree(*q);
+            *q = nullptr;
+        }
+        return cuda_fail(ctx, e, "cudaMalloc(cell table)");
+    }
+    for (int* q : {ctx->start, ctx->cell_cnt, ctx->cell_sums}) ctx->owned.push_back(q);
+    ctx->cell_cap = cap;
+    free_graphs(ctx);
     return ARMANDO_OK;
 }
 
@@ -905,17 +914,8 @@ armando_status plan_grid_batch(armando_ctx* ctx) {
         return fail(ctx, ARMANDO_ERR_GRID_OVERFLOW, "an instance's neighbour grid is too large or its periodic box shorter than 3 cells");
     long long cap = std::max<long long>(2LL * total, 4096);
     if (cap > (1LL << 30)) return fail(ctx, ARMANDO_ERR_GRID_OVERFLOW, "the batch's neighbour grids need more than 2^30 cells");
-    int bits = 1;
-    while ((1LL << bits) < cap) ++bits;
-    ctx->passes = (bits + 7) / 8;
-    ctx->cell_cap = cap;
-    cudaError_t e = cudaSuccess;
-    ctx->start = dalloc<int>((size_t)cap + 1, e);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(cell table)");
-    ctx->owned.push_back(ctx->start);
     CK(cudaMemsetAsync(ctx->flags, 0, sizeof(unsigned), st));
-    free_graphs(ctx);
-    return ARMANDO_OK;
+    return alloc_cells(ctx, cap);
 }
 
 armando_status plan_grid(armando_ctx* ctx) {
@@ -933,17 +933,8 @@ armando_status plan_grid(armando_ctx* ctx) {
     if (!g.ok) return fail(ctx, ARMANDO_ERR_GRID_OVERFLOW, "neighbour grid too large or periodic box shorter than 3 cells");
     long long cap = std::max<long long>(2LL * g.ncells, 4096);
     if (cap > (1LL << 30)) return fail(ctx, ARMANDO_ERR_GRID_OVERFLOW, "neighbour grid needs more than 2^30 cells");
-    int bits = 1;
-    while ((1LL << bits) < cap) ++bits;
-    ctx->passes = (bits + 7) / 8;
-    ctx->cell_cap = cap;
-    cudaError_t e = cudaSuccess;
-    ctx->start = dalloc<int>((size_t)cap + 1, e);
-    if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(cell table)");
-    ctx->owned.push_back(ctx->start);
     CK(cudaMemsetAsync(ctx->flags, 0, sizeof(unsigned), st));
-    free_graphs(ctx);
-    return ARMANDO_OK;
+    return alloc_cells(ctx, cap);
 }
 
 // The wall grid of a call with mirror ghosts: the walls do not move within
@@ -1183,22 +1174,8 @@ armando_status fit_cells_to_box(armando_ctx* ctx) {
     }
     if (cells <= ctx->cell_cap) return ARMANDO_OK;
     if (cells > (1LL << 30)) return fail(ctx, ARMANDO_ERR_GRID_OVERFLOW, "open-boundary box needs more than 2^30 cells");
-    auto it = std::find(ctx->owned.begin(), ctx->owned.end(), (void*)ctx->start);
-    if (it != ctx->owned.end()) ctx->owned.erase(it);
-    cudaFree(ctx->start);
-    cudaError_t e = cudaSuccess;
-    ctx->start = dalloc<int>((size_t)cells + 1, e);
-    if (e != cudaSuccess) {
-        ctx->start = nullptr;
-        return cuda_fail(ctx, e, "cudaMalloc(cell table)");
-    }
-    ctx->owned.push_back(ctx->start);
-    ctx->cell_cap = cells;
-    int bits = 1;
-    while ((1LL << bits) < cells) ++bits;
-    ctx->passes = (bits + 7) / 8;
-    free_graphs(ctx);
-    return ARMANDO_OK;
+    CK(cudaStreamSynchronize(ctx->stream));
+    return alloc_cells(ctx, cells);
 }
 
 // The output order of an open run: ascending serial number (survivors of the
@@ -1701,8 +1678,8 @@ armando_status save_tape(armando_ctx* ctx, int t) {
     const TapeSlot& T = ctx->tape[t];
     const int n = (int)ctx->n;
     cudaStream_t st = ctx->stream;
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     if (ctx->dim == 2)
         k_tape_save<2><<<blocks_for(n, 256), 256, 0, st>>>(ctx->B, skeys, perm, ctx->A.ap, T, n);
     else
@@ -2116,13 +2093,6 @@ armando_status armando_set_params(armando_ctx* ctx, const armando_params* params
 
 namespace {
 
-void release(armando_ctx* c, void* p) {
-    if (!p) return;
-    auto it = std::find(c->owned.begin(), c->owned.end(), p);
-    if (it != c->owned.end()) c->owned.erase(it);
-    cudaFree(p);
-}
-
 armando_status check_tuning(armando_ctx* ctx, const armando_tuning& t) {
     if (t.reach < 1 || t.reach > 3) return fail(ctx, ARMANDO_ERR_INVALID_ARG, "reach must be 1, 2 or 3");
     if (t.threads_per_particle != 1 && t.threads_per_particle != 2 && t.threads_per_particle != 4)
@@ -2155,8 +2125,10 @@ armando_status apply_tuning(armando_ctx* ctx, const armando_tuning& t) {
             if (st != ARMANDO_OK) return st;
         }
         CK(cudaStreamSynchronize(ctx->stream));
-        release(ctx, ctx->start);
-        ctx->start = nullptr;
+        for (int** q : {&ctx->start, &ctx->cell_cnt, &ctx->cell_sums}) {
+            release(ctx, *q);
+            *q = nullptr;
+        }
         for (const TapeSlot& T : ctx->tape)
             for (void* q : {(void*)T.xh, (void*)T.vm, (void*)T.vmin, (void*)T.rp, (void*)T.p,
                             (void*)T.itype, (void*)T.nmask, (void*)T.keys, (void*)T.perm,
@@ -2615,8 +2587,8 @@ armando_status armando_neighbours(armando_ctx* ctx, const float* x, const float*
     int L = ctx->dim == 2 ? launch_grid_and_sort<2>(ctx, nullptr, st)
                           : launch_grid_and_sort<3>(ctx, nullptr, st);
     ctx->next_its = 0;  // A now holds these positions, not a step's state
-    const unsigned* skeys = ctx->keys[ctx->passes & 1];
-    const int* perm = ctx->vals[ctx->passes & 1];
+    const unsigned* skeys = ctx->keys[1];
+    const int* perm = ctx->vals[1];
     k_reorder_xh<<<blocks_for(nn, 256), 256, 0, st>>>(ctx->A, perm, ctx->B, nn);
     if (ctx->dim == 2)
         k_count_nbrs<2><<<blocks_for(nn, 128), 128, 0, st>>>(ctx->B, skeys, ctx->start, ctx->grid, cnt, nn);

@@ -66,12 +66,16 @@ struct armando_ctx {
     StateB B{};
     unsigned* keys[2] = {nullptr, nullptr};
     int* vals[2] = {nullptr, nullptr};
+    // Cell sort: keys[0] the cells by slot, vals[0] the arrival numbers, placed the
+    // particles of each cell in order of arrival; keys[1] and vals[1] the sorted
+    // cells and the permutation. cell_cnt (zero between sorts), cell_sums: the scan.
+    int *placed = nullptr, *cell_cnt = nullptr, *cell_sums = nullptr;
+    unsigned* ticket = nullptr;  // k_bbox_grid
     unsigned* hist = nullptr;
     unsigned* dtotal = nullptr;
     int num_tiles = 0;
     int* start = nullptr;
     long long cell_cap = 0;
-    int passes = 0;
     float* bbox_part = nullptr;
     DevGrid* grid = nullptr;
     unsigned* flags = nullptr;
