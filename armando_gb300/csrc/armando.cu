@@ -302,6 +302,16 @@ void swap_state(armando_ctx* ctx) {
     ctx->acur ^= 1;
 }
 
+// The shear tensor (physical viscosity).
+template <int DIM>
+void launch_shear(armando_ctx* ctx, const unsigned* skeys, cudaStream_t st) {
+    const int n = (int)ctx->n_work, b = blocks_for(n, kPassThreads);
+    if (use_lists(ctx))
+        k_shear<DIM, true><<<b, kPassThreads, 0, st>>>(ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
+    else
+        k_shear<DIM, false><<<b, kPassThreads, 0, st>>>(ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
+}
+
 // Reorder/predictor and the pair passes.
 // reorder = false: the caller launched the reorder copy itself (the fused
 // predictor's step graph, where only iterations that sort need it).
@@ -325,8 +335,7 @@ int launch_passes(armando_ctx* ctx, const StepArgs& S, const int* rs, bool reord
         L += 2;
     }
     if (ctx->dp.visc) {
-        k_shear<DIM><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
-            ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
+        launch_shear<DIM>(ctx, skeys, st);
         ++L;
     }
     launch_force<DIM>(ctx, skeys, S);
@@ -578,8 +587,7 @@ int launch_step_phased(armando_ctx* ctx, const StepArgs& S, cudaEvent_t* ev) {
     cudaEventRecord(ev[4], st);
     L += 2;
     if (ctx->dp.visc) {
-        k_shear<DIM><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
-            ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
+        launch_shear<DIM>(ctx, skeys, st);
         ++L;
     }
     cudaEventRecord(ev[5], st);
@@ -678,8 +686,7 @@ int launch_overlapped_step(armando_ctx* ctx, const StepArgs& S, float* rho_out, 
     cudaEventRecord(ctx->ev_ovl[3], s2);
     L += 4;
     if (ctx->dp.visc) {
-        k_shear<DIM><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
-            ctx->B, skeys, ctx->start, ctx->grid, ctx->dp, n);
+        launch_shear<DIM>(ctx, skeys, st);
         ++L;
     }
     launch_force<DIM>(ctx, skeys, S);

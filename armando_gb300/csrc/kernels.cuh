@@ -2009,68 +2009,119 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
 // ---------------------------------------------------------------------------
 // Pass 1b: shear tensor (physical viscosity), every particle.
 // ---------------------------------------------------------------------------
-template <int DIM>
+// The sums M_ab = sum_j m_j/rho_j G (v_j - v_i)_a (x_i - x_j)_b give the tensor
+// T_ab = M_ab + M_ba - (2/3) delta_ab tr M once per particle (internal_force.f:
+// 75-171 forms it per pair). Listed particles (LST) walk their lists; the others
+// collect the cells' candidates that pass the pair test in s_list. A cell walk of
+// its own, with divisions and a square root per pair in the branch of the test,
+// took 23.8 us at 26,880 particles; the lists' walk 11.
+template <int DIM, bool LST = false>
 __device__ __forceinline__ void shear_body(const StateB& B, const unsigned* __restrict__ keys,
                                            const int* __restrict__ start, const DevGrid& g,
-                                           const DevParams& P, const int s, const bool valid) {
-    if (!valid || !g.ok) return;
-    const float4 xi = B.xh[s];
-    const float4 vi = B.vm[s];
-    const float rhoi = B.rp[s].x;
-    const CellCoord cc = decode_key<DIM>(keys[s], g);
-    const float ihf = __frcp_rn(xi.w);
-    const float kgih_i = __fmul_rn(P.kg, pow_grad<DIM>(ihf));
-    float t[6] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f};  // xx yy zz xy xz yz
-    const int it_i = B.itype[s];
-    for_candidates<DIM>(g, start, cc, [&](int k) {
-        if (k == s) return;
-        if (P.wall_model == 1 && __ldg(B.itype + k) != it_i) return;  // push only
-        const float4 xj = __ldg(B.xh + k);
-        float d[3], dr2;
-        if (!pair_delta<DIM>(xi, xj, g, d, dr2)) return;
-        refine_periodic<DIM>(xi, xj, g, d, dr2);
-        const float4 vj = __ldg(B.vm + k);
-        const float mj = mass_of<DIM>(xj, vj);
-        const float rhoj = __ldg(&B.rp[k].x);
-        float ih = ihf, kgih = kgih_i;
-        if (xj.w != xi.w) {
-            ih = __frcp_rn(__fmul_rn(0.5f, __fadd_rn(xi.w, xj.w)));
-            kgih = __fmul_rn(P.kg, pow_grad<DIM>(ih));
+                                           const DevParams& P, const int s, const bool valid,
+                                           int (*s_list)[kPassThreads]) {
+    const int tid = threadIdx.x;
+    const bool work = valid && g.ok;
+    const int kself = valid ? s : 0;
+    float4 xi = make_float4(0.f, 0.f, 0.f, 1.f), vi = xi;
+    float rhoi = 1.f;
+    int it_i = 0;
+    if (work) {
+        xi = B.xh[s];
+        vi = B.vm[s];
+        rhoi = B.rp[s].x;
+        it_i = B.itype[s];
+    }
+    float m[DIM][DIM];
+#pragma unroll
+    for (int a = 0; a < DIM; ++a)
+#pragma unroll
+        for (int b = 0; b < DIM; ++b) m[a][b] = 0.f;
+    // Two entries; an absent one is the particle itself (d = 0, dv = 0). Beyond the
+    // support G = 0.
+    auto pair2 = [&](const int ka, const int kb) {
+        const float4 xa = __ldg(B.xh + ka), xb = __ldg(B.xh + kb);
+        const float4 va = __ldg(B.vm + ka), vb = __ldg(B.vm + kb);
+        f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
+        if (P.wall_model == 1) {  // push only
+            if (__ldg(B.itype + ka) != it_i) mj.x = 0.f;
+            if (__ldg(B.itype + kb) != it_i) mj.y = 0.f;
         }
-        const float gw = sph::wendland_grad_factor<DIM>(__fsqrt_rn(dr2), ih, kgih);
-        const float w0 = gw * d[0], w1 = gw * d[1], w2 = gw * d[2];
-        const float dv0 = vj.x - vi.x, dv1 = vj.y - vi.y, dv2 = (DIM == 3) ? vj.z - vi.z : 0.f;
-        float hxx, hyy, hzz = 0.f, hxy, hxz = 0.f, hyz = 0.f;
-        // explicit fused / unfused products: every instantiation rounds alike
-        const float e00 = __fmul_rn(dv0, w0), e11 = __fmul_rn(dv1, w1);
-        if (DIM == 2) {
-            hxx = fmaf(2.f, e00, -e11);
-            hyy = fmaf(2.f, e11, -e00);
-            hxy = fmaf(dv1, w0, __fmul_rn(dv0, w1));
-        } else {
-            const float e22 = __fmul_rn(dv2, w2);
-            hxx = fmaf(2.f, e00, -e11) - e22;
-            hyy = fmaf(2.f, e11, -e00) - e22;
-            hzz = fmaf(2.f, e22, -e00) - e11;
-            hyz = fmaf(dv2, w1, __fmul_rn(dv1, w2));
-            hxz = fmaf(dv2, w0, __fmul_rn(dv0, w2));
-            hxy = fmaf(dv1, w0, __fmul_rn(dv0, w1));
+        f2 d[3], dv[3];
+        d[0] = make_float2(xi.x - xa.x, xi.x - xb.x);
+        d[1] = make_float2(xi.y - xa.y, xi.y - xb.y);
+        dv[0] = make_float2(va.x - vi.x, vb.x - vi.x);
+        dv[1] = make_float2(va.y - vi.y, vb.y - vi.y);
+        if (g.periodic[0]) d[0] = min_image2(d[0], xi.x, xa.x, xb.x, g, 0);
+        if (g.periodic[1]) d[1] = min_image2(d[1], xi.y, xa.y, xb.y, g, 1);
+        f2 dr2 = fma2(d[1], d[1], fma2(d[0], d[0], bc2(kTinyDr2)));
+        if (DIM == 3) {
+            d[2] = make_float2(xi.z - xa.z, xi.z - xb.z);
+            dv[2] = make_float2(va.z - vi.z, vb.z - vi.z);
+            if (g.periodic[2]) d[2] = min_image2(d[2], xi.z, xa.z, xb.z, g, 2);
+            dr2 = fma2(d[2], d[2], dr2);
         }
-        const float c = mj / rhoj;
-        const float c23 = c * (2.f / 3.f);
-        t[0] = fmaf(c23, hxx, t[0]);
-        t[1] = fmaf(c23, hyy, t[1]);
-        t[2] = fmaf(c23, hzz, t[2]);
-        t[3] = fmaf(c, hxy, t[3]);
-        t[4] = fmaf(c, hxz, t[4]);
-        t[5] = fmaf(c, hyz, t[5]);
-    });
-    float q = fmaf(2.f * t[3], t[3], fmaf(t[1], t[1], __fmul_rn(t[0], t[0])));
-    if (DIM == 3) q = fmaf(2.f * t[4], t[4], fmaf(2.f * t[5], t[5], fmaf(t[2], t[2], q)));
+        const f2 ih = mul2(bc2(2.0f), rcp2(make_float2(xi.w + xa.w, xi.w + xb.w)));
+        const f2 ih2 = mul2(ih, ih);
+        f2 kg = mul2(bc2(P.kg), mul2(ih2, ih2));
+        if (DIM == 3) kg = mul2(kg, ih);
+        const f2 t = min2(fma2(mul2(dr2, rsqrt2(dr2)), ih, bc2(-2.0f)), 0.0f);
+        const f2 rj = rcp2(make_float2(__ldg(&B.rp[ka].x), __ldg(&B.rp[kb].x)));
+        const f2 c = mul2(mul2(mul2(mul2(t, t), t), kg), mul2(mj, rj));
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) {
+            const f2 u = mul2(c, dv[a]);
+#pragma unroll
+            for (int b = 0; b < DIM; ++b) m[a][b] = dot2(u, d[b], m[a][b]);
+        }
+    };
+    bool done = !work;
+    if (LST) {
+        const int lpk = work ? __ldg(B.ncount + s) : -1;
+        const int lc = lpk >= 0 ? list_near(lpk) + list_far(lpk) : -1;
+        const int cm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
+        for (int t = 0; t < cm; t += 2) {
+            const int ka = t < lc ? __ldg(B.nlist + (size_t)t * B.lstride + s) : kself;
+            const int kb = t + 1 < lc ? __ldg(B.nlist + (size_t)(t + 1) * B.lstride + s) : kself;
+            pair2(ka, kb);
+        }
+        if (lc >= 0) done = true;
+    }
+    if (__any_sync(0xffffffffu, !done)) {
+        CellCoord cc = {{0, 0, 0}};
+        if (!done) cc = decode_key<DIM>(keys[s], g);
+        Cursor cu = cursor_begin<DIM>(g);
+        while (__any_sync(0xffffffffu, !done)) {
+            int nl = 0;
+            while (!done && nl < cap_force<LST>()) {
+                if (cu.k >= cu.ke) {
+                    if (!cursor_next<DIM>(g, start, cc, cu)) done = true;
+                    continue;
+                }
+                const int k = cu.k++;
+                float d[3], dr2;
+                if (k != s && pair_delta<DIM>(xi, __ldg(B.xh + k), g, d, dr2)) s_list[nl++][tid] = k;
+            }
+            const int ml = __reduce_max_sync(0xffffffffu, nl);
+            for (int t = 0; t < ml; t += 2)
+                pair2(t < nl ? s_list[t][tid] : kself, t + 1 < nl ? s_list[t + 1][tid] : kself);
+        }
+    }
+    if (!work) return;
+    float tr = m[0][0] + m[1][1];
+    if (DIM == 3) tr += m[DIM - 1][DIM - 1];
+    const float c3 = (-2.f / 3.f) * tr;
+    const float txx = fmaf(2.f, m[0][0], c3), tyy = fmaf(2.f, m[1][1], c3);
+    const float tzz = DIM == 3 ? fmaf(2.f, m[DIM - 1][DIM - 1], c3) : 0.f;
+    const float txy = m[0][1] + m[1][0];
+    const float txz = DIM == 3 ? m[0][DIM - 1] + m[DIM - 1][0] : 0.f;
+    const float tyz = DIM == 3 ? m[1][DIM - 1] + m[DIM - 1][1] : 0.f;
+    float q = fmaf(2.f * txy, txy, fmaf(tyy, tyy, __fmul_rn(txx, txx)));
+    if (DIM == 3) q = fmaf(2.f * txz, txz, fmaf(2.f * tyz, tyz, fmaf(tzz, tzz, q)));
     B.tds[s] = 0.5f * P.eta / rhoi * q;
     const float sc = (P.pa_sph == 1) ? P.eta / (rhoi * rhoi) : P.eta;
-    B.tau[s] = make_float4(sc * t[0], sc * t[1], sc * t[3], sc * t[2]);
-    if (DIM == 3) B.tau2[s] = make_float4(sc * t[4], sc * t[5], 0.f, 0.f);
+    B.tau[s] = make_float4(sc * txx, sc * tyy, sc * txy, sc * tzz);
+    if (DIM == 3) B.tau2[s] = make_float4(sc * txz, sc * tyz, 0.f, 0.f);
 }
 
 // ---------------------------------------------------------------------------
@@ -2613,13 +2664,14 @@ __global__ void __launch_bounds__(kPassThreads)
     }
 }
 
-template <int DIM>
+template <int DIM, bool LST>
 __global__ void __launch_bounds__(kPassThreads)
     k_shear(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
             const DevGrid* __restrict__ gp, DevParams P, int n) {
+    __shared__ int s_list[cap_force<LST>()][kPassThreads];
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     const DevGrid g = *gp;
-    shear_body<DIM>(B, keys, start, g, P, s, s < n);
+    shear_body<DIM, LST>(B, keys, start, g, P, s, s < n, s_list);
 }
 
 template <int DIM, int TPP, int BS, bool PER, bool LEAN, bool OPT = false, bool LST = false,
@@ -2716,10 +2768,11 @@ __global__ void __launch_bounds__(kPassThreads)
     k_shear_batch(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
                   const DevGrid* __restrict__ grids, const DevParams* __restrict__ params,
                   const WorkItem* __restrict__ items, int n_items, int* __restrict__ queue) {
+    __shared__ int s_list[kListCap][kPassThreads];
     __shared__ ItemCtx c;
     while (next_item(c, items, n_items, queue, params, grids, nullptr)) {
         const int s = c.w.s0 + threadIdx.x;
-        if (c.P.visc) shear_body<DIM>(B, keys, start, c.g, c.P, s, s < c.w.s1);
+        if (c.P.visc) shear_body<DIM>(B, keys, start, c.g, c.P, s, s < c.w.s1, s_list);
     }
 }
 
