@@ -1681,6 +1681,11 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
     // The place of an absent entry: the particle itself, with no mass.
     int kself = valid ? s : 0;
     if (STG) kself = work ? s + SV.shift[DIM == 2 ? g.reach : g.reach * (2 * g.reach + 2)] : 0;
+    // The divisors of normalised density; 1 beyond the support, where a particle
+    // without density has no part.
+    auto rho_in = [&](const int ka, const int kb, const f2 t) {
+        return make_float2(t.x > 0.f ? __ldg(B.q + ka) : 1.f, t.y > 0.f ? __ldg(B.q + kb) : 1.f);
+    };
     // Two entries. NEAR: float-float weights on the exact pair difference, else
     // (2D) FP32 weights, the pair's r and q rounded once. The kernel is zero beyond
     // its support, so entries in a list's skin margin need no pair test.
@@ -1748,7 +1753,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                 const ff2 m = UNI ? mul_ff2_f(f, mj) : mul_ff2(f, cm);
                 acc_ff2(Sh, Sl, m);
                 if ((PH & 4) && nor)
-                    acc_ff2(Wh, Wl, mul_ff2(m, recip_ff2(make_float2(__ldg(B.q + ka), __ldg(B.q + kb)))));
+                    acc_ff2(Wh, Wl, mul_ff2(m, recip_ff2(rho_in(ka, kb, t))));
             }
         } else {
             // With uniform h and m every pair would share the rounding of K m / h^dim
@@ -1768,7 +1773,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                 const f2 m = UNI ? mul2(mj, f) : fma2(cm.hi, f, mul2(cm.lo, f));
                 acc_ff2(Sh, Sl, m);
                 if ((PH & 4) && nor)
-                    acc_ff2(Wh, Wl, mul2(m, rcp2(make_float2(__ldg(B.q + ka), __ldg(B.q + kb)))));
+                    acc_ff2(Wh, Wl, mul2(m, rcp2(rho_in(ka, kb, t))));
             }
         }
         if ((PH & 1) && need_div) {  // art_heat.f:46-67: grad W = kg (q - 2)^3 d = -8 kg t^3 d
@@ -2066,7 +2071,7 @@ __device__ __forceinline__ void shear_body(const StateB& B, const unsigned* __re
         f2 kg = mul2(bc2(P.kg), mul2(ih2, ih2));
         if (DIM == 3) kg = mul2(kg, ih);
         const f2 t = min2(fma2(mul2(dr2, rsqrt2(dr2)), ih, bc2(-2.0f)), 0.0f);
-        const f2 rj = rcp2(make_float2(__ldg(&B.rp[ka].x), __ldg(&B.rp[kb].x)));
+        const f2 rj = within2(t, rcp2(make_float2(__ldg(&B.rp[ka].x), __ldg(&B.rp[kb].x))));
         const f2 c = mul2(mul2(mul2(mul2(t, t), t), kg), mul2(mj, rj));
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
@@ -2185,7 +2190,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         }
     }
     const bool work = valid && it > 0 && g.ok;
-    const float ihf = __frcp_rn(xi.w);
+    const float ihf = DIM == 2 ? __fdividef(1.0f, xi.w) : __frcp_rn(xi.w);
     const float kgih_i = P.kg * pow_grad<DIM>(ihf);
     float4 ti = make_float4(0.f, 0.f, 0.f, 0.f), ti2 = make_float4(0.f, 0.f, 0.f, 0.f);
     const bool visc = !LEAN && P.visc, heat_art = !LEAN && P.heat_art;
@@ -2221,7 +2226,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
                     float tt, float t, float ih, float& mj, float& p0, float& p1, float& p2) {
         if (__ldg(B.itype + k) == it) return;
         const float r = fast_sqrt_pos(dr2);
-        if (dr2 > 2.0f * kTinyDr2) {
+        if (dr2 > 2.0f * kTinyDr2 && t < 0.f) {
             const float w = 0.0625f * tt * tt * fmaf(2.0f, t, 5.0f);  // W / W(0)
             const float c2 = P.c0 * P.c0;
             float f;
@@ -2241,7 +2246,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     // Terms of two entries (pressure, viscosity, art_visc, art_heat, options).
     // va, vb: the neighbours' 2D {vx, vy, rho, P} (ra, rb unused) or 3D v and
     // {rho, P, u, psi}. No pair test: the kernel's gradient is zero beyond its
-    // support, so the entries in the skin margin add nothing.
+    // support, so the entries in the skin margin add nothing. P of a particle
+    // without density (no mass near it) is not finite, and a zero gradient times
+    // it no zero: within2 leaves the margin's P out.
     //
     // Pressure, art_visc and their energy rates share one factor per pair: with
     // s = m_j G (grad W = G d), T = P_i + P_j + Pi_ij and dv = v_j - v_i,
@@ -2250,6 +2257,11 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     // art_visc: Pi_ij = alpha c0 A + beta rho_bar A^2, A = mh (dv.d)+ / (rho_bar
     // (r^2 + (eta mh)^2)): one reciprocal, of rho_bar's and the distance's product,
     // serves both of its divisions, and (dv.d)+ = max(dv.d, 0) its condition.
+    // In 2D the pressure's products are rounded in the order of the written formula,
+    // m_j ((P_i + P_j) (G d)), and Pi_ij's terms added by themselves: the pressure terms
+    // nearly cancel in a column of water at rest, and with the shared factor their
+    // rounding moved 2,000 coordinates of a 2.03 M dam break by an ulp in 6 iterations,
+    // which then move dv/dt there by up to 8e-4.
     // The pass was bound by issue (62% of cycles) and its neighbours' loads: about 80
     // instructions an entry, 50 now. Measured: 2D lists (2.03 M dam break) 0.213 ->
     // 0.160 ms, 3D lists (8.78 M channel) 6.77 -> 4.41 ms, 2D cells (42 k) 17.6 -> 16.1 us.
@@ -2265,8 +2277,8 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         if (g.periodic[0]) d0 = min_image2(d0, xi.x, xa.x, xb.x, g, 0);
         if (g.periodic[1]) d1 = min_image2(d1, xi.y, xa.y, xb.y, g, 1);
         if (DIM == 3 && g.periodic[2]) d2 = min_image2(d2, xi.z, xa.z, xb.z, g, 2);
-        f2 dr2 = fma2(d1, d1, fma2(d0, d0, bc2(kTinyDr2)));
-        if (DIM == 3) dr2 = fma2(d2, d2, dr2);
+        const f2 dd0 = fma2(d0, d0, bc2(kTinyDr2));
+        const f2 dr2 = DIM == 2 ? add2(dd0, prod2(d1, d1)) : fma2(d2, d2, fma2(d1, d1, dd0));
         f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
         f2 ih = bc2(ihf), kg = bc2(kgih_i), hs = bc2(2.0f * xi.w);
         if (!UNI) {
@@ -2277,14 +2289,16 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             if (DIM == 3) kg = mul2(kg, ih);
         }
         const f2 r = mul2(dr2, rsqrt2(dr2));
-        const f2 t = min2(fma2(r, ih, bc2(-2.0f)), 0.0f);  // q - 2, 0 beyond the support
+        // q - 2, 0 beyond the support
+        const f2 t = min2(DIM == 2 ? add2(prod2(r, ih), bc2(-2.0f)) : fma2(r, ih, bc2(-2.0f)), 0.0f);
         const f2 tt = mul2(t, t);
         const f2 rhoj = DIM == 2 ? make_float2(va.z, vb.z) : make_float2(ra.x, rb.x);
         if ((PH & 4) && repulsive_walls(P)) {
             push(ka, xa, rhoj.x, d0.x, d1.x, d2.x, dr2.x, tt.x, t.x, ih.x, mj.x, a0, a1, a2);
             push(kb, xb, rhoj.y, d0.y, d1.y, d2.y, dr2.y, tt.y, t.y, ih.y, mj.y, a0, a1, a2);
         }
-        const f2 sm = mul2(mul2(tt, t), mul2(mj, kg));
+        const f2 gw = mul2(mul2(mul2(kg, t), t), t);  // G (2D)
+        const f2 sm = DIM == 2 ? mul2(mj, gw) : mul2(mul2(tt, t), mul2(mj, kg));
         const f2 vx = make_float2(va.x - vi.x, vb.x - vi.x), vy = make_float2(va.y - vi.y, vb.y - vi.y);
         const f2 vz = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : zero2;
         f2 vr = fma2(vy, d1, mul2(vx, d0));
@@ -2293,26 +2307,38 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         f2 T = DIM == 2 ? make_float2(rpi.y + va.w, rpi.y + vb.w) : make_float2(rpi.y + ra.y, rpi.y + rb.y);
         f2 sv = sm;  // the viscous terms' factor
         if (P.pa_sph != 1) {
-            const f2 irr = rcp2(mul2(bc2(rpi.x), rhoj));
+            f2 irr = rcp2(mul2(bc2(rpi.x), rhoj));
+            if (LST && (PH & 2)) irr = within2(t, irr);
             T = mul2(T, irr);
             sv = mul2(sv, irr);
         }
+        if (LST) T = within2(t, T);
         const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
         const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
                          : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);
         const f2 rc = rcp2(mul2(D, rs));
         const f2 A = mul2(max2(vr, 0.0f), rc);
-        T = fma2(A, UNI ? bc2(k_alpha * (2.0f * xi.w)) : mul2(bc2(k_alpha), hs), T);
-        if (k_beta != 0.f) T = fma2(mul2(mul2(A, A), rs), mul2(bc2(k_beta), hs2), T);
-        const f2 c = neg2(mul2(sm, T));
-        a0 = dot2(c, d0, a0);
-        a1 = dot2(c, d1, a1);
-        if (DIM == 3) a2 = dot2(c, d2, a2);
+        const f2 ka2 = UNI ? bc2(k_alpha * (2.0f * xi.w)) : mul2(bc2(k_alpha), hs);
+        f2 V = DIM == 2 ? mul2(A, ka2) : fma2(A, ka2, T);  // Pi_ij (3D: and T)
+        if (k_beta != 0.f) V = fma2(mul2(mul2(A, A), rs), mul2(bc2(k_beta), hs2), V);
+        const f2 c = neg2(mul2(sm, DIM == 2 ? add2(T, V) : V));
+        if (DIM == 2) {  // m_j ((-T) (G d)), then -(m_j Pi_ij) (G d)
+            const f2 w0 = mul2(gw, d0), w1 = mul2(gw, d1), fs = neg2(T), mv = neg2(mul2(mj, V));
+            const f2 h0 = mul2(fs, w0), h1 = mul2(fs, w1);
+            a0 = fmaf(mv.x, w0.x, fmaf(mj.x, h0.x, a0));
+            a1 = fmaf(mv.x, w1.x, fmaf(mj.x, h1.x, a1));
+            a0 = fmaf(mv.y, w0.y, fmaf(mj.y, h0.y, a0));
+            a1 = fmaf(mv.y, w1.y, fmaf(mj.y, h1.y, a1));
+        } else {
+            a0 = dot2(c, d0, a0);
+            a1 = dot2(c, d1, a1);
+            a2 = dot2(c, d2, a2);
+        }
         e_sum = dot2(c, vr, e_sum);
         if (cont) drho_s = dot2(neg2(sm), vr, drho_s);  // con_density, density.f:203-216
         if (sle2) {                                   // hsml.f:75-90
-            divh = fmaf(__fdiv_rn(sm.x, rhoj.x), vr.x, divh);
-            divh = fmaf(__fdiv_rn(sm.y, rhoj.y), vr.y, divh);
+            const f2 dq = within2(t, make_float2(__fdiv_rn(sm.x, rhoj.x), __fdiv_rn(sm.y, rhoj.y)));
+            divh = dot2(dq, vr, divh);
         }
         if (xsph) {  // av_vel.f:47-58: -eps m_j / rho_ij (v_i - v_j) W_ij, eps = 0.3
             const f2 ih2 = mul2(ih, ih);
@@ -2335,8 +2361,11 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
                 const f2 sxz = make_float2(ti2.x + ua.x, ti2.x + ub.x), syz = make_float2(ti2.y + ua.y, ti2.y + ub.y);
                 h0 = fma2(sxz, d2, h0);
                 h1 = fma2(syz, d2, h1);
-                a2 = dot2(sv, fma2(szz, d2, fma2(syz, d1, mul2(sxz, d0))), a2);
+                f2 h2 = fma2(szz, d2, fma2(syz, d1, mul2(sxz, d0)));
+                if (LST) h2 = within2(t, h2);
+                a2 = dot2(sv, h2, a2);
             }
+            if (LST) h0 = within2(t, h0), h1 = within2(t, h1);
             a0 = dot2(sv, h0, a0);
             a1 = dot2(sv, h1, a1);
         }
@@ -2352,7 +2381,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             const f2 ps = make_float2(rpi.w + qa.w, rpi.w + qb.w);
             const f2 lo = make_float2(ulo_i - __ldg(B.ulo + ka), ulo_i - __ldg(B.ulo + kb));
             const f2 du2 = add2(make_float2(rpi.z - qa.z, rpi.z - qb.z), lo);
-            ah_du = dot2(mul2(mul2(mul2(sm, dr2), mul2(ps, rh)), bc2(2.0f)), du2, ah_du);
+            f2 pr = mul2(ps, rh);
+            if (LST) pr = within2(t, pr);
+            ah_du = dot2(mul2(mul2(mul2(sm, dr2), pr), bc2(2.0f)), du2, ah_du);
         }
     };
     // The entries, two at a time, with every particle's h alike or not.

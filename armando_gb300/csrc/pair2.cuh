@@ -4,8 +4,8 @@
 // cycles of the FMA pipe but one issue slot. The neighbour passes were bound by
 // issue (a list entry's address, loads, comparisons and reciprocals share the
 // slots with its arithmetic), so their pair arithmetic runs on two entries at
-// once. Every operation below is an explicit rounding: all instantiations of a
-// pass round alike, whatever the compiler contracts elsewhere.
+// once. A packed product is fused with an addition that takes it (measured: also the
+// .rn forms), unlike the scalar __fmul_rn; prod2 keeps its own rounding.
 #pragma once
 
 namespace ag {
@@ -20,6 +20,16 @@ __device__ __forceinline__ f2 add2(f2 a, f2 b) { return __fadd2_rn(a, b); }
 __device__ __forceinline__ f2 sub2(f2 a, f2 b) { return __fadd2_rn(a, neg2(b)); }
 __device__ __forceinline__ f2 max2(f2 a, float b) { return make_float2(fmaxf(a.x, b), fmaxf(a.y, b)); }
 __device__ __forceinline__ f2 min2(f2 a, float b) { return make_float2(fminf(a.x, b), fminf(a.y, b)); }
+// Added to squared distances before a reciprocal square root: no effect on any
+// distance above 1e-15 times the unit, and a coincident pair (or a particle
+// with itself) gets r = 0 without a comparison.
+constexpr float kTinyDr2 = 1.0e-37f;
+// a b rounded, also where an addition takes it (for results above 1e-29).
+__device__ __forceinline__ f2 prod2(f2 a, f2 b) { return __ffma2_rn(a, b, make_float2(kTinyDr2, kTinyDr2)); }
+// v where t < 0, else 0 (also in place of an infinity or NaN).
+__device__ __forceinline__ f2 within2(f2 t, f2 v) {
+    return make_float2(t.x < 0.f ? v.x : 0.f, t.y < 0.f ? v.y : 0.f);
+}
 // acc + a.x b.x + a.y b.y, in that order (one rounding per term).
 __device__ __forceinline__ float dot2(f2 a, f2 b, float acc) { return fmaf(a.y, b.y, fmaf(a.x, b.x, acc)); }
 
@@ -88,11 +98,6 @@ __device__ __forceinline__ void acc_ff2(f2& hi, f2& lo, f2 x) {
     hi = s.hi;
     lo = add2(lo, s.lo);
 }
-
-// Added to squared distances before a reciprocal square root: no effect on any
-// distance above 1e-15 times the unit, and a coincident pair (or a particle
-// with itself) gets r = 0 without a comparison.
-constexpr float kTinyDr2 = 1.0e-37f;
 
 // sqrt: the hardware reciprocal square root and one Newton correction from the exact
 // residual a.hi - r^2 (relative error ~2^-44). 0 for a = 0.
