@@ -262,7 +262,10 @@ template <int DIM>
 int launch_build_list(armando_ctx* ctx, const int* rs, cudaStream_t st) {
     const int n = (int)ctx->n_work;
     const unsigned* skeys = ctx->keys[1];
-    if (ctx->dp.periodic[0] || ctx->dp.periodic[1] || ctx->dp.periodic[2])
+    if (ctx->prm.scheme != 0)  // (no periodic axes)
+        k_build_list<DIM, false, true><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
+            ctx->B, skeys, ctx->start, ctx->grid, n, rs);
+    else if (ctx->dp.periodic[0] || ctx->dp.periodic[1] || ctx->dp.periodic[2])
         k_build_list<DIM, true><<<blocks_for(n, kPassThreads), kPassThreads, 0, st>>>(
             ctx->B, skeys, ctx->start, ctx->grid, n, rs);
     else
@@ -408,7 +411,7 @@ armando_status build_lazy_graph(armando_ctx* ctx, const StepArgs& S, cudaGraphEx
         return fail_graph(e, "cudaStreamBeginCaptureToGraph(body)");
     body_cap = true;
     int body = launch_grid_and_sort<DIM>(ctx, nullptr, ctx->stream2,
-                                         ctx->prm.scheme == 0 && use_lists(ctx));
+                                         use_lists(ctx));
     // With the fused predictor only the iterations that sort copy the state
     // into cell order: the copy joins the body.
     const bool body_reorder = ctx->prm.scheme == 0 && fused(ctx);
@@ -451,23 +454,30 @@ int launch_gpuc_passes(armando_ctx* ctx, const StepArgs& S, const int* rs) {
     const int nm = ctx->materials.empty() ? ARMANDO_MAX_MATERIALS : (int)ctx->materials.size();
     const unsigned* skeys = ctx->keys[1];
     const int* perm = ctx->vals[1];
-    ctx->gs.xsort = rs ? ctx->xsort_buf : nullptr;
-    k_gpuc_gather<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, ctx->gs, ctx->d_mat, nm,
+    const bool lists = rs && use_lists(ctx);
+    GpucState& gs = ctx->gs;
+    gs.xsort = rs ? ctx->xsort_buf : nullptr;
+    gs.nlist = ctx->B.nlist;
+    gs.ncount = ctx->B.ncount;
+    gs.lstride = ctx->B.lstride;
+    gs.pass = ctx->B.nmask;  // at least a list's capacity of bits per particle
+    k_gpuc_gather<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->A, perm, gs, ctx->d_mat, nm,
                                                            ctx->flags, n, rs);
     static const float alphas[3] = {1.0f, 0.25f, 2.0f / 3.0f};
     for (int q = 0; q < 3; ++q) {
         const int cur = q & 1;
-        with_tuning(ctx->tune, false, false, false, false, [&](auto tpp, auto bs, auto, auto, auto, auto) {
+        with_tuning(ctx->tune, false, false, false, lists, [&](auto tpp, auto bs, auto, auto, auto, auto lst) {
             constexpr int T = decltype(tpp)::value, BSZ = decltype(bs)::value;
+            constexpr bool LST = decltype(lst)::value;
             const int blocks = blocks_for((int64_t)n * T, BSZ);
             if (ctx->prm.scheme == 1)
-                k_gpuc_stage<DIM, 1, T, BSZ><<<blocks, BSZ, 0, st>>>(
-                    ctx->gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
-                    ctx->flags, alphas[q], S.dt, n);
+                k_gpuc_stage<DIM, 1, T, BSZ, LST><<<blocks, BSZ, 0, st>>>(
+                    gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
+                    ctx->flags, alphas[q], S.dt, n, q);
             else
-                k_gpuc_stage<DIM, 2, T, BSZ><<<blocks, BSZ, 0, st>>>(
-                    ctx->gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
-                    ctx->flags, alphas[q], S.dt, n);
+                k_gpuc_stage<DIM, 2, T, BSZ, LST><<<blocks, BSZ, 0, st>>>(
+                    gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
+                    ctx->flags, alphas[q], S.dt, n, q);
         });
     }
     k_gpuc_scatter<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->gs, 1, ctx->A, n, ctx->grid,
@@ -479,7 +489,7 @@ int launch_gpuc_passes(armando_ctx* ctx, const StepArgs& S, const int* rs) {
 template <int DIM>
 int launch_gpuc_step(armando_ctx* ctx, const StepArgs& S, const int* rs) {
     const int L0 = rs ? launch_resort_begin(ctx) : 0;
-    const int L = launch_grid_and_sort<DIM>(ctx, rs, ctx->stream);
+    const int L = launch_grid_and_sort<DIM>(ctx, rs, ctx->stream, rs && use_lists(ctx));
     return L0 + L + launch_gpuc_passes<DIM>(ctx, S, rs);
 }
 
@@ -1252,19 +1262,19 @@ armando_status prepare_gpuc(armando_ctx* ctx) {
         g.v0 = dalloc<float4>(n, e);
         g.q0 = dalloc<float2>(n, e);
         for (int k = 0; k < 2; ++k) {
-            g.xw[k] = dalloc<float4>(n, e);
-            g.vw[k] = dalloc<float4>(n, e);
-            g.sw[k] = dalloc<float4>(n, e);
+            g.w0[k] = dalloc<float4>(n, e);
+            g.w1[k] = dalloc<float4>(n, e);
+            g.w2[k] = dalloc<float4>(n, e);
+            g.uw[k] = dalloc<float>(ctx->dim == 3 ? n : 1, e);
         }
         g.rates = dalloc<float4>(n, e);
-        g.itype = dalloc<int>(n, e);
         g.id = dalloc<int>(n, e);
         ctx->d_mat = dalloc<DevMaterial>(ARMANDO_MAX_MATERIALS, e);
         ctx->d_zones = dalloc<DevZones>(1, e);
-        for (void* q : {(void*)g.x0, (void*)g.v0, (void*)g.q0, (void*)g.xw[0], (void*)g.xw[1],
-                        (void*)g.vw[0], (void*)g.vw[1], (void*)g.sw[0], (void*)g.sw[1],
-                        (void*)g.rates, (void*)g.itype, (void*)g.id, (void*)ctx->d_mat,
-                        (void*)ctx->d_zones})
+        for (void* q : {(void*)g.x0, (void*)g.v0, (void*)g.q0, (void*)g.w0[0], (void*)g.w0[1],
+                        (void*)g.w1[0], (void*)g.w1[1], (void*)g.w2[0], (void*)g.w2[1],
+                        (void*)g.uw[0], (void*)g.uw[1], (void*)g.rates, (void*)g.id,
+                        (void*)ctx->d_mat, (void*)ctx->d_zones})
             ctx->owned.push_back(q);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(GPU-C state)");
         ctx->gs_ready = true;
@@ -2148,10 +2158,9 @@ armando_status apply_tuning(armando_ctx* ctx, const armando_tuning& t) {
     ctx->adj_ready = false;
     ctx->next_its = 0;  // the device state no longer belongs to the last call
     free_graphs(ctx);
-    // Neighbour lists for a lazily sorting CERN step with one lane per
-    // particle, allocated on first use and kept.
-    if (ctx->lists && lazy(ctx) && t.threads_per_particle == 1 && ctx->prm.scheme == 0 &&
-        !ctx->B.nlist && ctx->prm.wall_model != 3) {
+    // Neighbour lists for a lazily sorting step with one lane per particle,
+    // allocated on first use and kept.
+    if (ctx->lists && lazy(ctx) && t.threads_per_particle == 1 && !ctx->B.nlist && ctx->prm.wall_model != 3) {
         const int lcap = ctx->dim == 2 ? kListCap2 : kListCap3;
         cudaError_t e = cudaSuccess;
         int* nl = dalloc<int>((size_t)lcap * (size_t)std::max<int64_t>(ctx->cap, 1), e);

@@ -191,15 +191,14 @@ inline const int* resort_flags(armando_ctx* ctx) { return reinterpret_cast<const
 // Whether the context sorts lazily (a sort skin; one particle system).
 inline bool lazy(const armando_ctx* ctx) { return ctx->tune.skin > 0 && ctx->n_inst == 1; }
 
-// Neighbour lists: a lazily sorting CERN step with one lane per particle and
+// Neighbour lists: a lazily sorting step with one lane per particle and
 // the lists allocated (ensure_lists); the iterations between sorts then read
 // the lists instead of walking the cells.
 // Not in reverse mode: its iterations sort every time, and the adjoint passes
 // decode the neighbour bits that the density pass leaves only for particles
 // walking their cells.
 inline bool use_lists(const armando_ctx* ctx) {
-    return lazy(ctx) && ctx->tune.threads_per_particle == 1 && ctx->prm.scheme == 0 &&
-           ctx->B.nlist != nullptr && !ctx->reverse_run;
+    return lazy(ctx) && ctx->tune.threads_per_particle == 1 && ctx->B.nlist != nullptr && !ctx->reverse_run;
 }
 
 inline bool any_periodic(const DevParams& p) { return p.periodic[0] || p.periodic[1] || p.periodic[2]; }
@@ -216,7 +215,7 @@ inline bool step_options(const armando_params& p) {
 // reorder copy) and write the next state into the other buffer: lists, lean
 // physics, no step option.
 inline bool fused_wanted(const armando_ctx* ctx) {
-    return ctx->fuse_ok && use_lists(ctx) && lean_physics(ctx->dp) && !step_options(ctx->prm);
+    return ctx->fuse_ok && ctx->prm.scheme == 0 && use_lists(ctx) && lean_physics(ctx->dp) && !step_options(ctx->prm);
 }
 inline bool fused(const armando_ctx* ctx) { return fused_wanted(ctx) && ctx->A_alt.xh != nullptr; }
 

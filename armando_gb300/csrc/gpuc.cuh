@@ -19,9 +19,9 @@
 // the candidates of the step's cell grid against the start positions (kept
 // for the step anyway) and evaluates the physics at the stage's positions.
 //
-// State in cell order: the step's start (x0, v0, rho0/u0) and two working
-// copies {x, v, (rho, u, p, c)} that the stages ping-pong between; the last
-// stage's rates go out as dv/dt, de/dt.
+// State in cell order: the step's start (x0, v0, rho0/u0) and two working copies
+// that the stages ping-pong between, laid out so that a pair reads two float4s of
+// its neighbour in 2D and three in 3D; the last stage's rates go out as dv/dt, de/dt.
 #pragma once
 #include "kernels.cuh"
 
@@ -58,14 +58,57 @@ struct GpucState {
     float4* x0;    // {x, y, m, h} (2D) / {x, y, z, h} (3D) at the step's start
     float4* v0;    // {v, -} (2D) / {v, m} (3D)
     float2* q0;    // {rho, u} at the step's start
-    float4* xw[2];
-    float4* vw[2];
-    float4* sw[2];  // {rho, u, p, c}
+    // Working copies, 2D: w0 {x, y, vx, vy}, w1 {rho, p, m, itype's bits}, w2 {u, c, h, -}
+    //                 3D: w0 {x, y, z, m}, w1 {vx, vy, vz, itype's bits}, w2 {rho, p, c, h}
+    float4* w0[2];
+    float4* w1[2];
+    float4* w2[2];
+    float* uw[2];   // 3D: u
     float4* rates;  // {dv/dt, de/dt} of the last stage
-    int* itype;
     int* id;
     float4* xsort;  // lazy sorting: positions at the last sort (nullptr: every step sorts)
+    // Neighbour lists of the last sort (StateB's; entries within 2 h_i + skin in cursor
+    // order) and, per step, the entries in reach at the step's start: bit t % 32 of
+    // pass[(t / 32) * n + i].
+    const int* nlist;
+    const int* ncount;
+    int lstride;
+    unsigned* pass;
 };
+
+// One particle of a working copy.
+struct GpucPart {
+    float x[3], v[3], m, h, rho, u, p, c;
+    int it;
+};
+template <int DIM>
+__device__ __forceinline__ GpucPart gpuc_load(const GpucState& S, int w, int i) {
+    const float4 a = (w ? S.w0[1] : S.w0[0])[i], b = (w ? S.w1[1] : S.w1[0])[i];
+    const float4 c = (w ? S.w2[1] : S.w2[0])[i];
+    GpucPart q;
+    if (DIM == 2)
+        q = {{a.x, a.y, 0.f}, {a.z, a.w, 0.f}, b.z, c.z, b.x, c.x, b.y, c.y, __float_as_int(b.w)};
+    else
+        q = {{a.x, a.y, a.z}, {b.x, b.y, b.z}, a.w, c.w, c.x, (w ? S.uw[1] : S.uw[0])[i], c.y, c.z,
+             __float_as_int(b.w)};
+    return q;
+}
+template <int DIM>
+__device__ __forceinline__ void gpuc_store(const GpucState& S, int w, int i, const GpucPart& q) {
+    float4* a = w ? S.w0[1] : S.w0[0];
+    float4* b = w ? S.w1[1] : S.w1[0];
+    float4* c = w ? S.w2[1] : S.w2[0];
+    if (DIM == 2) {
+        a[i] = make_float4(q.x[0], q.x[1], q.v[0], q.v[1]);
+        b[i] = make_float4(q.rho, q.p, q.m, __int_as_float(q.it));
+        c[i] = make_float4(q.u, q.c, q.h, 0.f);
+    } else {
+        a[i] = make_float4(q.x[0], q.x[1], q.x[2], q.m);
+        b[i] = make_float4(q.v[0], q.v[1], q.v[2], __int_as_float(q.it));
+        c[i] = make_float4(q.rho, q.p, q.c, q.h);
+        (w ? S.uw[1] : S.uw[0])[i] = q.u;
+    }
+}
 
 // The EOS of one particle after its update (acpu.c:932-962 with the property
 // functions of acpu.c:560-870; ESS of Code/armando.cu:572-598 on absolute
@@ -162,10 +205,8 @@ __global__ void k_gpuc_gather(StateA A, const int* __restrict__ perm, GpucState 
     S.x0[s] = xh;
     S.v0[s] = vm;
     S.q0[s] = make_float2(rho, u);
-    S.xw[0][s] = xh;
-    S.vw[0][s] = vm;
-    S.sw[0][s] = make_float4(rho, u, p, c);
-    S.itype[s] = it;
+    gpuc_store<DIM>(S, 0, s, GpucPart{{xh.x, xh.y, DIM == 3 ? xh.z : 0.f}, {vm.x, vm.y, vm.z},
+                                      mass_of<DIM>(xh, vm), xh.w, rho, u, p, c, it});
     S.id[s] = A.id[j];
 }
 
@@ -176,22 +217,6 @@ template <int DIM>
 __device__ __forceinline__ void gpuc_kernel_norm(float h, float K, float& ih, float& alpha) {
     ih = __frcp_rn(h);
     alpha = DIM == 2 ? __fmul_rn(K, __fmul_rn(ih, ih)) : __fmul_rn(K, __fmul_rn(__fmul_rn(ih, ih), ih));
-}
-
-template <int DIM>
-__device__ __forceinline__ void gpuc_kernel(float r, float h, float ih, float alpha, float& w,
-                                            float& dwdr) {
-    const float q = __fdiv_rn(r, h);
-    w = 0.f;
-    dwdr = 0.f;
-    if (!(q < 2.f)) return;
-    float t = fmaf(-0.5f, q, 1.0f);
-    t = __fmul_rn(t, t);
-    t = __fmul_rn(t, t);
-    w = __fmul_rn(__fmul_rn(t, fmaf(2.0f, q, 1.0f)), alpha);
-    const float qm2 = q - 2.0f;
-    dwdr = __fmul_rn(__fmul_rn(__fmul_rn(0.625f, q), __fmul_rn(__fmul_rn(qm2, qm2), qm2)),
-                     __fmul_rn(alpha, ih));
 }
 
 // The smallest t with sqrt_rn(t) >= lim, so that sqrt_rn(r2) < lim exactly when
@@ -223,112 +248,199 @@ __host__ __device__ constexpr int gpuc_list_len() {
     return want * BS * 4 > 48 * 1024 ? 48 * 1024 / (4 * BS) : want;
 }
 
-// One RK3 stage: rates of every particle from working copy `cur`, update into
-// `nxt` (X0 + alpha (X + dt dX/dt - X0)), EOS. VAR 1: host path, 2: device.
+// One RK3 stage: rates of every particle from working copy `cur`, update into the
+// other (X0 + alpha (X + dt dX/dt - X0)), EOS. VAR 1: host path, 2: device.
 // TPP lanes per particle split its candidates (lane `sub` takes slots
 // k0 + sub, k0 + sub + TPP, ... of every cell range) and sum their rates with
-// an xor butterfly; lane 0 updates. TPP = 1 sums in candidate order. Each lane
-// first lists the candidates that pass the start-position test (in shared
-// memory, candidate order kept) and then evaluates the list, so the lanes of a
-// warp run the pair physics together instead of idling through candidates.
-template <int DIM, int VAR, int TPP = 1, int BS = kPassThreads>
-__global__ void __launch_bounds__(BS)
+// an xor butterfly; lane 0 updates. TPP = 1 sums in candidate order.
+// LST: between sorts the neighbours come from the lists of the last sort, whose
+// entries the step's first stage (stage 0) tests against the start positions;
+// its pass bits serve the other two. Without lists, and for particles whose list
+// overflowed, each lane lists the candidates that pass the start-position test
+// in shared memory (candidate order) and evaluates that list. Both evaluate two
+// neighbours at a time (pair2.cuh), each operation rounded as a single pair's in the
+// reference's order, divisions and square roots too (div2, sqrt2 in pair2.cuh).
+//
+// Issue and latency bound the stage (42-57% of cycles): it walked its cells three
+// times a step, with the divider's code five times a pair. Measured a stage,
+// 85,773 / 361,201 particles: 28.7 / 84.9 us walking the cells, 16.0 / 37.8 on lists
+// (10 / 23 us a sort to build them); 96 registers, so that five blocks of 128 fit.
+template <int DIM, int VAR, int TPP = 1, int BS = kPassThreads, bool LST = false>
+__global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
     k_gpuc_stage(GpucState S, int cur, const unsigned* __restrict__ keys,
                  const int* __restrict__ start, const DevGrid* __restrict__ gp, DevParams P,
                  const DevMaterial* __restrict__ mat, int n_mat, const DevZones* __restrict__ zones,
-                 unsigned* __restrict__ flags, float alpha, float dt, int n) {
-    const int i = blockIdx.x * (BS / TPP) + (int)threadIdx.x / TPP;
+                 unsigned* __restrict__ flags, float alpha, float dt, int n, int stage) {
+    static_assert(!LST || TPP == 1, "lists: one lane per particle");
+    const int i0 = blockIdx.x * (BS / TPP) + (int)threadIdx.x / TPP;
     const int sub = (TPP == 1) ? 0 : (int)(threadIdx.x & (TPP - 1));
-    if (i >= n) return;  // whole groups: the lanes of a particle share i
+    const bool valid = i0 < n;
+    const int i = valid ? i0 : n - 1;  // (a lane past the end repeats the last particle's walk)
     const DevGrid g = *gp;
-    // working copies picked without indexing the parameter arrays (no stack)
-    const float4* __restrict__ xc = cur ? S.xw[1] : S.xw[0];
-    const float4* __restrict__ vc = cur ? S.vw[1] : S.vw[0];
-    const float4* __restrict__ sc = cur ? S.sw[1] : S.sw[0];
-    float4* __restrict__ xo = cur ? S.xw[0] : S.xw[1];
-    float4* __restrict__ vo = cur ? S.vw[0] : S.vw[1];
-    float4* __restrict__ so = cur ? S.sw[0] : S.sw[1];
-    const float4 x0i = S.x0[i];
-    const float4 xi = xc[i], vi = vc[i], si = sc[i];
-    const int it = S.itype[i];
-    const float hi = x0i.w;
-    const float mi = (DIM == 2) ? x0i.z : S.v0[i].w;
-    const float r2_bound = sqrt_less_bound(__fmul_rn(2.0f, hi));
+    const float4* __restrict__ n0 = cur ? S.w0[1] : S.w0[0];
+    const float4* __restrict__ n1 = cur ? S.w1[1] : S.w1[0];
+    const float4* __restrict__ n2 = cur ? S.w2[1] : S.w2[0];
+    const GpucPart q = gpuc_load<DIM>(S, cur, i);
+    const float r2_bound = sqrt_less_bound(__fmul_rn(2.0f, q.h));
     float ih, kal;
-    gpuc_kernel_norm<DIM>(hi, P.kw_hi, ih, kal);
-    float w0, d0;
-    gpuc_kernel<DIM>(0.f, hi, ih, kal, w0, d0);
+    gpuc_kernel_norm<DIM>(q.h, P.kw_hi, ih, kal);
+    const float aih = __fmul_rn(kal, ih), dead = __fmul_rn(0.01f, q.h);
     // the device variant's own pressure term (armando.cu:483-485)
-    const float p_i = (VAR == 2) ? __fdiv_rn(si.z, __fmul_rn(si.x, si.x)) : 0.f;
+    const float p_i = (VAR == 2) ? __fdiv_rn(q.p, __fmul_rn(q.rho, q.rho)) : q.p;
     float rd = 0.f, a0 = 0.f, a1 = 0.f, a2 = 0.f;
-    auto pair = [&](int k) {
-        const float4 xk = __ldg(xc + k), vk = __ldg(vc + k);
-        const float4 sk = __ldg(sc + k);
-        const int itk = __ldg(S.itype + k);
-        const float dx = xi.x - xk.x, dy = xi.y - xk.y, dz = (DIM == 3) ? xi.z - xk.z : 0.f;
-        const float dr = __fsqrt_rn(fmaf(dz, dz, fmaf(dy, dy, __fmul_rn(dx, dx))));
-        if (dr < __fmul_rn(0.01f, hi)) return;  // dr := 100 h: W = dW/dr = 0 (acpu.c:379)
-        float w, dwdr;
-        gpuc_kernel<DIM>(dr, hi, ih, kal, w, dwdr);
-        const float mk = mass_of<DIM>(xk, vk);  // the working copies carry m and h
-        const float dvr = fmaf(dz, vi.z - vk.z, fmaf(dy, vi.y - vk.y, __fmul_rn(dx, vi.x - vk.x)));
-        const float rhoi = si.x, rhok = sk.x;
-        const float ir = __fdiv_rn(1.0f, dr);
-        float f = 0.f;  // times dW/dr along (x_i - x_k)/dr
-        const bool same = it == itk;
-        if (VAR == 1 || same) {
-            rd = fmaf(__fmul_rn(mk, dvr), __fmul_rn(dwdr, ir), rd);
-            if (VAR == 1)
-                f = __fmul_rn(mk, __fdiv_rn(-(si.z + sk.z), __fmul_rn(rhoi, rhok)));
-            else
-                f = __fmul_rn(mk, -(p_i + __fdiv_rn(sk.z, __fmul_rn(rhok, rhok))));
-            const float cs = __fdiv_rn(__fmul_rn(2.0f, si.w), rhoi + rhok);
-            rd = fmaf(__fmul_rn(mk, __fmul_rn(rhoi - rhok, cs)), dwdr, rd);
-            if (dvr < 0.f) {
-                const float sh = __fdiv_rn(__fmul_rn(dvr, hi), fmaf(0.01f * hi, hi, __fmul_rn(dr, dr)));
-                f = fmaf(mk, __fmul_rn(__fmul_rn(sh, cs), 0.03f), f);
-            }
-        }
-        float push = 0.f;
-        if (!same) {
-            if (VAR == 1)
-                push = __fmul_rn(__fdiv_rn(mk, mi + mk),
-                                 __fdiv_rn(__fmul_rn(__fmul_rn(0.02f, __fdiv_rn(w, w0)), __fmul_rn(si.w, sk.w)), dr));
-            else
-                push = __fmul_rn(__fdiv_rn(__fdiv_rn(__fmul_rn(__fmul_rn(0.5f, w), mk), rhok), xk.w),
-                                 __fmul_rn(sk.w, sk.w));
-        }
-        const float tot = __fmul_rn(fmaf(f, dwdr, push), ir);
-        a0 = fmaf(tot, dx, a0);
-        a1 = fmaf(tot, dy, a1);
-        if (DIM == 3) a2 = fmaf(tot, dz, a2);
+    // Push between particles of different itype (acpu.c:424-429; armando.cu:507-513).
+    auto push = [&](int k, float mk, float rhok, float ck3, float hk3, float dr, float qk) {
+        if (!(qk < 2.f)) return 0.f;
+        const float4 o = DIM == 2 ? __ldg(n2 + k) : make_float4(0.f, ck3, hk3, 0.f);
+        float t = fmaf(-0.5f, qk, 1.0f);
+        t = __fmul_rn(t, t);
+        t = __fmul_rn(t, t);
+        const float w = __fmul_rn(__fmul_rn(t, fmaf(2.0f, qk, 1.0f)), kal);
+        if (VAR == 1)
+            return __fmul_rn(__fdiv_rn(mk, q.m + mk),
+                             __fdiv_rn(__fmul_rn(__fmul_rn(0.02f, __fdiv_rn(w, kal)), __fmul_rn(q.c, o.y)), dr));
+        return __fmul_rn(__fdiv_rn(__fdiv_rn(__fmul_rn(__fmul_rn(0.5f, w), mk), rhok), o.z),
+                         __fmul_rn(o.y, o.y));
     };
-    if (g.ok) {
-        constexpr int ML = gpuc_list_len<DIM, TPP, BS>();
+    // Two neighbours; ina, inb: whether they count.
+    auto pair2 = [&](int ka, int kb, const float4& xa, const float4& xb, const float4& ya,
+                     const float4& yb, const float4& za, const float4& zb, bool ina, bool inb) {
+        const f2 d0 = make_float2(q.x[0] - xa.x, q.x[0] - xb.x), d1 = make_float2(q.x[1] - xa.y, q.x[1] - xb.y);
+        const f2 d2 = DIM == 3 ? make_float2(q.x[2] - xa.z, q.x[2] - xb.z) : bc2(0.f);
+        f2 r2 = fma2(d1, d1, fma2(d0, d0, bc2(kTinyDr2)));
+        if (DIM == 3) r2 = fma2(d2, d2, r2);
+        const f2 rs = rsqrt2(r2);
+        const f2 dr = sqrt2(r2, rs);
+        // dr < 0.01 h: dr := 100 h, W = dW/dr = 0 (acpu.c:379)
+        f2 mk = DIM == 2 ? make_float2(ya.z, yb.z) : make_float2(xa.w, xb.w);
+        // (the others' terms are left out by selects: they may be infinite or NaN)
+        ina = ina && !(dr.x < dead);
+        inb = inb && !(dr.y < dead);
+        mk.x = ina ? mk.x : 0.f;
+        mk.y = inb ? mk.y : 0.f;
+        const f2 ir = rcp2_rn(dr, rs);
+        // dW/dr = K/h^(dim+1) 5/8 q (q - 2)^3 (acpu.c:146-201)
+        const f2 qk = div2(dr, bc2(q.h), bc2(ih));
+        const f2 qm = min2(sub2(qk, bc2(2.0f)), 0.0f);
+        const f2 dw = mul2(mul2(mul2(bc2(0.625f), qk), mul2(mul2(qm, qm), qm)), bc2(aih));
+        f2 dvr;
+        if (DIM == 2) {
+            dvr = mul2(d0, make_float2(q.v[0] - xa.z, q.v[0] - xb.z));
+            dvr = fma2(d1, make_float2(q.v[1] - xa.w, q.v[1] - xb.w), dvr);
+        } else {
+            dvr = mul2(d0, make_float2(q.v[0] - ya.x, q.v[0] - yb.x));
+            dvr = fma2(d1, make_float2(q.v[1] - ya.y, q.v[1] - yb.y), dvr);
+            dvr = fma2(d2, make_float2(q.v[2] - ya.z, q.v[2] - yb.z), dvr);
+        }
+        const f2 rk = DIM == 2 ? make_float2(ya.x, yb.x) : make_float2(za.x, zb.x);
+        const f2 pk = DIM == 2 ? make_float2(ya.y, yb.y) : make_float2(za.y, zb.y);
+        const int ita = __float_as_int(ya.w), itb = __float_as_int(yb.w);
+        f2 ms = mk;  // the pairs that take the density, pressure and shock terms
+        if (VAR == 2) {
+            if (ita != q.it) ms.x = 0.f;
+            if (itb != q.it) ms.y = 0.f;
+        }
+        f2 f;
+        if (VAR == 1) {
+            f = div2(neg2(make_float2(q.p + pk.x, q.p + pk.y)), mul2(bc2(q.rho), rk));
+        } else {
+            const f2 pr = div2(pk, mul2(rk, rk));
+            f = neg2(make_float2(p_i + pr.x, p_i + pr.y));
+        }
+        f = mul2(ms, f);
+        const f2 cs = div2(bc2(__fmul_rn(2.0f, q.c)), make_float2(q.rho + rk.x, q.rho + rk.y));
+        f2 sh = div2(mul2(dvr, bc2(q.h)), fma2(bc2(0.01f * q.h), bc2(q.h), mul2(dr, dr)));
+        sh = mul2(mul2(sh, cs), bc2(0.03f));
+        f2 mq = ms;
+        if (!(dvr.x < 0.f)) mq.x = 0.f;
+        if (!(dvr.y < 0.f)) mq.y = 0.f;
+        f = fma2(mq, sh, f);
+        f2 ps = bc2(0.f);
+        if (ita != q.it && ina) ps.x = push(ka, mk.x, rk.x, za.z, za.w, dr.x, qk.x);
+        if (itb != q.it && inb) ps.y = push(kb, mk.y, rk.y, zb.z, zb.w, dr.y, qk.y);
+        f2 c1 = mul2(ms, dvr), c2 = mul2(dw, ir);
+        f2 c3 = mul2(ms, mul2(make_float2(q.rho - rk.x, q.rho - rk.y), cs));
+        if (!ina) c1.x = c3.x = f.x = 0.f;
+        if (!inb) c1.y = c3.y = f.y = 0.f;
+        rd = fmaf(c3.x, dw.x, fmaf(c1.x, c2.x, rd));
+        rd = fmaf(c3.y, dw.y, fmaf(c1.y, c2.y, rd));
+        const f2 tot = mul2(fma2(f, dw, ps), ir);
+        a0 = dot2(tot, d0, a0);
+        a1 = dot2(tot, d1, a1);
+        if (DIM == 3) a2 = dot2(tot, d2, a2);
+    };
+    const int lc = (LST && g.ok) ? list_near(__ldg(S.ncount + i)) : -1;
+    if (LST) prefetch_list_rows(S.nlist, S.lstride, i, lc);
+    const float4 x0i = S.x0[i];
+    // updateListHost's test on the step's start positions (unfused)
+    auto in_reach = [&](const float4& x0k) {
+        const float e0 = __fsub_rn(x0i.x, x0k.x), e1 = __fsub_rn(x0i.y, x0k.y);
+        float r2 = __fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1));
+        if (DIM == 3) {
+            const float e2 = __fsub_rn(x0i.z, x0k.z);
+            r2 = __fadd_rn(r2, __fmul_rn(e2, e2));
+        }
+        return r2 < r2_bound;
+    };
+    if (LST) {
+        constexpr int NB = DIM == 2 ? 4 : 2;
+        const int cm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
+        unsigned word = 0u;
+        for (int t0 = 0; t0 < cm; t0 += NB) {
+            if (t0 % 32 == 0) word = (stage != 0 && t0 < lc) ? S.pass[(size_t)(t0 / 32) * n + i] : 0u;
+            int kb[NB];
+            float4 xb[NB], yb[NB], zb[NB];
+#pragma unroll
+            for (int u = 0; u < NB; ++u)
+                kb[u] = t0 + u < lc ? __ldg(S.nlist + (size_t)(t0 + u) * S.lstride + i) : i;
+#pragma unroll
+            for (int u = 0; u < NB; ++u) {
+                xb[u] = __ldg(n0 + kb[u]);
+                yb[u] = __ldg(n1 + kb[u]);
+                zb[u] = DIM == 3 ? __ldg(n2 + kb[u]) : yb[u];
+            }
+            if (stage == 0) {  // the working positions are the start's
+#pragma unroll
+                for (int u = 0; u < NB; ++u)
+                    if (t0 + u < lc && in_reach(xb[u])) word |= 1u << ((t0 + u) % 32);
+                if (((t0 + NB) % 32 == 0 || t0 + NB >= lc) && t0 < lc && valid)
+                    S.pass[(size_t)(t0 / 32) * n + i] = word;
+            }
+            const unsigned w = word >> (t0 % 32);
+#pragma unroll
+            for (int u = 0; u < NB; u += 2)
+                pair2(kb[u], kb[u + 1], xb[u], xb[u + 1], yb[u], yb[u + 1], zb[u], zb[u + 1],
+                      (w >> u) & 1u, (w >> (u + 1)) & 1u);
+            if ((t0 + NB) % 32 == 0) word = 0u;
+        }
+    }
+    if (g.ok && (!LST || __any_sync(0xffffffffu, lc < 0))) {
+        constexpr int ML = LST ? kListCapLst : gpuc_list_len<DIM, TPP, BS>();
         __shared__ int s_list[ML][BS];
         const int tid = threadIdx.x;
         int nl = 0;
-        const CellCoord cc = decode_key<DIM>(keys[i], g);
-        Cursor cu = cursor_begin<DIM>(g);
-        while (cursor_next<DIM>(g, start, cc, cu))
-            for (int k = cu.k + sub; k < cu.ke; k += TPP) {
-                if (k == i) continue;
-                // updateListHost's test on the step's start positions
-                const float4 x0k = __ldg(S.x0 + k);
-                const float e0 = __fsub_rn(x0i.x, x0k.x), e1 = __fsub_rn(x0i.y, x0k.y);
-                float r2 = __fadd_rn(__fmul_rn(e0, e0), __fmul_rn(e1, e1));
-                if (DIM == 3) {
-                    const float e2 = __fsub_rn(x0i.z, x0k.z);
-                    r2 = __fadd_rn(r2, __fmul_rn(e2, e2));
-                }
-                if (!(r2 < r2_bound)) continue;
-                s_list[nl++][tid] = k;
-                if (nl == ML) {  // a full list: evaluate it and go on collecting
-                    for (int q = 0; q < ML; ++q) pair(s_list[q][tid]);
-                    nl = 0;
-                }
+        auto eval = [&](int cnt) {
+            for (int e = 0; e < cnt; e += 2) {
+                const int ka = s_list[e][tid], kb = e + 1 < cnt ? s_list[e + 1][tid] : i;
+                const float4 xa = __ldg(n0 + ka), xb = __ldg(n0 + kb), ya = __ldg(n1 + ka), yb = __ldg(n1 + kb);
+                const float4 za = DIM == 3 ? __ldg(n2 + ka) : ya, zb = DIM == 3 ? __ldg(n2 + kb) : yb;
+                pair2(ka, kb, xa, xb, ya, yb, za, zb, true, e + 1 < cnt);
             }
-        for (int q = 0; q < nl; ++q) pair(s_list[q][tid]);
+        };
+        if (!LST || lc < 0) {
+            const CellCoord cc = decode_key<DIM>(keys[i], g);
+            Cursor cu = cursor_begin<DIM>(g);
+            while (cursor_next<DIM>(g, start, cc, cu))
+                for (int k = cu.k + sub; k < cu.ke; k += TPP) {
+                    if (k == i || !in_reach(__ldg(S.x0 + k))) continue;
+                    s_list[nl++][tid] = k;
+                    if (nl == ML) {  // a full list: evaluate it and go on collecting
+                        eval(ML);
+                        nl = 0;
+                    }
+                }
+        }
+        eval(nl);
     }
     if (TPP > 1) {  // the particle's lanes reach this point together
         rd = group_sum<TPP>(rd);
@@ -337,16 +449,19 @@ __global__ void __launch_bounds__(BS)
         if (DIM == 3) a2 = group_sum<TPP>(a2);
         if (sub != 0) return;
     }
+    if (!valid) return;
     // the start state, read after the pair loop (not held in registers across it)
     const float4 v0i = S.v0[i];
     const float2 q0 = S.q0[i];
+    const int it = q.it;
+    const float4 xi = make_float4(q.x[0], q.x[1], q.x[2], 0.f);
     float wz = 0.f;
     if (it > 0) {  // updateLoadsHost: gravity over every fluid particle, then the zones
         float g0 = P.gravity[0], g1 = P.gravity[1], g2 = P.gravity[2];
         const int nl = __ldg(&zones->n_load);
 #pragma unroll 1
-        for (int q = 0; q < nl; ++q) {
-            const DevLoadZone* Z = zones->load + q;
+        for (int z = 0; z < nl; ++z) {
+            const DevLoadZone* Z = zones->load + z;
             if (!in_zone<DIM>(Z->lo, Z->hi, xi)) continue;
             g0 = __fadd_rn(g0, __ldg(&Z->g[0]));
             g1 = __fadd_rn(g1, __ldg(&Z->g[1]));
@@ -355,60 +470,55 @@ __global__ void __launch_bounds__(BS)
         }
         const int np = __ldg(&zones->n_fix);
 #pragma unroll 1
-        for (int q = 0; q < np; ++q) {  // pump zones: (vel - v) / tau (Code/armando.cu:1046-1055)
-            const DevFixZone* Z = zones->fix + q;
+        for (int z = 0; z < np; ++z) {  // pump zones: (vel - v) / tau (Code/armando.cu:1046-1055)
+            const DevFixZone* Z = zones->fix + z;
             const float tau = __ldg(&Z->tau);
             if (!(tau > 0.f) || !in_zone<DIM>(Z->lo, Z->hi, xi)) continue;
-            g0 = __fadd_rn(g0, __fdiv_rn(__fsub_rn(__ldg(&Z->v[0]), vi.x), tau));
-            g1 = __fadd_rn(g1, __fdiv_rn(__fsub_rn(__ldg(&Z->v[1]), vi.y), tau));
-            if (DIM == 3) g2 = __fadd_rn(g2, __fdiv_rn(__fsub_rn(__ldg(&Z->v[2]), vi.z), tau));
+            g0 = __fadd_rn(g0, __fdiv_rn(__fsub_rn(__ldg(&Z->v[0]), q.v[0]), tau));
+            g1 = __fadd_rn(g1, __fdiv_rn(__fsub_rn(__ldg(&Z->v[1]), q.v[1]), tau));
+            if (DIM == 3) g2 = __fadd_rn(g2, __fdiv_rn(__fsub_rn(__ldg(&Z->v[2]), q.v[2]), tau));
         }
         a0 += g0;
         a1 += g1;
         if (DIM == 3) a2 += g2;
     }
     // balanceEnergyHost on top of the loads' w
-    const float du = __fadd_rn(wz, __fdiv_rn(__fmul_rn(si.z, rd), __fmul_rn(si.x, si.x)));
+    const float du = __fadd_rn(wz, __fdiv_rn(__fmul_rn(q.p, rd), __fmul_rn(q.rho, q.rho)));
     S.rates[i] = make_float4(a0, a1, a2, du);
-    float4 xn = xi, vn = vi, sn = si;
+    GpucPart o = q;
     if (VAR == 2 || it != 0) {  // acpu.c:894 leaves itype 0 alone
-        xn.x = fmaf(alpha, fmaf(dt, vi.x, xi.x) - x0i.x, x0i.x);
-        xn.y = fmaf(alpha, fmaf(dt, vi.y, xi.y) - x0i.y, x0i.y);
-        if (DIM == 3) xn.z = fmaf(alpha, fmaf(dt, vi.z, xi.z) - x0i.z, x0i.z);
-        vn.x = fmaf(alpha, fmaf(dt, a0, vi.x) - v0i.x, v0i.x);
-        vn.y = fmaf(alpha, fmaf(dt, a1, vi.y) - v0i.y, v0i.y);
-        if (DIM == 3) vn.z = fmaf(alpha, fmaf(dt, a2, vi.z) - v0i.z, v0i.z);
-        float rho = fmaf(alpha, fmaf(dt, rd, si.x) - q0.x, q0.x);
-        const float u = fmaf(alpha, fmaf(dt, du, si.y) - q0.y, q0.y);
+        o.x[0] = fmaf(alpha, fmaf(dt, q.v[0], q.x[0]) - x0i.x, x0i.x);
+        o.x[1] = fmaf(alpha, fmaf(dt, q.v[1], q.x[1]) - x0i.y, x0i.y);
+        if (DIM == 3) o.x[2] = fmaf(alpha, fmaf(dt, q.v[2], q.x[2]) - x0i.z, x0i.z);
+        o.v[0] = fmaf(alpha, fmaf(dt, a0, q.v[0]) - v0i.x, v0i.x);
+        o.v[1] = fmaf(alpha, fmaf(dt, a1, q.v[1]) - v0i.y, v0i.y);
+        if (DIM == 3) o.v[2] = fmaf(alpha, fmaf(dt, a2, q.v[2]) - v0i.z, v0i.z);
+        o.rho = fmaf(alpha, fmaf(dt, rd, q.rho) - q0.x, q0.x);
+        o.u = fmaf(alpha, fmaf(dt, du, q.u) - q0.y, q0.y);
         const DevMaterial& M = mat[gpuc_material(it, n_mat, flags)];
-        if (VAR == 1 && it <= 0) {  // acpu.c:910-914
-            vn.x = v0i.x;
-            vn.y = v0i.y;
-            if (DIM == 3) vn.z = v0i.z;
-        }
+        auto keep_v = [&]() {
+            o.v[0] = v0i.x;
+            o.v[1] = v0i.y;
+            if (DIM == 3) o.v[2] = v0i.z;
+        };
+        if (VAR == 1 && it <= 0) keep_v();  // acpu.c:910-914
+        const float4 xn = make_float4(o.x[0], o.x[1], o.x[2], 0.f);
         const int nf = __ldg(&zones->n_fix);
 #pragma unroll 1
-        for (int q = 0; q < nf; ++q) {  // fix zones at the new position
-            const DevFixZone* Z = zones->fix + q;
+        for (int z = 0; z < nf; ++z) {  // fix zones at the new position
+            const DevFixZone* Z = zones->fix + z;
             if (__ldg(&Z->tau) > 0.f || !in_zone<DIM>(Z->lo, Z->hi, xn)) continue;  // pumps: above
-            vn.x = __ldg(&Z->v[0]);
-            vn.y = __ldg(&Z->v[1]);
-            if (DIM == 3) vn.z = __ldg(&Z->v[2]);
+            o.v[0] = __ldg(&Z->v[0]);
+            o.v[1] = __ldg(&Z->v[1]);
+            if (DIM == 3) o.v[2] = __ldg(&Z->v[2]);
         }
-        if (M.type == 0) {  // boundary materials keep their velocity
-            vn.x = v0i.x;
-            vn.y = v0i.y;
-            if (DIM == 3) vn.z = v0i.z;
-        }
-        float p = 0.f, c = si.w;
-        gpuc_eos(M, rho, u, p, c);
-        sn = make_float4(rho, u, p, c);
-        const float chk = xn.x + xn.y + xn.z + vn.x + vn.y + vn.z + rho + u + p;
+        if (M.type == 0) keep_v();  // boundary materials keep their velocity
+        o.p = 0.f;
+        gpuc_eos(M, o.rho, o.u, o.p, o.c);
+        const float chk = o.x[0] + o.x[1] + o.x[2] + o.v[0] + o.v[1] + o.v[2] + o.rho + o.u + o.p;
         if (!isfinite(chk)) atomicOr(flags, (unsigned)FLAG_NONFINITE);
     }
-    xo[i] = xn;
-    vo[i] = vn;
-    so[i] = sn;
+    gpuc_store<DIM>(S, cur ^ 1, i, o);
 }
 
 // The step's result back to A (cell order of this step, like the force pass).
@@ -421,8 +531,9 @@ __global__ void k_gpuc_scatter(GpucState S, int cur, StateA A, int n,
                                unsigned* __restrict__ flags = nullptr) {
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= n) return;
-    const float4 sv = (cur ? S.sw[1] : S.sw[0])[s];
-    const float4 xn = (cur ? S.xw[1] : S.xw[0])[s];
+    const GpucPart q = gpuc_load<DIM>(S, cur, s);
+    const float4 xn = DIM == 2 ? make_float4(q.x[0], q.x[1], q.m, q.h)
+                               : make_float4(q.x[0], q.x[1], q.x[2], q.h);
     if (S.xsort && gp && flags) {
         const float h2 = gp->half_skin2;
         const float4 xb = S.xsort[s];
@@ -431,12 +542,12 @@ __global__ void k_gpuc_scatter(GpucState S, int cur, StateA A, int n,
             atomicExch(flags + 2, 1u);
     }
     A.xh[s] = xn;
-    A.vm[s] = (cur ? S.vw[1] : S.vw[0])[s];
-    A.rho[s] = sv.x;
-    A.u[s] = sv.y;
-    A.p[s] = sv.z;
+    A.vm[s] = make_float4(q.v[0], q.v[1], q.v[2], DIM == 3 ? q.m : 0.f);
+    A.rho[s] = q.rho;
+    A.u[s] = q.u;
+    A.p[s] = q.p;
     A.ap[s] = S.rates[s];
-    A.itype[s] = S.itype[s];
+    A.itype[s] = q.it;
     A.id[s] = S.id[s];
 }
 

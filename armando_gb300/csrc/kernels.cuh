@@ -2643,7 +2643,8 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
 // later in the iteration). Until the next sort every particle stays within
 // half the skin of where it was binned, so every pair the exact test accepts
 // (r < h_i + h_j) on those iterations is in the list.
-template <int DIM, bool PER>
+// OWN (the GPU-C schemes): the candidates within 2 h_s + skin, all of them near.
+template <int DIM, bool PER, bool OWN = false>
 __global__ void __launch_bounds__(kPassThreads)
     k_build_list(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
                  const DevGrid* __restrict__ gp, int n, const int* __restrict__ resort = nullptr) {
@@ -2671,11 +2672,11 @@ __global__ void __launch_bounds__(kPassThreads)
                 if (k >= cu.ke || k == s) continue;
                 float d[3], dr2;
                 pair_delta<DIM>(xi, xb[u], g, d, dr2);
-                const float lim = __fmul_rn(__fadd_rn(__fadd_rn(xi.w, xb[u].w), g.skin), pad);
+                const float lim = __fmul_rn(__fadd_rn(__fadd_rn(xi.w, OWN ? xi.w : xb[u].w), g.skin), pad);
                 if (!(dr2 < __fmul_rn(lim, lim))) continue;
                 const float hs = xi.w + xb[u].w;  // the density pass's near test
                 const bool near =
-                    DIM == 3 || dr2 < (0.25f * list_near_q2() * list_near_q2()) * hs * hs;
+                    DIM == 3 || OWN || dr2 < (0.25f * list_near_q2() * list_near_q2()) * hs * hs;
                 if (cn + cf < B.lcap) B.nlist[(size_t)(near ? cn : B.lcap - 1 - cf) * B.lstride + s] = k;
                 if (near) ++cn;
                 else ++cf;

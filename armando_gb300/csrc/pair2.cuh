@@ -99,6 +99,25 @@ __device__ __forceinline__ void acc_ff2(f2& hi, f2& lo, f2 x) {
     lo = add2(lo, s.lo);
 }
 
+// ---- correctly rounded results (Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990): an estimate and the exact FMA residual of the
+// result, so the rounding differs from IEEE's at most where the exact value is within
+// 2^-21 ulp of a tie. For operands and results far from the overflow and underflow
+// limits (the estimates flush there).
+// a / b; y: an estimate of 1/b.
+__device__ __forceinline__ f2 div2(f2 a, f2 b, f2 y) {
+    const f2 q = mul2(a, y);
+    return fma2(fma2(neg2(b), q, a), y, q);
+}
+__device__ __forceinline__ f2 div2(f2 a, f2 b) { return div2(a, b, rcp2(b)); }
+// 1 / b.
+__device__ __forceinline__ f2 rcp2_rn(f2 b, f2 y) { return fma2(fma2(neg2(b), y, bc2(1.0f)), y, y); }
+// sqrt(a); y: an estimate of 1/sqrt(a).
+__device__ __forceinline__ f2 sqrt2(f2 a, f2 y) {
+    const f2 r = mul2(a, y);
+    return fma2(fma2(neg2(r), r, a), mul2(y, bc2(0.5f)), r);
+}
+
 // sqrt: the hardware reciprocal square root and one Newton correction from the exact
 // residual a.hi - r^2 (relative error ~2^-44). 0 for a = 0.
 __device__ __forceinline__ ff2 sqrt_ff2(ff2 a) {
