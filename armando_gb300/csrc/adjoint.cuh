@@ -179,65 +179,6 @@ static __global__ void k_adj_out(StateB B, const float* __restrict__ du_out, Adj
     vpart[s] = make_float4(vt.x, vt.y, vt.z, ub);
 }
 
-// Adjoint of the force and energy-rate terms of pair (i, j), i fluid:
-//   a_i  += -S d,   du_i += -S (w.d)/2,   S = m_j (P_i + P_j + Pi_ij) G(r),
-// d = x_i - x_j, w = vh_j - vh_i, Pi_ij the art_visc term (0 unless w.d > 0).
-// ab = {a_bar_i, du_bar_i}. Outputs cotangents on d and w, on P_i and P_j
-// (equal), on rho_i and rho_j (equal halves of rho_bar), and on alpha, beta, c0.
-struct PairAdj {
-    float db[3], wb[3];
-    float Pb, rb, al, be, c0;
-};
-
-template <int DIM>
-__device__ __forceinline__ void pair_adjoint(const float* d, const float* w, float dr2, float G,
-                                             float dGdr_r, float mh, float rho_bar, float Pi,
-                                             float Pj, float mj, const float4& ab,
-                                             const DevParams& P, PairAdj& o) {
-    float wd = w[0] * d[0] + w[1] * d[1];
-    float ad = ab.x * d[0] + ab.y * d[1];
-    if (DIM == 3) {
-        wd += w[2] * d[2];
-        ad += ab.z * d[2];
-    }
-    const float vr = -wd;  // (vh_i - vh_j) . (x_i - x_j)
-    float pv = 0.f, phi = 0.f, den = 1.f;
-    const bool av = P.visc_art && vr < 0.f;
-    if (av) {
-        den = dr2 + mh * mh * P.av_eta2;
-        phi = mh * vr / den;
-        pv = (P.av_beta * phi - P.av_alpha * P.c0) * phi / rho_bar;
-    }
-    const float T = Pi + Pj + pv;
-    const float Sv = mj * T * G;
-    const float Sb = -(ad + 0.5f * ab.w * wd);
-    const float abv[3] = {ab.x, ab.y, ab.z};
-    const float Gb = mj * T * Sb;
-#pragma unroll
-    for (int k = 0; k < DIM; ++k) {
-        o.db[k] = -Sv * (abv[k] + 0.5f * ab.w * w[k]) + Gb * dGdr_r * d[k];
-        o.wb[k] = -0.5f * Sv * ab.w * d[k];
-    }
-    const float Tb = mj * G * Sb;
-    o.Pb = Tb;
-    o.rb = o.al = o.be = o.c0 = 0.f;
-    if (av) {
-        const float pb = Tb;
-        const float phib = pb * (2.f * P.av_beta * phi - P.av_alpha * P.c0) / rho_bar;
-        o.rb = -0.5f * pb * pv / rho_bar;
-        o.al = -pb * P.c0 * phi / rho_bar;
-        o.be = pb * phi * phi / rho_bar;
-        o.c0 = -pb * P.av_alpha * phi / rho_bar;
-        const float vrb = phib * mh / den;
-        const float r2b = -phib * phi / den;
-#pragma unroll
-        for (int k = 0; k < DIM; ++k) {
-            o.wb[k] -= vrb * d[k];
-            o.db[k] += -vrb * w[k] + 2.f * r2b * d[k];
-        }
-    }
-}
-
 // Neighbours of a fluid particle in warp-converged rounds (same candidates and
 // pair test as the forward passes; 2D reuses the density pass's bit mask).
 template <int DIM>
@@ -346,28 +287,45 @@ __device__ __forceinline__ void shear_m(const float4& a, const float4& b, float4
     mb = b;
 }
 
-// Forward pair geometry shared by the adjoint gathers.
+// Forward geometry of two pairs shared by the adjoint gathers: differences, r^2, the
+// gradient factor G and G'(r)/r (0 for a coincident pair), h_i + h_j. An absent entry
+// is the particle itself: d = 0, and every cotangent below vanishes.
 template <int DIM>
-struct PairGeo {
-    float d[3], dr2, G, dGdr_r, mh;
+struct PairGeo2 {
+    f2 d[3], dr2, G, dG, hs;
 };
 
 template <int DIM>
-__device__ __forceinline__ void pair_geo(const float4& xi, const float4& xj, const DevGrid& g,
-                                         const DevParams& P, PairGeo<DIM>& pg) {
-    pair_delta<DIM>(xi, xj, g, pg.d, pg.dr2);
-    refine_periodic<DIM>(xi, xj, g, pg.d, pg.dr2);
-    const float ih = (xj.w == xi.w) ? __fdividef(1.0f, xi.w) : __fdividef(2.0f, xi.w + xj.w);
-    const float kgih = P.kg * pow_grad<DIM>(ih);
-    const float r = fast_sqrt_pos(pg.dr2);
-    const float t = r * ih - 2.0f;
-    pg.G = kgih * t * t * t;
-    pg.dGdr_r = r > 0.f ? 3.0f * kgih * ih * t * t / r : 0.f;
-    pg.mh = 0.5f * (xi.w + xj.w);
+__device__ __forceinline__ void pair_geo2(const float4& xi, const float4& xa, const float4& xb,
+                                          const DevGrid& g, const DevParams& P, PairGeo2<DIM>& o) {
+    o.d[0] = make_float2(xi.x - xa.x, xi.x - xb.x);
+    o.d[1] = make_float2(xi.y - xa.y, xi.y - xb.y);
+    o.d[2] = DIM == 3 ? make_float2(xi.z - xa.z, xi.z - xb.z) : bc2(0.f);
+    if (g.periodic[0]) o.d[0] = min_image2(o.d[0], xi.x, xa.x, xb.x, g, 0);
+    if (g.periodic[1]) o.d[1] = min_image2(o.d[1], xi.y, xa.y, xb.y, g, 1);
+    if (DIM == 3 && g.periodic[2]) o.d[2] = min_image2(o.d[2], xi.z, xa.z, xb.z, g, 2);
+    o.dr2 = fma2(o.d[1], o.d[1], fma2(o.d[0], o.d[0], bc2(kTinyDr2)));
+    if (DIM == 3) o.dr2 = fma2(o.d[2], o.d[2], o.dr2);
+    o.hs = make_float2(xi.w + xa.w, xi.w + xb.w);
+    const f2 ih = mul2(bc2(2.0f), rcp2(o.hs)), ih2 = mul2(ih, ih);
+    f2 kg = mul2(bc2(P.kg), mul2(ih2, ih2));
+    if (DIM == 3) kg = mul2(kg, ih);
+    const f2 rs = rsqrt2(o.dr2);
+    const f2 t = min2(fma2(mul2(o.dr2, rs), ih, bc2(-2.0f)), 0.0f);
+    const f2 kt = mul2(kg, mul2(t, t));
+    o.G = mul2(kt, t);
+    o.dG = mul2(mul2(kt, mul2(ih, bc2(3.0f))), rs);
+    if (!(o.dr2.x > 2.0f * kTinyDr2)) o.dG.x = 0.f;
+    if (!(o.dr2.y > 2.0f * kTinyDr2)) o.dG.y = 0.f;
 }
 
-template <int DIM>
-__global__ void __launch_bounds__(kPassThreads)
+// EXT: artificial heat or physical viscosity is on; without them their operands are
+// compiled out. The pair's two directions share one set of terms, on two neighbours
+// at a time, with two reciprocals a pair; formed apart, with nine divisions each, they
+// took 152 us at 260,904 particles (2D), now 71; EXT's operands are what
+// held it to three blocks an SM.
+template <int DIM, bool EXT>
+__global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
     k_adj_force(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
                 const DevGrid* __restrict__ gp, DevParams P, StepArgs S,
                 const float4* __restrict__ abar, const float* __restrict__ pbar_loss,
@@ -380,8 +338,8 @@ __global__ void __launch_bounds__(kPassThreads)
     const int s = blockIdx.x * blockDim.x + tid;
     const bool valid = s < n;
     const DevGrid g = *gp;
-    const bool ah = P.heat_art != 0;
-    const bool vs = P.visc != 0;
+    const bool ah = EXT && P.heat_art != 0;
+    const bool vs = EXT && P.visc != 0;
     const int it = valid ? B.itype[s] : 0;
     const bool work = valid && g.ok && it > 0;
     // walls take part for artificial heat (their psi enters their neighbours'
@@ -406,10 +364,14 @@ __global__ void __launch_bounds__(kPassThreads)
         tai = B.tau[s];
         if (DIM == 3) tbi = B.tau2[s];
     }
-    float xb[3] = {0.f, 0.f, 0.f}, vb[3] = {0.f, 0.f, 0.f}, Pb = 0.f, rb = 0.f;
-    float psib = 0.f, uhb = 0.f;  // artificial heat: psi_bar, u_half_bar of this particle
-    // parameter cotangents, float-float (hi in pa, rounding residuals in palo):
-    // pair terms of both signs cancel in these sums
+    const f2 z2 = bc2(0.f);
+    f2 xb2[3] = {z2, z2, z2}, vb2[3] = {z2, z2, z2}, Pb2 = z2, rb2 = z2;
+    f2 psib2 = z2, uhb2 = z2;  // artificial heat: psi_bar, u_half_bar of this particle
+    // Sums of the art_visc parameters' cotangents, float-float (pair terms of both
+    // signs cancel): X = sum T_bar phi / rho_bar, Y = sum T_bar phi^2 / rho_bar;
+    // alpha_bar = -c0 X, beta_bar = Y, c0_bar gains -alpha X.
+    f2 Xh = z2, Xl = z2, Yh = z2, Yl = z2;
+    // per-particle terms, float-float (hi in pa, rounding residuals in palo)
     float pa[ADJ_NPARAM] = {0.f, 0.f, 0.f, 0.f}, palo[ADJ_NPARAM] = {0.f, 0.f, 0.f, 0.f};
     auto pacc = [&](int q, float v) {
         const sph::ff t = sph::two_sum(pa[q], v);
@@ -418,102 +380,148 @@ __global__ void __launch_bounds__(kPassThreads)
     };
     NbrStream<DIM> ns;
     nbr_init<DIM>(ns, B, g, s, act, work);
+    const int kself = valid ? s : 0;
     while (__any_sync(0xffffffffu, !ns.done)) {
         const int nl = nbr_fill<DIM>(ns, B, g, start, cc, xi, s, s_list);
         const int ml = __reduce_max_sync(0xffffffffu, nl);
-        for (int t = 0; t < ml; ++t) {
-            if (t >= nl) continue;
-            const int j = s_list[t][tid];
-            const float4 xj = __ldg(B.xh + j);
-            const float4 vj = __ldg(B.vm + j);
-            const float4 rpj = __ldg(B.rp + j);
-            const float4 abj = __ldg(abar + j);
-            const float mj = mass_of<DIM>(xj, vj);
-            PairGeo<DIM> pg;
-            pair_geo<DIM>(xi, xj, g, P, pg);
-            const float rho_bar = 0.5f * (rpi.x + rpj.x);
-            float w[3] = {vj.x - vi.x, vj.y - vi.y, DIM == 3 ? vj.z - vi.z : 0.f};
-            PairAdj o;
+        for (int t = 0; t < ml; t += 2) {
+            const int ja = t < nl ? s_list[t][tid] : kself, jb = t + 1 < nl ? s_list[t + 1][tid] : kself;
+            const float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            const float4 va = __ldg(B.vm + ja), vb = __ldg(B.vm + jb);
+            const float4 ra = __ldg(B.rp + ja), rb = __ldg(B.rp + jb);
+            const float4 ca = __ldg(abar + ja), cb = __ldg(abar + jb);
+            const f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
+            PairGeo2<DIM> pg;
+            pair_geo2<DIM>(xi, xa, xb, g, P, pg);
+            const f2 rs = make_float2(rpi.x + ra.x, rpi.x + rb.x);  // 2 rho_bar
+            const f2 w0 = make_float2(va.x - vi.x, vb.x - vi.x), w1 = make_float2(va.y - vi.y, vb.y - vi.y);
+            const f2 w2 = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : z2;
+            // The rates of s and of j from the pair: with d = x_s - x_j, w = v_j - v_s,
+            // T = P_s + P_j + Pi_sj,
+            //   a_s -= m_j T G d, du_s -= m_j T G (w.d)/2, a_j += m_s T G d, du_j likewise:
+            // their cotangents enter as A = m_j a_bar_s - m_s a_bar_j and
+            // b = m_j du_bar_s + m_s du_bar_j, S_bar = -(A.d + b (w.d)/2) on T G.
+            f2 A0 = fma2(mj, bc2(abi.x), mul2(bc2(-mi), make_float2(ca.x, cb.x)));
+            f2 A1 = fma2(mj, bc2(abi.y), mul2(bc2(-mi), make_float2(ca.y, cb.y)));
+            f2 A2 = DIM == 3 ? fma2(mj, bc2(abi.z), mul2(bc2(-mi), make_float2(ca.z, cb.z))) : z2;
             if (work) {
-                // Pair (s, j): the rates of s.
-                pair_adjoint<DIM>(pg.d, w, pg.dr2, pg.G, pg.dGdr_r, pg.mh, rho_bar, rpi.y, rpj.y,
-                                  mj, abi, P, o);
-#pragma unroll
-                for (int k = 0; k < DIM; ++k) {
-                    xb[k] += o.db[k];
-                    vb[k] -= o.wb[k];
+                const f2 hb = mul2(bc2(0.5f), fma2(mj, bc2(abi.w), mul2(bc2(mi), make_float2(ca.w, cb.w))));
+                f2 wd = fma2(w1, pg.d[1], mul2(w0, pg.d[0]));
+                f2 Ad = fma2(A1, pg.d[1], mul2(A0, pg.d[0]));
+                f2 ad = fma2(bc2(abi.y), pg.d[1], mul2(bc2(abi.x), pg.d[0]));
+                if (DIM == 3) {
+                    wd = fma2(w2, pg.d[2], wd);
+                    Ad = fma2(A2, pg.d[2], Ad);
+                    ad = fma2(bc2(abi.z), pg.d[2], ad);
                 }
-                Pb += o.Pb;
-                rb += o.rb;
-                pacc(ADJ_ALPHA, o.al);
-                pacc(ADJ_BETA, o.be);
-                pacc(ADJ_C0, o.c0);
-                // Pair (j, s): the rates of j (zero cotangents for walls).
-                if (abj.x != 0.f || abj.y != 0.f || abj.z != 0.f || abj.w != 0.f) {
-                    float dn[3] = {-pg.d[0], -pg.d[1], -pg.d[2]};
-                    float wn[3] = {-w[0], -w[1], -w[2]};
-                    pair_adjoint<DIM>(dn, wn, pg.dr2, pg.G, pg.dGdr_r, pg.mh, rho_bar, rpj.y,
-                                      rpi.y, mi, abj, P, o);
-#pragma unroll
-                    for (int k = 0; k < DIM; ++k) {
-                        xb[k] -= o.db[k];
-                        vb[k] += o.wb[k];
-                    }
-                    Pb += o.Pb;
-                    rb += o.rb;
+                const f2 Sb = neg2(fma2(hb, wd, Ad));
+                f2 T = make_float2(rpi.y + ra.y, rpi.y + rb.y);
+                f2 Tb = mul2(pg.G, Sb), rv = z2, r2b = z2;
+                if (P.visc_art) {  // Pi = (beta phi - alpha c0) phi / rho_bar, phi = mh vr / den, vr = -w.d < 0
+                    const f2 mh = mul2(pg.hs, bc2(0.5f));
+                    const f2 den = fma2(mul2(mh, mh), bc2(P.av_eta2), pg.dr2);
+                    const f2 rc = rcp2(mul2(den, rs));
+                    const f2 iden = mul2(rc, rs), irho = mul2(mul2(rc, den), bc2(2.0f));
+                    const f2 phi = mul2(mul2(mh, neg2(max2(wd, 0.0f))), iden);
+                    const f2 pf = mul2(phi, irho);
+                    const f2 pv = mul2(fma2(bc2(P.av_beta), phi, bc2(-P.av_alpha * P.c0)), pf);
+                    T = add2(T, pv);
+                    rb2 = fma2(mul2(bc2(-0.5f), Tb), mul2(pv, irho), rb2);
+                    f2 phib = mul2(mul2(Tb, irho), fma2(bc2(2.0f * P.av_beta), phi, bc2(-P.av_alpha * P.c0)));
+                    if (!(wd.x > 0.f)) phib.x = 0.f;
+                    if (!(wd.y > 0.f)) phib.y = 0.f;
+                    rv = mul2(mul2(phib, mh), iden);         // vr_bar
+                    r2b = mul2(mul2(phib, neg2(phi)), iden);  // (r^2)_bar
+                    // the parameters: the rates of s alone
+                    const f2 Ts = mul2(mul2(mj, pg.G), neg2(fma2(bc2(0.5f * abi.w), wd, ad)));
+                    const f2 x = mul2(Ts, pf);
+                    acc_ff2(Xh, Xl, x);
+                    acc_ff2(Yh, Yl, mul2(x, phi));
                 }
+                const f2 TG = mul2(T, pg.G), c = fma2(mul2(T, Sb), pg.dG, mul2(bc2(2.0f), r2b));
+                const f2 e = fma2(TG, hb, rv);  // on w: x_bar -= e w, and v_bar += e d
+                const f2 nTG = neg2(TG), ne = neg2(e);
+                xb2[0] = fma2(nTG, A0, fma2(ne, w0, fma2(c, pg.d[0], xb2[0])));
+                xb2[1] = fma2(nTG, A1, fma2(ne, w1, fma2(c, pg.d[1], xb2[1])));
+                vb2[0] = fma2(e, pg.d[0], vb2[0]);
+                vb2[1] = fma2(e, pg.d[1], vb2[1]);
+                if (DIM == 3) {
+                    xb2[2] = fma2(nTG, A2, fma2(ne, w2, fma2(c, pg.d[2], xb2[2])));
+                    vb2[2] = fma2(e, pg.d[2], vb2[2]);
+                }
+                Pb2 = add2(Pb2, Tb);
             }
             if (ah) {
-                // du_s and du_j terms m (psi_s + psi_j) A (u_s - u_j), A(r^2):
-                // weights du_bar_s m_j - du_bar_j m_s on the pair (s, j).
-                const float e = pg.mh * pg.mh * P.ah_eta2;
-                const float den = rho_bar * (e + pg.dr2);
-                const float A = pg.G * pg.dr2 / den;
-                const float dAds = (0.5f * pg.dGdr_r * pg.dr2 + pg.G) / den - A / (e + pg.dr2);
-                const float ps = rpi.w + rpj.w;
-                const float ulj = B.ulo ? __ldg(B.ulo + j) : 0.f;
-                const float du = (rpi.z - rpj.z) + (uloi - ulj);
-                const float cdu = abi.w * mj - abj.w * mi;
-                psib = fmaf(A * du, cdu, psib);
-                uhb = fmaf(ps * A, cdu, uhb);
-                rb -= 0.5f * ps * A * du * cdu / rho_bar;
-                const float cx = 2.f * dAds * ps * du * cdu;
+                // du_s and du_j terms m (psi_s + psi_j) A (u_s - u_j), A = G r^2 / (rho_bar
+                // (e + r^2)): weights du_bar_s m_j - du_bar_j m_s on the pair (s, j).
+                const f2 mh = mul2(pg.hs, bc2(0.5f));
+                const f2 den = fma2(mul2(mh, mh), bc2(P.ah_eta2), pg.dr2);
+                const f2 rc = rcp2(mul2(den, rs));
+                const f2 iden = mul2(rc, rs), irho = mul2(mul2(rc, den), bc2(2.0f));
+                const f2 q = mul2(iden, irho);  // 1 / (rho_bar den)
+                const f2 Ah = mul2(mul2(pg.G, pg.dr2), q);
+                const f2 dA = fma2(fma2(mul2(bc2(0.5f), pg.dG), pg.dr2, pg.G), q, neg2(mul2(Ah, iden)));
+                const f2 ps = make_float2(rpi.w + ra.w, rpi.w + rb.w);
+                f2 lo = z2;
+                if (B.ulo) lo = make_float2(uloi - __ldg(B.ulo + ja), uloi - __ldg(B.ulo + jb));
+                const f2 du = add2(make_float2(rpi.z - ra.z, rpi.z - rb.z), lo);
+                const f2 cdu = fma2(bc2(abi.w), mj, mul2(bc2(-mi), make_float2(ca.w, cb.w)));
+                const f2 Ac = mul2(Ah, cdu);
+                psib2 = fma2(Ac, du, psib2);
+                uhb2 = fma2(ps, Ac, uhb2);
+                rb2 = fma2(mul2(bc2(-0.5f), mul2(ps, Ac)), mul2(du, irho), rb2);
+                const f2 cx = mul2(mul2(mul2(bc2(2.0f), dA), mul2(ps, du)), cdu);
 #pragma unroll
-                for (int k = 0; k < DIM; ++k) xb[k] = fmaf(cx, pg.d[k], xb[k]);
+                for (int k = 0; k < DIM; ++k) xb2[k] = fma2(cx, pg.d[k], xb2[k]);
             }
             if (vs) {
                 // a_s += m_j (tau_s + tau_j) w, a_j += m_s (tau_j + tau_s) (-w), w = G d:
-                // cotangent b = m_j a_bar_s - m_s a_bar_j on (tau_s + tau_j) w.
-                const float4 taj = __ldg(B.tau + j);
-                float4 tbj = make_float4(0.f, 0.f, 0.f, 0.f);
-                if (DIM == 3) tbj = __ldg(B.tau2 + j);
-                const float bv[3] = {mj * abi.x - mi * abj.x, mj * abi.y - mi * abj.y,
-                                     DIM == 3 ? mj * abi.z - mi * abj.z : 0.f};
-                const float w0 = pg.G * pg.d[0], w1 = pg.G * pg.d[1];
-                const float w2 = (DIM == 3) ? pg.G * pg.d[2] : 0.f;
-                tba.x = fmaf(bv[0], w0, tba.x);
-                tba.y = fmaf(bv[1], w1, tba.y);
-                tba.z += bv[0] * w1 + bv[1] * w0;
+                // cotangent A on (tau_s + tau_j) w.
+                const float4 ta = __ldg(B.tau + ja), tb = __ldg(B.tau + jb);
+                float4 ua = make_float4(0.f, 0.f, 0.f, 0.f), ub = ua;
                 if (DIM == 3) {
-                    tba.w = fmaf(bv[2], w2, tba.w);
-                    tbb.x += bv[0] * w2 + bv[2] * w0;
-                    tbb.y += bv[1] * w2 + bv[2] * w1;
+                    ua = __ldg(B.tau2 + ja);
+                    ub = __ldg(B.tau2 + jb);
                 }
-                if (work) {  // d_bar = J u, u = (tau_s + tau_j) b, J = G I + (G'/r) d d^T
-                    const float4 sa = make_float4(tai.x + taj.x, tai.y + taj.y, tai.z + taj.z,
-                                                  tai.w + taj.w);
-                    const float4 sb = make_float4(tbi.x + tbj.x, tbi.y + tbj.y, 0.f, 0.f);
-                    float u[3];
-                    sym_apply<DIM>(sa, sb, bv, u);
-                    float du_ = u[0] * pg.d[0] + u[1] * pg.d[1];
-                    if (DIM == 3) du_ += u[2] * pg.d[2];
+                const float Av[2][3] = {{A0.x, A1.x, A2.x}, {A0.y, A1.y, A2.y}};
+                const float dv[2][3] = {{pg.d[0].x, pg.d[1].x, pg.d[2].x}, {pg.d[0].y, pg.d[1].y, pg.d[2].y}};
+                const float Gv[2] = {pg.G.x, pg.G.y}, dGv[2] = {pg.dG.x, pg.dG.y};
 #pragma unroll
-                    for (int k = 0; k < DIM; ++k)
-                        xb[k] += pg.G * u[k] + pg.dGdr_r * du_ * pg.d[k];
+                for (int e = 0; e < 2; ++e) {
+                    const float4 taj = e ? tb : ta, tbj = e ? ub : ua;
+                    const float* bv = Av[e];
+                    const float y0 = Gv[e] * dv[e][0], y1 = Gv[e] * dv[e][1], y2 = Gv[e] * dv[e][2];
+                    tba.x = fmaf(bv[0], y0, tba.x);
+                    tba.y = fmaf(bv[1], y1, tba.y);
+                    tba.z += bv[0] * y1 + bv[1] * y0;
+                    if (DIM == 3) {
+                        tba.w = fmaf(bv[2], y2, tba.w);
+                        tbb.x += bv[0] * y2 + bv[2] * y0;
+                        tbb.y += bv[1] * y2 + bv[2] * y1;
+                    }
+                    if (work) {  // d_bar = J u, u = (tau_s + tau_j) b, J = G I + (G'/r) d d^T
+                        const float4 sa = make_float4(tai.x + taj.x, tai.y + taj.y, tai.z + taj.z,
+                                                      tai.w + taj.w);
+                        const float4 sb = make_float4(tbi.x + tbj.x, tbi.y + tbj.y, 0.f, 0.f);
+                        float u[3];
+                        sym_apply<DIM>(sa, sb, bv, u);
+                        float du_ = u[0] * dv[e][0] + u[1] * dv[e][1];
+                        if (DIM == 3) du_ += u[2] * dv[e][2];
+#pragma unroll
+                        for (int k = 0; k < DIM; ++k) xb2[k].x += Gv[e] * u[k] + dGv[e] * du_ * dv[e][k];
+                    }
                 }
             }
         }
     }
+    float xb[3], vb[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        xb[k] = xb2[k].x + xb2[k].y;
+        vb[k] = vb2[k].x + vb2[k].y;
+    }
+    const float Pb = Pb2.x + Pb2.y, psib = psib2.x + psib2.y, uhb = uhb2.x + uhb2.y;
+    float rb = rb2.x + rb2.y;
     if (act && vs) {
         // tau = sc T, sc = eta / rho^2; du += tds = eta/(2 rho) T:T (fluid only).
         const float rho = rpi.x;
@@ -591,9 +599,14 @@ __global__ void __launch_bounds__(kPassThreads)
     if (valid && divsb) divsb[s] = dsb;
     // Deterministic per-block partial sums of the parameter cotangents, in
     // double (a fixed shuffle order, then the warps in order).
+    const double X = ((double)Xh.x + (double)Xh.y) + ((double)Xl.x + (double)Xl.y);
+    const double Y = ((double)Yh.x + (double)Yh.y) + ((double)Yl.x + (double)Yl.y);
 #pragma unroll
     for (int q = 0; q < ADJ_NPARAM; ++q) {
         double v = (double)pa[q] + (double)palo[q];
+        if (q == ADJ_ALPHA) v -= (double)P.c0 * X;
+        if (q == ADJ_BETA) v += Y;
+        if (q == ADJ_C0) v -= (double)P.av_alpha * X;
 #pragma unroll
         for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
         if ((tid & 31) == 0) s_red[q][tid >> 5] = v;
@@ -655,8 +668,11 @@ __global__ void __launch_bounds__(kPassThreads)
             float4 tbj = make_float4(0.f, 0.f, 0.f, 0.f);
             if (DIM == 3) tbj = __ldg(tbar2 + j);
             const float cj = mass_of<DIM>(xj, vj) / rhoj;
-            PairGeo<DIM> pg;
-            pair_geo<DIM>(xi, xj, g, P, pg);
+            PairGeo2<DIM> p2;
+            pair_geo2<DIM>(xi, xj, xj, g, P, p2);
+            struct {
+                float d[3], G, dGdr_r;
+            } pg = {{p2.d[0].x, p2.d[1].x, p2.d[2].x}, p2.G.x, p2.dG.x};
             const float w[3] = {pg.G * pg.d[0], pg.G * pg.d[1], DIM == 3 ? pg.G * pg.d[2] : 0.f};
             const float dv[3] = {vj.x - vi.x, vj.y - vi.y, DIM == 3 ? vj.z - vi.z : 0.f};
             const float4 Aa = make_float4(cj * tai.x + ci * taj.x, cj * tai.y + ci * taj.y,
@@ -729,39 +745,51 @@ __global__ void __launch_bounds__(kPassThreads)
     if (work) cc = decode_key<DIM>(keys[s], g);
     const bool ah = P.heat_art != 0 && divsb != nullptr;
     const float dsi = (work && ah) ? divsb[s] : 0.f;
-    float xb[3] = {0.f, 0.f, 0.f}, vdb[3] = {0.f, 0.f, 0.f};
+    const f2 z2 = bc2(0.f);
+    f2 xb2[3] = {z2, z2, z2}, vd2[3] = {z2, z2, z2};
     NbrStream<DIM> ns;
     nbr_init<DIM>(ns, B, g, s, work);
+    const int kself = valid ? s : 0;
     while (__any_sync(0xffffffffu, !ns.done)) {
         const int nl = nbr_fill<DIM>(ns, B, g, start, cc, xi, s, s_list);
         const int ml = __reduce_max_sync(0xffffffffu, nl);
-        for (int t = 0; t < ml; ++t) {
-            if (t >= nl) continue;
-            const int j = s_list[t][tid];
-            const float4 xj = __ldg(B.xh + j);
-            float4 vj = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (DIM == 3 || ah) vj = __ldg(B.vm + j);
-            const float mj = mass_of<DIM>(xj, vj);
-            const float rbj = __ldg(rhobar + j);
-            PairGeo<DIM> pg;
-            pair_geo<DIM>(xi, xj, g, P, pg);
-            const float c = (rbi * mj + rbj * mi) * pg.G;
+        for (int t = 0; t < ml; t += 2) {
+            const int ja = t < nl ? s_list[t][tid] : kself, jb = t + 1 < nl ? s_list[t + 1][tid] : kself;
+            const float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
+            if (DIM == 3 || ah) {
+                va = __ldg(B.vm + ja);
+                vb = __ldg(B.vm + jb);
+            }
+            const f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
+            PairGeo2<DIM> pg;
+            pair_geo2<DIM>(xi, xa, xb, g, P, pg);
+            const f2 c = mul2(fma2(bc2(rbi), mj, mul2(bc2(mi), make_float2(__ldg(rhobar + ja), __ldg(rhobar + jb)))),
+                              pg.G);
 #pragma unroll
-            for (int k = 0; k < DIM; ++k) xb[k] = fmaf(c, pg.d[k], xb[k]);
+            for (int k = 0; k < DIM; ++k) xb2[k] = fma2(c, pg.d[k], xb2[k]);
             if (ah) {
                 // d/d(vh_s), d/d(x_s) of divs_s (weight dsb_s m_j) and of divs_j
                 // (weight dsb_j m_s, d_js = -d, w_js = -w): the same forms.
-                const float cd = dsi * mj + __ldg(divsb + j) * mi;
-                const float w[3] = {vj.x - vi.x, vj.y - vi.y, DIM == 3 ? vj.z - vi.z : 0.f};
-                float wd = w[0] * pg.d[0] + w[1] * pg.d[1];
-                if (DIM == 3) wd += w[2] * pg.d[2];
+                const f2 cd = fma2(bc2(dsi), mj, mul2(bc2(mi), make_float2(__ldg(divsb + ja), __ldg(divsb + jb))));
+                const f2 w[3] = {make_float2(va.x - vi.x, vb.x - vi.x), make_float2(va.y - vi.y, vb.y - vi.y),
+                                 DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : z2};
+                f2 wd = fma2(w[1], pg.d[1], mul2(w[0], pg.d[0]));
+                if (DIM == 3) wd = fma2(w[2], pg.d[2], wd);
+                const f2 cg = mul2(cd, pg.G), ce = mul2(cd, mul2(pg.dG, wd));
 #pragma unroll
                 for (int k = 0; k < DIM; ++k) {
-                    vdb[k] = fmaf(-cd * pg.G, pg.d[k], vdb[k]);
-                    xb[k] = fmaf(cd, pg.G * w[k] + pg.dGdr_r * pg.d[k] * wd, xb[k]);
+                    vd2[k] = fma2(neg2(cg), pg.d[k], vd2[k]);
+                    xb2[k] = fma2(cg, w[k], fma2(ce, pg.d[k], xb2[k]));
                 }
             }
         }
+    }
+    float xb[3], vdb[3];
+#pragma unroll
+    for (int k = 0; k < 3; ++k) {
+        xb[k] = xb2[k].x + xb2[k].y;
+        vdb[k] = vd2[k].x + vd2[k].y;
     }
     if (!valid) return;
     float4 gx = make_float4(0.f, 0.f, 0.f, 0.f), gv = gx, ga = gx;

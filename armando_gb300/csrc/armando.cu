@@ -1719,7 +1719,8 @@ int launch_adjoint(armando_ctx* ctx, const StepArgs& S, const TapeSlot& T) {
     const StateB Bv = tape_view(ctx->B, T, n);
     k_adj_out<<<blocks_for(n, 256), 256, 0, st>>>(Bv, T.du, ctx->adjG, S, ctx->adj_abar,
                                                   ctx->adj_xpart, ctx->adj_vpart, n);
-    k_adj_force<DIM><<<nb, kPassThreads, 0, st>>>(Bv, T.keys, T.start, T.grid, ctx->dp, S,
+    auto force = ctx->dp.heat_art || ctx->dp.visc ? k_adj_force<DIM, true> : k_adj_force<DIM, false>;
+    force<<<nb, kPassThreads, 0, st>>>(Bv, T.keys, T.start, T.grid, ctx->dp, S,
                                                  ctx->adj_abar, ctx->adj_pbar, ctx->adj_rhobar,
                                                  ctx->adj_xF, ctx->adj_vhb, ctx->adj_divsb,
                                                  ctx->adj_tbar, ctx->adj_tbar2, ctx->adj_blk, n);
