@@ -2164,7 +2164,7 @@ armando_status apply_tuning(armando_ctx* ctx, const armando_tuning& t) {
     if (ctx->lists && lazy(ctx) && t.threads_per_particle == 1 && !ctx->B.nlist && ctx->prm.wall_model != 3) {
         const int lcap = ctx->dim == 2 ? kListCap2 : kListCap3;
         cudaError_t e = cudaSuccess;
-        int* nl = dalloc<int>((size_t)lcap * (size_t)std::max<int64_t>(ctx->cap, 1), e);
+        int* nl = dalloc<int>((size_t)list_blocks(lcap) * 4 * (size_t)std::max<int64_t>(ctx->cap, 1), e);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(neighbour lists)");
         ctx->owned.push_back(nl);
         int* nc = dalloc<int>((size_t)std::max<int64_t>(ctx->cap, 1), e);

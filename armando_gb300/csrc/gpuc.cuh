@@ -67,8 +67,8 @@ struct GpucState {
     float4* rates;  // {dv/dt, de/dt} of the last stage
     int* id;
     float4* xsort;  // lazy sorting: positions at the last sort (nullptr: every step sorts)
-    // Neighbour lists of the last sort (StateB's; entries within 2 h_i + skin in cursor
-    // order) and, per step, the entries in reach at the step's start: bit t % 32 of
+    // Neighbour lists of the last sort (StateB's blocks; entries within 2 h_i + skin in
+    // cursor order) and, per step, the entries in reach at the step's start: bit t % 32 of
     // pass[(t / 32) * n + i].
     const int* nlist;
     const int* ncount;
@@ -370,7 +370,7 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
         if (DIM == 3) a2 = dot2(tot, d2, a2);
     };
     const int lc = (LST && g.ok) ? list_near(__ldg(S.ncount + i)) : -1;
-    if (LST) prefetch_list_rows(S.nlist, S.lstride, i, lc);
+    if (LST) prefetch_list(S.nlist, S.lstride, i, lc);
     const float4 x0i = S.x0[i];
     // updateListHost's test on the step's start positions (unfused)
     auto in_reach = [&](const float4& x0k) {
@@ -383,35 +383,37 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
         return r2 < r2_bound;
     };
     if (LST) {
-        constexpr int NB = DIM == 2 ? 4 : 2;
-        const int cm = __reduce_max_sync(0xffffffffu, lc > 0 ? lc : 0);
+        constexpr int NB = DIM == 2 ? 4 : 2;  // entries whose loads issue together
+        const int nb = blocks_of(lc);
+        const int bm = __reduce_max_sync(0xffffffffu, nb);
         unsigned word = 0u;
-        for (int t0 = 0; t0 < cm; t0 += NB) {
+        for (int b = 0; b < bm; ++b) {
+            const int t0 = 4 * b;
             if (t0 % 32 == 0) word = (stage != 0 && t0 < lc) ? S.pass[(size_t)(t0 / 32) * n + i] : 0u;
-            int kb[NB];
-            float4 xb[NB], yb[NB], zb[NB];
+            const int4 q4 = list_block(S.nlist, S.lstride, i, b, nb, i);
+            const int kb[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
-            for (int u = 0; u < NB; ++u)
-                kb[u] = t0 + u < lc ? __ldg(S.nlist + (size_t)(t0 + u) * S.lstride + i) : i;
+            for (int v = 0; v < 4; v += NB) {
+                float4 xb[NB], yb[NB], zb[NB];
 #pragma unroll
-            for (int u = 0; u < NB; ++u) {
-                xb[u] = __ldg(n0 + kb[u]);
-                yb[u] = __ldg(n1 + kb[u]);
-                zb[u] = DIM == 3 ? __ldg(n2 + kb[u]) : yb[u];
+                for (int u = 0; u < NB; ++u) {
+                    xb[u] = __ldg(n0 + kb[v + u]);
+                    yb[u] = __ldg(n1 + kb[v + u]);
+                    zb[u] = DIM == 3 ? __ldg(n2 + kb[v + u]) : yb[u];
+                }
+                if (stage == 0) {  // the working positions are the start's
+#pragma unroll
+                    for (int u = 0; u < NB; ++u)
+                        if (t0 + v + u < lc && in_reach(xb[u])) word |= 1u << ((t0 + v + u) % 32);
+                }
+                const unsigned w = word >> ((t0 + v) % 32);
+#pragma unroll
+                for (int u = 0; u < NB; u += 2)
+                    pair2(kb[v + u], kb[v + u + 1], xb[u], xb[u + 1], yb[u], yb[u + 1], zb[u], zb[u + 1],
+                          (w >> u) & 1u, (w >> (u + 1)) & 1u);
             }
-            if (stage == 0) {  // the working positions are the start's
-#pragma unroll
-                for (int u = 0; u < NB; ++u)
-                    if (t0 + u < lc && in_reach(xb[u])) word |= 1u << ((t0 + u) % 32);
-                if (((t0 + NB) % 32 == 0 || t0 + NB >= lc) && t0 < lc && valid)
-                    S.pass[(size_t)(t0 / 32) * n + i] = word;
-            }
-            const unsigned w = word >> (t0 % 32);
-#pragma unroll
-            for (int u = 0; u < NB; u += 2)
-                pair2(kb[u], kb[u + 1], xb[u], xb[u + 1], yb[u], yb[u + 1], zb[u], zb[u + 1],
-                      (w >> u) & 1u, (w >> (u + 1)) & 1u);
-            if ((t0 + NB) % 32 == 0) word = 0u;
+            if (stage == 0 && valid && t0 < lc && ((t0 + 4) % 32 == 0 || t0 + 4 >= lc))
+                S.pass[(size_t)(t0 / 32) * n + i] = word;
         }
     }
     if (g.ok && (!LST || __any_sync(0xffffffffu, lc < 0))) {
