@@ -964,7 +964,8 @@ static __global__ void k_invert_ids(const int* __restrict__ id, int* __restrict_
 }
 
 // A -> caller arrays walking the caller order: the form for caller arrays in
-// host memory that the device maps, where every write crosses the host link.
+// host memory that the device maps, where every write crosses the host link, and for
+// large systems' arrays in device memory (kGatherOutMin).
 // The interleaved x, v, dv/dt of a block's kScatterSeq particles are staged in
 // shared memory and written as one contiguous run each (consecutive threads,
 // consecutive addresses: whole lines, no alignment needed); the reads of A are
