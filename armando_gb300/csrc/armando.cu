@@ -49,6 +49,7 @@ T* dalloc(size_t count, cudaError_t& err) {
 }
 
 constexpr int kFlagWords = 4;
+static_assert(sizeof(DevGrid) % sizeof(unsigned) == 0 && alignof(DevGrid) == alignof(unsigned), "status layout");
 
 }  // namespace
 
@@ -827,11 +828,11 @@ armando_status alloc_state(armando_ctx* ctx) {
     ctx->num_tiles = blocks_for(ctx->n, kSortTile);
     ctx->dtotal = dalloc<unsigned>(kRadix, e);
     ctx->bbox_part = dalloc<float>(kBBoxBlocks * 8, e);
-    ctx->grid = dalloc<DevGrid>(1, e);
+    // the status words and the grid, side by side: one copy brings both to the host.
     // [0] status bits, [1] this iteration sorts, [2] the next one must, [3] sorts done
-    ctx->flags = dalloc<unsigned>(kFlagWords, e);
-    for (void* p : {(void*)ctx->hist, (void*)ctx->dtotal, (void*)ctx->bbox_part, (void*)ctx->grid,
-                    (void*)ctx->flags})
+    ctx->flags = dalloc<unsigned>(kFlagWords + sizeof(DevGrid) / sizeof(unsigned), e);
+    ctx->grid = reinterpret_cast<DevGrid*>(ctx->flags + kFlagWords);
+    for (void* p : {(void*)ctx->hist, (void*)ctx->dtotal, (void*)ctx->bbox_part, (void*)ctx->flags})
         ctx->owned.push_back(p);
     if (ctx->mem_kind == ARMANDO_MEM_HOST) {
         const size_t nc = (size_t)std::max<int64_t>(ctx->n, 1), nd = nc * ctx->dim;
@@ -869,10 +870,9 @@ armando_status alloc_state(armando_ctx* ctx) {
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc");
     CK(cudaMemset(ctx->flags, 0, kFlagWords * sizeof(unsigned)));
     CK(cudaMemset(ctx->ticket, 0, sizeof(unsigned)));
-    cudaError_t he = cudaMallocHost((void**)&ctx->h_flags, kFlagWords * sizeof(unsigned));
+    cudaError_t he = cudaMallocHost((void**)&ctx->h_flags, kFlagWords * sizeof(unsigned) + sizeof(DevGrid));
     if (he != cudaSuccess) return cuda_fail(ctx, he, "cudaMallocHost");
-    he = cudaMallocHost((void**)&ctx->h_grid, sizeof(DevGrid));
-    if (he != cudaSuccess) return cuda_fail(ctx, he, "cudaMallocHost");
+    ctx->h_grid = reinterpret_cast<DevGrid*>(ctx->h_flags + kFlagWords);
     if (ctx->prm.wall_model == 3) {
         he = cudaMallocHost((void**)&ctx->h_wgrid, sizeof(WallGrid));
         if (he == cudaSuccess) he = cudaMallocHost((void**)&ctx->h_ng, sizeof(int));
@@ -1322,10 +1322,10 @@ armando_status prepare_gpuc(armando_ctx* ctx) {
 // Enqueues the copy of the device status words and the last grid to the
 // pinned host mirrors (complete once the stream passes this point).
 armando_status copy_flags(armando_ctx* ctx) {
-    CK(cudaMemcpyAsync(ctx->h_flags, ctx->flags, kFlagWords * sizeof(unsigned),
+    CK(cudaMemcpyAsync(ctx->h_flags, ctx->flags, kFlagWords * sizeof(unsigned) + sizeof(DevGrid),
                        cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaMemcpyAsync(ctx->h_grid, ctx->n_inst > 1 ? ctx->d_grids : ctx->grid, sizeof(DevGrid),
-                       cudaMemcpyDeviceToHost, ctx->stream));
+    if (ctx->n_inst > 1)
+        CK(cudaMemcpyAsync(ctx->h_grid, ctx->d_grids, sizeof(DevGrid), cudaMemcpyDeviceToHost, ctx->stream));
     return ARMANDO_OK;
 }
 
@@ -1513,14 +1513,14 @@ armando_status load_inputs(armando_ctx* ctx, const float* x, const float* vx, co
     if (ctx->dim == 2)
         k_gather_in<2><<<blocks_for(nn, 256), 256, 0, st>>>(x, vx, mass, rho, p, u, hsml, itype,
                                                             dvdt, dudt, ctx->A, nn, ctx->d_inst0,
-                                                            rfl, pfl);
+                                                            rfl, pfl, ctx->flags + 2);
     else
         k_gather_in<3><<<blocks_for(nn, 256), 256, 0, st>>>(x, vx, mass, rho, p, u, hsml, itype,
                                                             dvdt, dudt, ctx->A, nn, ctx->d_inst0,
-                                                            rfl, pfl);
+                                                            rfl, pfl, ctx->flags + 2);
     ctx->launches += 1;
     CK(cudaGetLastError());
-    return force_sort(ctx);  // A is in caller order now
+    return nn > 0 ? ARMANDO_OK : force_sort(ctx);
 }
 
 // A -> device arrays: below this size each slot writes its particle where the caller
@@ -3079,7 +3079,6 @@ armando_status armando_destroy(armando_ctx* ctx) {
     free_graphs(ctx);
     for (void* p : ctx->owned) cudaFree(p);
     if (ctx->h_flags) cudaFreeHost(ctx->h_flags);
-    if (ctx->h_grid) cudaFreeHost(ctx->h_grid);
     if (ctx->h_wgrid) cudaFreeHost(ctx->h_wgrid);
     if (ctx->h_ng) cudaFreeHost(ctx->h_ng);
     if (ctx->h_open_n) cudaFreeHost(ctx->h_open_n);

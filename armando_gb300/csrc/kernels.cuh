@@ -907,9 +907,10 @@ __global__ void k_gather_in(const float* __restrict__ x, const float* __restrict
                             const float* __restrict__ h, const int* __restrict__ itype,
                             const float* __restrict__ dvdt, const float* __restrict__ dudt,
                             StateA A, int n, const int* __restrict__ inst0, int rho_fl,
-                            int p_fl) {
+                            int p_fl, unsigned* __restrict__ sort_next) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
+    if (i == 0) *sort_next = 1u;  // A is in caller order now (lazy sorting)
     if (inst0) A.inst[i] = inst0[i];
     gather_pos_one<DIM>(i, x, m, h, A);
     gather_rest_one<DIM>(i, v, m, rho, p, u, itype, dvdt, dudt, A, rho_fl, p_fl);
