@@ -807,7 +807,7 @@ armando_status alloc_state(armando_ctx* ctx) {
     F1(ctx->B.ulo, n);
     ctx->B.vr = dalloc<float4>(ctx->dim == 2 ? n : 1, e);
     ctx->owned.push_back(ctx->B.vr);
-    ctx->xsort_buf = dalloc<float4>(n, e);  // B.xsort points here while sorting lazily
+    ctx->xsort_buf = dalloc<float4>(n + kListPad, e);  // B.xsort points here while sorting lazily
     ctx->owned.push_back(ctx->xsort_buf);
     ctx->B.nmask = dalloc<unsigned>(n * (ctx->dim == 2 ? mask_words<2>() : mask_words<3>()), e);
     ctx->B.mstride = (int)n;

@@ -1375,6 +1375,8 @@ constexpr int kListCap3 = 256;
 // Blocks of four per slot: the capacity's and room for the far entries' own while a
 // list is built.
 __host__ __device__ constexpr int list_blocks(int lcap) { return lcap / 4 + 2; }
+constexpr int kRing = 16;    // entries a thread of the build holds back of each kind
+constexpr int kListPad = 3;  // positions readable past the last slot
 static_assert(kListCap2 <= 32 * mask_words<2>() && kListCap3 <= 32 * mask_words<3>(),
               "a list's neighbour bits fit one lane's mask");
 constexpr int kListCapD = 24;     // density pass: near and far lists each
@@ -2649,10 +2651,10 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
 // order, the candidates k != s (cursor order) within h_s + h_k + skin, the
 // bound widened by 2^-14 over the rounding of the FP32 distances; in 2D the
 // pairs the density pass evaluates in FP32 (q >= list_near_q2() at the sort) after
-// the others (collected from the last block down, then moved up). Positions are those in cell order (B.xsort; the reorder of the
-// rest comes later in the iteration). Until the next sort every particle stays
-// within half the skin of where it was binned, so every pair the exact test accepts
-// (r < h_i + h_j) on those iterations is in the list.
+// the others (collected from the last block down, then moved up). Positions are those
+// in cell order (B.xsort; the reorder of the rest comes later in the iteration). Until
+// the next sort every particle stays within half the skin of where it was binned, so
+// every pair the exact test accepts (r < h_i + h_j) on those iterations is in the list.
 //
 // OWN (the GPU-C schemes): the candidates within 2 h_s + skin, all of them near.
 //
@@ -2662,10 +2664,12 @@ __global__ void __launch_bounds__(BS, 1024 / BS)
 // loops here, a wrapped row shifts the particle once instead of each difference, the
 // bound is a constant when every h is alike and four candidates are tested together.
 // Single entries, stored as found, touched 15 sectors a warp and entry, the lanes
-// being at different rows; four are collected in registers and stored as one int4, and
-// the passes read four at a time. Measured, 185 k particles (3D): 208 us a build, 140
-// with single entries, 162 with blocks, which the passes win back: 8.78 M, four
-// iterations, 39.5 -> 34.8 ms.
+// being at different rows; four leave as one int4, and the passes read four at a
+// time. They wait in shared memory (a store and an index; collected in registers they
+// took seven instructions and a branch each), and the particle's own row is walked
+// around it instead of asking each candidate. Measured a build: 185 k particles (3D)
+// 208 -> 141 us, 8.78 M 6.60 -> 3.77 ms, 2.03 M (2D) 222 -> 214 us, the last now
+// waiting for its loads. (Skipping the cells beyond the bound's sphere: 162 -> 173 us.)
 template <int DIM, bool PER, bool OWN = false>
 __global__ void __launch_bounds__(kPassThreads)
     k_build_list(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
@@ -2690,32 +2694,36 @@ __global__ void __launch_bounds__(kPassThreads)
         return __fmul_rn(lim, lim);
     };
     const float lim_u = bound2(xi.w), near_u = kNear2 * (2.0f * xi.w) * (2.0f * xi.w);
+    // Entries wait in the thread's column of a ring in shared memory; whole blocks of
+    // four leave it for global memory.
+    __shared__ int s_ring[SPLIT ? 2 : 1][kRing][kPassThreads];
+    int(*const ring_n)[kPassThreads] = s_ring[0];
+    int(*const ring_f)[kPassThreads] = s_ring[SPLIT ? 1 : 0];
+    const int tid = threadIdx.x;
     int cn = 0, cf = 0;  // near and far entries
+    int bn = 0, bf = 0;  // those of them stored: near blocks upwards from the first, far
+                         // ones downwards from the last
     const int last = list_blocks(B.lcap) - 1;
     int4* const l4 = reinterpret_cast<int4*>(B.nlist) + s;
-    int4* pn = l4;                                  // next block of near entries, upwards
-    int4* pf = l4 + (size_t)last * B.lstride;       // of far entries, downwards
-    int4 qn = make_int4(s, s, s, s), qf = qn;       // the last four entries of each kind
-    auto add_near = [&](int k) {
-        qn = make_int4(qn.y, qn.z, qn.w, k);
-        if ((++cn & 3) == 0) {
-            if (cn + cf <= B.lcap) *pn = qn;
-            pn += B.lstride;
+    auto flush = [&](int(*const ring)[kPassThreads], const int count, int& done, const bool up) {
+        for (; count - done >= 4; done += 4) {
+            const int t = done & (kRing - 1);
+            const int4 q = make_int4(ring[t][tid], ring[t + 1][tid], ring[t + 2][tid], ring[t + 3][tid]);
+            const int b = up ? done >> 2 : last - (done >> 2);
+            if (cn + cf <= B.lcap) l4[(size_t)b * B.lstride] = q;
         }
     };
-    auto add_far = [&](int k) {
-        qf = make_int4(qf.y, qf.z, qf.w, k);
-        if ((++cf & 3) == 0) {
-            if (cn + cf <= B.lcap) *pf = qf;
-            pf -= B.lstride;
-        }
-    };
+    auto add_near = [&](int k) { ring_n[cn++ & (kRing - 1)][tid] = k; };
+    auto add_far = [&](int k) { ring_f[cf++ & (kRing - 1)][tid] = k; };
     // Slots [kb, ke) against the particle at (x, y, z) (wrapped rows: shifted).
     auto range = [&](int kb, int ke, float x, float y, float z) {
         for (int k0 = kb; k0 < ke; k0 += 4) {
+            const float4* const src = B.xsort + k0;  // (kListPad entries past the last slot)
             float4 xb[4];
 #pragma unroll
-            for (int u = 0; u < 4; ++u) xb[u] = __ldg(B.xsort + min(k0 + u, ke - 1));
+            for (int u = 0; u < 4; ++u) xb[u] = __ldg(src + u);
+            if (cn - bn > kRing - 4) flush(ring_n, cn, bn, true);
+            if (SPLIT && cf - bf > kRing - 4) flush(ring_f, cf, bf, false);
 #pragma unroll
             for (int u = 0; u < 4; u += 2) {
                 const f2 d0 = make_float2(x - xb[u].x, x - xb[u + 1].x);
@@ -2729,7 +2737,7 @@ __global__ void __launch_bounds__(kPassThreads)
                 for (int e = 0; e < 2; ++e) {
                     const int k = k0 + u + e;
                     const float rr = e ? r2.y : r2.x, hk = xb[u + e].w;
-                    const bool in = rr < (uni ? lim_u : bound2(hk)) && k < ke && k != s;
+                    const bool in = rr < (uni ? lim_u : bound2(hk)) && k < ke;
                     const bool near = !SPLIT || rr < (uni ? near_u : kNear2 * (xi.w + hk) * (xi.w + hk));
                     if (in && near) add_near(k);
                     if (SPLIT && in && !near) add_far(k);
@@ -2755,13 +2763,17 @@ __global__ void __launch_bounds__(kPassThreads)
                 cy += cy < 0 ? g.n[1] : -g.n[1];
             }
             const int* row = start + g.cell_off + (cz * g.n[1] + cy) * g.n[0];
-            range(__ldg(row + c0), __ldg(row + c1), xi.x, y, z);
+            const int b = __ldg(row + c0), e = __ldg(row + c1);
+            const bool own = dy == 0 && dz == 0;  // the particle's row: around itself
+            range(b, own ? s : e, xi.x, y, z);
+            if (own) range(s + 1, e, xi.x, y, z);
             if (PER && g.periodic[0]) {  // the part of the row past either end
                 if (cc.c[0] < f)
                     range(__ldg(row + cc.c[0] - f + g.n[0]), __ldg(row + g.n[0]), xi.x + g.L[0], y, z);
                 else if (cc.c[0] + f >= g.n[0])
                     range(__ldg(row), __ldg(row + cc.c[0] + f - g.n[0] + 1), xi.x - g.L[0], y, z);
             }
+            flush(ring_n, cn, bn, true);
         }
     }
     if (cn + cf > B.lcap) {
@@ -2769,25 +2781,28 @@ __global__ void __launch_bounds__(kPassThreads)
         return;
     }
     B.ncount[s] = cn | (cf << 16);
+    flush(ring_n, cn, bn, true);
     if (SPLIT) {
-        // The far entries behind the near ones, the latest first: those in qf, then the
-        // blocks upwards from the last one stored. A block is read before the near
+        // The far entries behind the near ones, the latest first: those in the ring, then
+        // the blocks upwards from the last one stored. A block is read before the near
         // side, at most (cn + cf) / 4 blocks, can reach it.
-        const int tail = cf & 3, full = cf >> 2;
+        int left = cf;
         cf = 0;
-        if (tail > 0) add_near(qf.w);
-        if (tail > 1) add_near(qf.z);
-        if (tail > 2) add_near(qf.y);
-        for (int b = 0; b < full; ++b) {
-            pf += B.lstride;
-            const int4 q = *pf;
+        while (left > bf) {
+            add_near(ring_f[--left & (kRing - 1)][tid]);
+            flush(ring_n, cn, bn, true);
+        }
+        for (; left > 0; left -= 4) {
+            const int4 q = l4[(size_t)(last - (left >> 2) + 1) * B.lstride];
             add_near(q.w);
             add_near(q.z);
             add_near(q.y);
             add_near(q.x);
+            flush(ring_n, cn, bn, true);
         }
     }
     while (cn & 3) add_near(s);
+    flush(ring_n, cn, bn, true);
 }
 
 template <int DIM, bool LST>
