@@ -263,8 +263,8 @@ __host__ __device__ constexpr int gpuc_list_len() {
 //
 // Issue and latency bound the stage (42-57% of cycles): it walked its cells three
 // times a step, with the divider's code five times a pair. Measured a stage,
-// 85,773 / 361,201 particles: 28.7 / 84.9 us walking the cells, 16.0 / 37.8 on lists
-// (10 / 23 us a sort to build them); 96 registers, so that five blocks of 128 fit.
+// 85,773 / 361,201 particles: 28.7 / 84.9 us walking the cells, 15.1 / 34.2 on lists
+// (8 / 22 us a sort to build them); 96 registers, so that five blocks of 128 fit.
 template <int DIM, int VAR, int TPP = 1, int BS = kPassThreads, bool LST = false>
 __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
     k_gpuc_stage(GpucState S, int cur, const unsigned* __restrict__ keys,
@@ -387,10 +387,12 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
         const int nb = blocks_of(lc);
         const int bm = __reduce_max_sync(0xffffffffu, nb);
         unsigned word = 0u;
+        int4 kn = list_block(S.nlist, S.lstride, i, 0, nb, i);
         for (int b = 0; b < bm; ++b) {
             const int t0 = 4 * b;
             if (t0 % 32 == 0) word = (stage != 0 && t0 < lc) ? S.pass[(size_t)(t0 / 32) * n + i] : 0u;
-            const int4 q4 = list_block(S.nlist, S.lstride, i, b, nb, i);
+            const int4 q4 = kn;
+            if (b + 1 < bm) kn = list_block(S.nlist, S.lstride, i, b + 1, nb, i);
             const int kb[4] = {q4.x, q4.y, q4.z, q4.w};
 #pragma unroll
             for (int v = 0; v < 4; v += NB) {
