@@ -216,6 +216,11 @@ __device__ __forceinline__ int nbr_fill(NbrStream<DIM>& ns, const StateB& B, con
                                         const float4& xi, int s, int (*s_list)[kPassThreads]) {
     const int tid = threadIdx.x;
     int nl = 0;
+    if (DIM == 2 && !ns.done && ns.from_mask && ns.wi == 0 && ns.rbase == 0 && ns.cu.ke == 0 &&
+        __popc(ns.ch.x) + __popc(ns.ch.y) + __popc(ns.ch.z) + __popc(ns.ch.w) <= kListCap) {
+        mask_slots(ns.ch, g, start, cc, [&](const int k, int) { s_list[nl++][tid] = k; });
+        ns.done = true;
+    }
     while (!ns.done && ns.from_mask) {
         if (nl == kListCap) break;
         while (ns.wbits == 0u && ns.wi < mask_words<DIM>() - 1) {

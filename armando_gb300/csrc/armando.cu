@@ -786,7 +786,9 @@ armando_status alloc_state(armando_ctx* ctx) {
     auto F4 = [&](float4*& p) { p = dalloc<float4>(n, e); ctx->owned.push_back(p); };
     auto F1 = [&](float*& p, size_t k) { p = dalloc<float>(k, e); ctx->owned.push_back(p); };
     auto I1 = [&](int*& p) { p = dalloc<int>(n, e); ctx->owned.push_back(p); };
-    F4(ctx->A.xh);
+    // (positions: readable kListPad entries past the last slot)
+    auto X4 = [&](float4*& p) { p = dalloc<float4>(n + kListPad, e); ctx->owned.push_back(p); };
+    X4(ctx->A.xh);
     F4(ctx->A.vm);
     F1(ctx->A.u, n);
     F4(ctx->A.ap);
@@ -794,7 +796,7 @@ armando_status alloc_state(armando_ctx* ctx) {
     F1(ctx->A.p, n);
     I1(ctx->A.itype);
     I1(ctx->A.id);
-    F4(ctx->B.xh);
+    X4(ctx->B.xh);
     F4(ctx->B.vm);
     F4(ctx->B.vmin);
     F4(ctx->B.rp);
@@ -1612,7 +1614,7 @@ armando_status store_outputs(armando_ctx* ctx, float* x, float* vx, float* rho, 
 armando_status alloc_stateA(armando_ctx* ctx, StateA& a) {
     cudaError_t e = cudaSuccess;
     const size_t n = (size_t)std::max<int64_t>(ctx->n, 1);
-    a.xh = dalloc<float4>(n, e);
+    a.xh = dalloc<float4>(n + kListPad, e);
     a.vm = dalloc<float4>(n, e);
     a.u = dalloc<float>(n, e);
     a.ap = dalloc<float4>(n, e);
