@@ -474,16 +474,14 @@ int launch_gpuc_passes(armando_ctx* ctx, const StepArgs& S, const int* rs) {
             if (ctx->prm.scheme == 1)
                 k_gpuc_stage<DIM, 1, T, BSZ, LST><<<blocks, BSZ, 0, st>>>(
                     gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
-                    ctx->flags, alphas[q], S.dt, n, q);
+                    ctx->flags, alphas[q], S.dt, n, q, ctx->A);
             else
                 k_gpuc_stage<DIM, 2, T, BSZ, LST><<<blocks, BSZ, 0, st>>>(
                     gs, cur, skeys, ctx->start, ctx->grid, ctx->dp, ctx->d_mat, nm, ctx->d_zones,
-                    ctx->flags, alphas[q], S.dt, n, q);
+                    ctx->flags, alphas[q], S.dt, n, q, ctx->A);
         });
     }
-    k_gpuc_scatter<DIM><<<blocks_for(n, 256), 256, 0, st>>>(ctx->gs, 1, ctx->A, n, ctx->grid,
-                                                            ctx->flags);
-    return 5;
+    return 4;
 }
 
 // rs: the lazy-sorting flags (nullptr: the step sorts).
@@ -1269,13 +1267,12 @@ armando_status prepare_gpuc(armando_ctx* ctx) {
             g.w2[k] = dalloc<float4>(n, e);
             g.uw[k] = dalloc<float>(ctx->dim == 3 ? n : 1, e);
         }
-        g.rates = dalloc<float4>(n, e);
         g.id = dalloc<int>(n, e);
         ctx->d_mat = dalloc<DevMaterial>(ARMANDO_MAX_MATERIALS, e);
         ctx->d_zones = dalloc<DevZones>(1, e);
         for (void* q : {(void*)g.x0, (void*)g.v0, (void*)g.q0, (void*)g.w0[0], (void*)g.w0[1],
                         (void*)g.w1[0], (void*)g.w1[1], (void*)g.w2[0], (void*)g.w2[1],
-                        (void*)g.uw[0], (void*)g.uw[1], (void*)g.rates, (void*)g.id,
+                        (void*)g.uw[0], (void*)g.uw[1], (void*)g.id,
                         (void*)ctx->d_mat, (void*)ctx->d_zones})
             ctx->owned.push_back(q);
         if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(GPU-C state)");

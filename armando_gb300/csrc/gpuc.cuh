@@ -64,7 +64,6 @@ struct GpucState {
     float4* w1[2];
     float4* w2[2];
     float* uw[2];   // 3D: u
-    float4* rates;  // {dv/dt, de/dt} of the last stage
     int* id;
     float4* xsort;  // lazy sorting: positions at the last sort (nullptr: every step sorts)
     // Neighbour lists of the last sort (StateB's blocks; entries within 2 h_i + skin in
@@ -270,7 +269,7 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
     k_gpuc_stage(GpucState S, int cur, const unsigned* __restrict__ keys,
                  const int* __restrict__ start, const DevGrid* __restrict__ gp, DevParams P,
                  const DevMaterial* __restrict__ mat, int n_mat, const DevZones* __restrict__ zones,
-                 unsigned* __restrict__ flags, float alpha, float dt, int n, int stage) {
+                 unsigned* __restrict__ flags, float alpha, float dt, int n, int stage, StateA A) {
     static_assert(!LST || TPP == 1, "lists: one lane per particle");
     const int i0 = blockIdx.x * (BS / TPP) + (int)threadIdx.x / TPP;
     const int sub = (TPP == 1) ? 0 : (int)(threadIdx.x & (TPP - 1));
@@ -488,7 +487,6 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
     }
     // balanceEnergyHost on top of the loads' w
     const float du = __fadd_rn(wz, __fdiv_rn(__fmul_rn(q.p, rd), __fmul_rn(q.rho, q.rho)));
-    S.rates[i] = make_float4(a0, a1, a2, du);
     GpucPart o = q;
     if (VAR == 2 || it != 0) {  // acpu.c:894 leaves itype 0 alone
         o.x[0] = fmaf(alpha, fmaf(dt, q.v[0], q.x[0]) - x0i.x, x0i.x);
@@ -522,37 +520,31 @@ __global__ void __launch_bounds__(BS, LST && BS <= 256 ? 640 / BS : 1)
         const float chk = o.x[0] + o.x[1] + o.x[2] + o.v[0] + o.v[1] + o.v[2] + o.rho + o.u + o.p;
         if (!isfinite(chk)) atomicOr(flags, (unsigned)FLAG_NONFINITE);
     }
-    gpuc_store<DIM>(S, cur ^ 1, i, o);
-}
-
-// The step's result back to A (cell order of this step, like the force pass).
-// Lazy sorting: a particle farther than half the skin from where it was binned
-// makes the next step sort (the cells of the last sort hold every pair within
-// 2 max(h) of the step's start positions only while none is).
-template <int DIM>
-__global__ void k_gpuc_scatter(GpucState S, int cur, StateA A, int n,
-                               const DevGrid* __restrict__ gp = nullptr,
-                               unsigned* __restrict__ flags = nullptr) {
-    const int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= n) return;
-    const GpucPart q = gpuc_load<DIM>(S, cur, s);
-    const float4 xn = DIM == 2 ? make_float4(q.x[0], q.x[1], q.m, q.h)
-                               : make_float4(q.x[0], q.x[1], q.x[2], q.h);
-    if (S.xsort && gp && flags) {
-        const float h2 = gp->half_skin2;
-        const float4 xb = S.xsort[s];
-        const float e0 = xn.x - xb.x, e1 = xn.y - xb.y, e2 = (DIM == 3) ? xn.z - xb.z : 0.f;
-        if (h2 > 0.f && e0 * e0 + e1 * e1 + e2 * e2 > h2 && *(volatile unsigned*)(flags + 2) == 0u)
+    if (stage < 2) {
+        gpuc_store<DIM>(S, cur ^ 1, i, o);
+        return;
+    }
+    // The step's result to A (cell order of this step, like the force pass). As a kernel
+    // of its own five steps took 464 us at 86 k particles, now 454, and at 361 k, where
+    // the copy itself counts, 1,013 and 1,010.
+    // Lazy sorting: a particle farther than half the skin from where it was binned
+    // makes the next step sort (the cells of the last sort hold every pair within
+    // 2 max(h) of the step's start positions only while none is).
+    if (S.xsort) {
+        const float4 xb = S.xsort[i];
+        const float e0 = o.x[0] - xb.x, e1 = o.x[1] - xb.y, e2 = (DIM == 3) ? o.x[2] - xb.z : 0.f;
+        if (g.half_skin2 > 0.f && e0 * e0 + e1 * e1 + e2 * e2 > g.half_skin2 &&
+            *(volatile unsigned*)(flags + 2) == 0u)
             atomicExch(flags + 2, 1u);
     }
-    A.xh[s] = xn;
-    A.vm[s] = make_float4(q.v[0], q.v[1], q.v[2], DIM == 3 ? q.m : 0.f);
-    A.rho[s] = q.rho;
-    A.u[s] = q.u;
-    A.p[s] = q.p;
-    A.ap[s] = S.rates[s];
-    A.itype[s] = q.it;
-    A.id[s] = S.id[s];
+    A.xh[i] = DIM == 2 ? make_float4(o.x[0], o.x[1], o.m, o.h) : make_float4(o.x[0], o.x[1], o.x[2], o.h);
+    A.vm[i] = make_float4(o.v[0], o.v[1], o.v[2], DIM == 3 ? o.m : 0.f);
+    A.rho[i] = o.rho;
+    A.u[i] = o.u;
+    A.p[i] = o.p;
+    A.ap[i] = make_float4(a0, a1, a2, du);
+    A.itype[i] = o.it;
+    A.id[i] = S.id[i];
 }
 
 }  // namespace ag
