@@ -188,7 +188,7 @@ StepArgs make_args(const armando_ctx* c, float dt, int its) {
 }
 
 void free_graphs(armando_ctx* c) {
-    for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second);
+    for (auto& kv : c->graphs) cudaGraphExecDestroy(kv.second.exec);
     c->graphs.clear();
     if (c->batch_graph) cudaGraphExecDestroy(c->batch_graph);
     c->batch_graph = nullptr;
@@ -717,7 +717,12 @@ armando_status run_overlapped_step(armando_ctx* ctx, const StepArgs& S, float* r
     return ARMANDO_OK;
 }
 
-armando_status run_step(armando_ctx* ctx, const StepArgs& S) {
+// first: the first step after a load, which always sorts: small systems take it without
+// the conditional node around its sort, which costs 14 us on the way in and 5 out. Ten
+// steps of 27 k particles 480.5 -> 467.7 us, five GPU-C steps of 86 k 450.5 -> 446.2; at
+// 361 k nothing, and at 2.03 M the second graph's launch costs more (2,732 -> 2,752 us).
+constexpr int64_t kFirstPlainMax = 1 << 18;
+armando_status run_step(armando_ctx* ctx, const StepArgs& S, bool first = false) {
     if (ctx->n_inst > 1) return run_batch_step(ctx);
     if (ctx->prm.wall_model == 3)
         return ctx->dim == 2 ? run_ghost_step<2>(ctx, S) : run_ghost_step<3>(ctx, S);
@@ -727,10 +732,11 @@ armando_status run_step(armando_ctx* ctx, const StepArgs& S) {
         free_graphs(ctx);
     }
     const bool fuse = fused(ctx);
-    GraphKey key{S.kdt, S.hdt, S.dt, S.heat_on, fuse ? 1 + ctx->acur : 0, use_lists(ctx) ? 1 : 0};
+    GraphKey key{S.kdt, S.hdt, S.dt, S.heat_on, fuse ? 1 + ctx->acur : 0, use_lists(ctx) ? 1 : 0,
+                 first && lazy(ctx) && ctx->n_work <= kFirstPlainMax ? 1 : 0};
     auto itg = ctx->graphs.find(key);
     cudaGraphExec_t exec = nullptr;
-    if (itg == ctx->graphs.end() && lazy(ctx) && !ctx->no_conditional) {
+    if (itg == ctx->graphs.end() && lazy(ctx) && !key.first && !ctx->no_conditional) {
         int L = 0;
         armando_status gs;
         {
@@ -739,9 +745,7 @@ armando_status run_step(armando_ctx* ctx, const StepArgs& S) {
                                : build_lazy_graph<3>(ctx, S, &exec, &L);
         }
         if (gs == ARMANDO_OK) {
-            ctx->graphs[key] = exec;
-            ctx->launches_per_step = L;
-            itg = ctx->graphs.find(key);
+            itg = ctx->graphs.insert({key, {exec, L - ctx->lazy_body}}).first;
         } else {
             ctx->no_conditional = true;  // the plain sequence below instead
             exec = nullptr;
@@ -763,15 +767,12 @@ armando_status run_step(armando_ctx* ctx, const StepArgs& S) {
         cudaError_t ie = cudaGraphInstantiate(&exec, graph, 0);
         cudaGraphDestroy(graph);
         if (ie != cudaSuccess) return cuda_fail(ctx, ie, "cudaGraphInstantiate");
-        ctx->graphs[key] = exec;
-        ctx->launches_per_step = L;
-        ctx->lazy_body = 0;
-    } else {
-        exec = itg->second;
+        itg = ctx->graphs.insert({key, {exec, L}}).first;
     }
-    CK(cudaGraphLaunch(exec, ctx->stream));
+    CK(cudaGraphLaunch(itg->second.exec, ctx->stream));
     // the conditional body's kernels are counted when the device reports its sorts
-    ctx->launches += ctx->launches_per_step - ctx->lazy_body;
+    ctx->launches += itg->second.launches;
+    if (key.first) ctx->first_sorts += 1;
     ctx->steps_done += 1;
     if (!lazy(ctx)) ctx->sorts_host += 1;
     if (fuse) swap_state(ctx);
@@ -1362,7 +1363,9 @@ armando_status eval_flags(armando_ctx* ctx) {
     ctx->last_grid = *ctx->h_grid;
     ctx->have_grid = true;
     if ((int64_t)ctx->h_flags[3] >= ctx->sorts_done)
-        ctx->launches += ((int64_t)ctx->h_flags[3] - ctx->sorts_done) * ctx->lazy_body;
+        ctx->launches += std::max<int64_t>((int64_t)ctx->h_flags[3] - ctx->sorts_done - ctx->first_sorts, 0) *
+                         ctx->lazy_body;
+    ctx->first_sorts = 0;
     ctx->sorts_done = ctx->h_flags[3];
     const unsigned f = *ctx->h_flags;
     if (f & FLAG_PERIODIC_SMALL) return fail(ctx, ARMANDO_ERR_INVALID_ARG, "periodic box shorter than 3 cells of 2*max(h)");
@@ -2461,7 +2464,7 @@ armando_status armando_integrate(armando_ctx* ctx, float* x, float* vx, const fl
     if (st != ARMANDO_OK) return st;
     for (int k = 0; k < steps; ++k) {
         st = split ? run_overlapped_step(ctx, make_args(ctx, dt, its0 + k), rho, p)
-                   : run_step(ctx, make_args(ctx, dt, its0 + k));
+                   : run_step(ctx, make_args(ctx, dt, its0 + k), k == 0);
         if (st != ARMANDO_OK) return st;
     }
     st = keep_options(ctx);

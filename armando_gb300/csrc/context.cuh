@@ -22,10 +22,16 @@ struct GraphKey {
     int heat_on;
     int par;  // 0: one state buffer; 1, 2: which of the two is current (fused predictor)
     int lst;  // neighbour lists in use
+    int first;  // a lazily sorting call's first step, which always sorts
     bool operator<(const GraphKey& o) const {
-        return std::tie(kdt, hdt, dt, heat_on, par, lst) <
-               std::tie(o.kdt, o.hdt, o.dt, o.heat_on, o.par, o.lst);
+        return std::tie(kdt, hdt, dt, heat_on, par, lst, first) <
+               std::tie(o.kdt, o.hdt, o.dt, o.heat_on, o.par, o.lst, o.first);
     }
+};
+
+struct StepGraph {
+    cudaGraphExec_t exec = nullptr;
+    int launches = 0;  // kernels outside a conditional body
 };
 
 inline int blocks_for(int64_t n, int t) { return (int)((n + t - 1) / t); }
@@ -87,10 +93,11 @@ struct armando_ctx {
     int* s_itype = nullptr;
     std::vector<void*> owned;
     int* inv = nullptr;  // caller index -> cell-order slot (outputs to mapped host memory)
-    std::map<GraphKey, cudaGraphExec_t> graphs;
+    std::map<GraphKey, StepGraph> graphs;
     std::string err = "no error";
     int64_t steps_done = 0, launches = 0;
     int launches_per_step = 0;
+    int64_t first_sorts = 0;  // sorts of first steps, whose kernels are counted with their graph
     int lazy_body = 0;  // kernels in the conditional body of the lazy step graph (run on sorting steps)
     DevGrid last_grid{};
     bool have_grid = false;
