@@ -1764,7 +1764,8 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
     // K/h^dim once per sum, Fast2Sum where the larger term is known and no residuals
     // for `plain` particles save about 30 of 85 operations a near pair. Measured: 3D
     // lists (8.78 M channel) 5.24 -> 3.45 ms, 2D lists (2.03 M dam break) 0.179 ->
-    // 0.154 ms, 2D cells (42 k) 21.6 -> 19.8 us.
+    // 0.154 ms, 2D cells (42 k) 21.6 -> 19.8 us (with blocks of entries 3.00 and 0.126
+    // ms, with the walk by rows 13.2 us).
     auto pair2 = [&](auto uni, auto ph, auto near, bool ina, bool inb, const int ka, const int kb,
                      const float4& xa, const float4& xb, const float4& va, const float4& vb) {
         constexpr bool UNI = decltype(uni)::value, NEAR = decltype(near)::value;
@@ -2456,7 +2457,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     // The pass was bound by issue (62% of cycles) and its neighbours' loads: about 80
     // instructions an entry, 50 now. Measured: 2D lists (2.03 M dam break) 0.213 ->
     // 0.160 ms, 3D lists (8.78 M channel) 6.77 -> 4.41 ms (3.84 with blocks of entries),
-    // 2D cells (42 k) 17.6 -> 16.1 us.
+    // 2D cells (42 k) 17.6 -> 16.1 us (10.5 with bits decoded by rows).
     // UNI: every particle has the same h (g.huni), whose factors are constants.
     // PH: the physics beyond pressure and art_visc compiled in, bits 1 art_heat,
     // 2 physical viscosity, 4 repulsive walls and the single_step options.

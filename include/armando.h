@@ -314,7 +314,7 @@ armando_status armando_get_stream(armando_ctx* ctx, void** stream);
 
 /* Phases of one step, in launch order, for armando_profile_phases. */
 #define ARMANDO_N_PHASES 6
-/* 0 grid (bbox + cell hash), 1 radix sort, 2 cell table + reorder/predictor,
+/* 0 grid (bbox + cells counted), 1 counting sort, 2 neighbour lists + reorder/predictor,
  * 3 density + EOS, 4 shear tensor (physical viscosity only), 5 forces +
  * corrector. */
 

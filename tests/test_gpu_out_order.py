@@ -1,9 +1,11 @@
-"""Outputs to device arrays on both sides of the size from which they are written
-in the caller's order (armando.cu, kGatherOutMin = 131,072).
+"""Calls on both sides of the sizes at which their form changes: from 131,072
+particles on outputs are written in the caller's order (armando.cu,
+kGatherOutMin), above 262,144 a lazily sorting call's first step sorts inside
+the conditional node like the later ones (kFirstPlainMax).
 
-Two particles alone in a gap carry a system of 131,071 over it: they interact
-with nobody and lie inside its bounds, so the grid, the order of every sum and
-each output of the others stay the same to the bit.
+Two particles alone in a gap carry a system of one less over the size: they
+interact with nobody and lie inside its bounds, so the grid, the order of every
+sum and each output of the others stay the same to the bit.
 """
 import numpy as np
 import pytest
@@ -14,7 +16,7 @@ from armando_gb300 import cases
 pytestmark = pytest.mark.gpu
 
 FIELDS = ("x", "v", "rho", "p", "u", "dvdt", "dudt")
-BELOW = 131071
+SIZES = {131071: (0.004, 131), 262143: (0.0028, 190)}  # dam dx, channel n_x
 
 
 @pytest.fixture(scope="module", autouse=True)
@@ -34,12 +36,13 @@ def _pick(c, idx):
     return out
 
 
-def _case(dim):
-    """131,071 particles around a gap, and two wall particles inside it."""
+def _case(dim, below):
+    """`below` particles around a gap, and two wall particles inside it."""
+    dx, n_x = SIZES[below]
     if dim == 2:
-        c = cases.perturbed(cases.dam_break(dx=0.004, jitter=0.1), seed=95, dv=0.1)
+        c = cases.perturbed(cases.dam_break(dx=dx, jitter=0.1), seed=95, dv=0.1)
     else:
-        c = cases.perturbed(cases.channel(n_x=131, n_yz=33, length=131 * 7.9e-4, width=33 * 7.9e-4,
+        c = cases.perturbed(cases.channel(n_x=n_x, n_yz=33, length=n_x * 7.9e-4, width=33 * 7.9e-4,
                                           layers=3, jitter=0.01), seed=95, dv=0.02)
         c.params.periodic[:] = (0, 0, 0)
     x = c.x.reshape(-1, dim)
@@ -47,10 +50,10 @@ def _case(dim):
     centre = x[fl].mean(axis=0)
     d = np.linalg.norm(x - centre, axis=1)
     d[c.itype <= 0] = np.inf
-    keep = np.sort(np.argsort(-d, kind="stable")[:BELOW])
+    keep = np.sort(np.argsort(-d, kind="stable")[:below])
     few = _pick(c, keep)
     wall = np.flatnonzero(few.itype <= 0)[:2]
-    many = _pick(few, np.concatenate([np.arange(BELOW), wall]))
+    many = _pick(few, np.concatenate([np.arange(below), wall]))
     y = many.x.reshape(-1, dim)
     y[-2:] = centre.astype(np.float32)
     y[-1, 0] += np.float32(0.5) * c.h[0]
@@ -75,9 +78,10 @@ def _run(c, call):
 
 @pytest.mark.parametrize("call", ["step", "run"])
 @pytest.mark.parametrize("dim", [2, 3])
-def test_outputs_alike_on_both_sides(dim, call):
-    few, many = _case(dim)
+@pytest.mark.parametrize("below", sorted(SIZES))
+def test_outputs_alike_on_both_sides(below, dim, call):
+    few, many = _case(dim, below)
     a, b = _run(few, call), _run(many, call)
     for f in FIELDS:
-        u, w = a[f].reshape(BELOW, -1), b[f].reshape(BELOW + 2, -1)[:BELOW]
+        u, w = a[f].reshape(below, -1), b[f].reshape(below + 2, -1)[:below]
         assert np.array_equal(u, w), f
