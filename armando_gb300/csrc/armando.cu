@@ -1631,16 +1631,10 @@ armando_status alloc_stateA(armando_ctx* ctx, StateA& a) {
 }
 
 armando_status copy_stateA(armando_ctx* ctx, const StateA& dst, const StateA& src) {
-    const size_t n = (size_t)ctx->n;
-    cudaStream_t st = ctx->stream;
-    CK(cudaMemcpyAsync(dst.xh, src.xh, n * 16, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.vm, src.vm, n * 16, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.u, src.u, n * 4, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.ap, src.ap, n * 16, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.rho, src.rho, n * 4, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.p, src.p, n * 4, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.itype, src.itype, n * 4, cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(dst.id, src.id, n * 4, cudaMemcpyDeviceToDevice, st));
+    const int n = (int)ctx->n;
+    k_copy_state<<<blocks_for(n, 256), 256, 0, ctx->stream>>>(dst, src, n);
+    ctx->launches += 1;
+    CK(cudaGetLastError());
     return ARMANDO_OK;
 }
 
@@ -1717,15 +1711,10 @@ armando_status save_tape(armando_ctx* ctx, int t) {
     cudaStream_t st = ctx->stream;
     const unsigned* skeys = ctx->keys[1];
     const int* perm = ctx->vals[1];
-    if (ctx->dim == 2)
-        k_tape_save<2><<<blocks_for(n, 256), 256, 0, st>>>(ctx->B, skeys, perm, ctx->A.ap, T, n);
-    else
-        k_tape_save<3><<<blocks_for(n, 256), 256, 0, st>>>(ctx->B, skeys, perm, ctx->A.ap, T, n);
+    auto save = ctx->dim == 2 ? k_tape_save<2> : k_tape_save<3>;
+    save<<<blocks_for(n, 256), 256, 0, st>>>(ctx->B, skeys, perm, ctx->A.ap, ctx->start, ctx->grid, T, n);
     ctx->launches += 1;
     CK(cudaGetLastError());
-    CK(cudaMemcpyAsync(T.start, ctx->start, ((size_t)ctx->cell_cap + 1) * sizeof(int),
-                       cudaMemcpyDeviceToDevice, st));
-    CK(cudaMemcpyAsync(T.grid, ctx->grid, sizeof(DevGrid), cudaMemcpyDeviceToDevice, st));
     return ARMANDO_OK;
 }
 
@@ -2707,7 +2696,7 @@ armando_status armando_forward_checkpointed(armando_ctx* ctx, float* x, float* v
         if (k % K == 0 && (st = copy_stateA(ctx, ctx->ckpts[k / K], ctx->A)) != ARMANDO_OK) return st;
         // Reverse mode sorts every iteration, so a replay from a checkpoint
         // repeats the forward bit for bit.
-        if ((st = force_sort(ctx)) != ARMANDO_OK) return st;
+        if (lazy(ctx) && (st = force_sort(ctx)) != ARMANDO_OK) return st;
         if ((st = run_step(ctx, make_args(ctx, dt, its0 + k))) != ARMANDO_OK) return st;
         if (k >= last && (st = save_tape(ctx, k - last)) != ARMANDO_OK) return st;
     }
@@ -2773,7 +2762,7 @@ armando_status armando_backward(armando_ctx* ctx, const float* x_bar, const floa
             ctx->tape_seg = -1;
             if ((st = copy_stateA(ctx, ctx->A, ctx->ckpts[c])) != ARMANDO_OK) return st;
             for (int t = 0; t < len; ++t) {
-                if ((st = force_sort(ctx)) != ARMANDO_OK) return st;
+                if (lazy(ctx) && (st = force_sort(ctx)) != ARMANDO_OK) return st;
                 if ((st = run_step(ctx, make_args(ctx, dt, its0 + a0 + t))) != ARMANDO_OK) return st;
                 if ((st = save_tape(ctx, t)) != ARMANDO_OK) return st;
             }
