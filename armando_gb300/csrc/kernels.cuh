@@ -1331,20 +1331,6 @@ __device__ __forceinline__ void exact_delta(const float4& xi, const float4& xj, 
     }
 }
 
-// On periodic axes the pair test's difference is rounded twice ((x_i - x_j)
-// then +- L); the force passes use the correctly rounded one instead.
-template <int DIM>
-__device__ __forceinline__ void refine_periodic(const float4& xi, const float4& xj,
-                                                const DevGrid& g, float* d, float& dr2) {
-    if (!(g.periodic[0] | g.periodic[1] | g.periodic[2])) return;
-    float dh[3], dl[3];
-    exact_delta<DIM>(xi, xj, g, dh, dl);
-#pragma unroll
-    for (int k = 0; k < DIM; ++k)
-        if (g.periodic[k]) d[k] = __fadd_rn(dh[k], dl[k]);
-    dr2 = sph::dist2_exact<DIM>(d);
-}
-
 // Minimum image of two differences x_i - x_a, x_i - x_b along axis k, for the force
 // passes: a difference that wraps is the exact one rounded once (exact_delta); one
 // that does not is already.

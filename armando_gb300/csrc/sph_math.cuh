@@ -85,7 +85,6 @@ SPH_HD void ff_acc(ff& acc, ff x) {
     acc.hi = s.hi;
     acc.lo = __fadd_rn(acc.lo, __fadd_rn(s.lo, x.lo));
 }
-SPH_HD ff ff_from_double_parts(float hi, float lo) { return {hi, lo}; }
 
 // 1/h as float-float: Newton residual of the correctly rounded reciprocal.
 SPH_HD ff ff_recip(float h) {
@@ -111,60 +110,6 @@ SPH_HD float min_image(float dx, float L, float half) {
     if (dx > half) return __fsub_rn(dx, L);
     if (dx < -half) return __fadd_rn(dx, L);
     return dx;
-}
-
-// ---- Wendland weight in float-float (density pass) ----
-// Returns m_j * W(r, h) with relative error ~1e-12 for the exact pair
-// difference x_i - x_j = dh + dl per axis (a float difference is not exact
-// when the coordinates differ by more than a factor 2, e.g. near the origin),
-// h = (h_i + h_j)/2 passed as its reciprocal ih and the prefactor
-// alpha = K_dim * ih^dim (both float-float).
-// CLAMP: zero beyond the support (q >= 2), so pairs need no separate test.
-template <int DIM, bool CLAMP = false>
-SPH_HD ff wendland_mw_ff(const float* dh, const float* dl, ff ih, ff alpha, float mj) {
-    // dr^2 = sum (dh + dl)^2 as hi + lo (dl^2 is below the float-float unit).
-    ff s0 = two_prod(dh[0], dh[0]);
-    float hi = s0.hi;
-    float lo = fmaf(__fmul_rn(2.0f, dh[0]), dl[0], s0.lo);
-#pragma unroll
-    for (int a = 1; a < DIM; ++a) {
-        ff sa = two_prod(dh[a], dh[a]);
-        float la = fmaf(__fmul_rn(2.0f, dh[a]), dl[a], sa.lo);
-        ff t = two_sum(hi, sa.hi);
-        hi = t.hi;
-        lo = __fadd_rn(lo, __fadd_rn(t.lo, la));
-    }
-    ff dr2 = fast_two_sum(hi, lo);
-    // r = sqrt(dr2): hardware reciprocal square root (a few ulp) and one exact
-    // Newton correction from the FMA residual dr2 - r0^2.
-    ff r = {0.0f, 0.0f};
-    if (dr2.hi > 0.0f) {
-        const float rs = rsqrtf(dr2.hi);
-        r.hi = __fmul_rn(dr2.hi, rs);
-        const float res = fmaf(-r.hi, r.hi, dr2.hi);
-        r.lo = __fmul_rn(__fadd_rn(res, dr2.lo), __fmul_rn(0.5f, rs));
-    }
-    ff q = ff_mul(r, ih);
-    // t = 1 - q/2 (q < 2 so |1| >= |q/2|).
-    ff t = fast_two_sum(1.0f, __fmul_rn(-0.5f, q.hi));
-    t.lo = fmaf(-0.5f, q.lo, t.lo);
-    if (CLAMP && !(t.hi + t.lo > 0.0f)) t = ff{0.0f, 0.0f};
-    ff t2 = ff_sqr(t);
-    ff t4 = ff_sqr(t2);
-    // g = 1 + 2q.
-    ff g = two_sum(1.0f, __fmul_rn(2.0f, q.hi));
-    g.lo = fmaf(2.0f, q.lo, g.lo);
-    ff f = ff_mul(t4, g);
-    return ff_mul(f, ff_mul_f(alpha, mj));
-}
-
-// ---- Wendland gradient factor, plain FP32 (force passes) ----
-// dW/dx_i = gw * (x_i - x_j), gw = K_dim * 5/8 * ih^(dim+2) * (q - 2)^3.
-template <int DIM>
-SPH_HD float wendland_grad_factor(float r, float ih, float kg_ih) {
-    float q = __fmul_rn(r, ih);
-    float t = __fsub_rn(q, 2.0f);
-    return __fmul_rn(kg_ih, __fmul_rn(__fmul_rn(t, t), t));
 }
 
 // Tait pressure from d = rho/rho0 - 1: B * ((1+d)^7 - 1), B = rho0 c0^2 / 7.
