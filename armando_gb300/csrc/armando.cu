@@ -909,6 +909,10 @@ armando_status alloc_cells(armando_ctx* ctx, long long cap) {
         return cuda_fail(ctx, e, "cudaMalloc(cell table)");
     }
     for (int* q : {ctx->start, ctx->cell_cnt, ctx->cell_sums}) ctx->owned.push_back(q);
+    for (TapeSlot& T : ctx->tape) {  // its copies of the cell table are allocated anew
+        release(ctx, T.start);
+        T.start = nullptr;
+    }
     ctx->cell_cap = cap;
     free_graphs(ctx);
     return ARMANDO_OK;
@@ -1638,35 +1642,31 @@ armando_status copy_stateA(armando_ctx* ctx, const StateA& dst, const StateA& sr
     return ARMANDO_OK;
 }
 
+// The reverse mode's buffers, each allocated when it is first needed: the parameters
+// may turn viscosity or artificial heat on after an earlier call.
+template <class T>
+void need(armando_ctx* ctx, T*& p, size_t count, cudaError_t& e) {
+    if (p) return;
+    p = dalloc<T>(count, e);
+    if (p) ctx->owned.push_back(p);
+}
+
 armando_status alloc_adjoint(armando_ctx* ctx) {
-    if (ctx->adj_abar) return ARMANDO_OK;
     cudaError_t e = cudaSuccess;
     const size_t n = (size_t)std::max<int64_t>(ctx->n, 1);
-    for (AdjState* g : {&ctx->adjG, &ctx->adjGp}) {
-        g->xb = dalloc<float4>(n, e);
-        g->vb = dalloc<float4>(n, e);
-        g->ab = dalloc<float4>(n, e);
-        for (void* p : {(void*)g->xb, (void*)g->vb, (void*)g->ab}) ctx->owned.push_back(p);
-    }
-    ctx->adj_abar = dalloc<float4>(n, e);
-    ctx->adj_xpart = dalloc<float4>(n, e);
-    ctx->adj_vpart = dalloc<float4>(n, e);
-    ctx->adj_xF = dalloc<float4>(n, e);
-    ctx->adj_vhb = dalloc<float4>(n, e);
-    ctx->adj_rhobar = dalloc<float>(n, e);
-    ctx->adj_pbar = dalloc<float>(n, e);
-    ctx->adj_blk = dalloc<double>((size_t)blocks_for(ctx->n, kPassThreads) * ADJ_NPARAM + 4, e);
-    ctx->adj_pacc = dalloc<double>(ADJ_NPARAM, e);
-    if (ctx->prm.heat_artificial) ctx->adj_divsb = dalloc<float>(n, e);
+    for (AdjState* g : {&ctx->adjG, &ctx->adjGp})
+        for (float4** q : {&g->xb, &g->vb, &g->ab}) need(ctx, *q, n, e);
+    for (float4** q : {&ctx->adj_abar, &ctx->adj_xpart, &ctx->adj_vpart, &ctx->adj_xF, &ctx->adj_vhb})
+        need(ctx, *q, n, e);
+    need(ctx, ctx->adj_rhobar, n, e);
+    need(ctx, ctx->adj_pbar, n, e);
+    need(ctx, ctx->adj_blk, (size_t)blocks_for(ctx->n, kPassThreads) * ADJ_NPARAM + 4, e);
+    need(ctx, ctx->adj_pacc, ADJ_NPARAM, e);
+    if (ctx->prm.heat_artificial) need(ctx, ctx->adj_divsb, n, e);
     if (ctx->prm.visc) {
-        ctx->adj_tbar = dalloc<float4>(n, e);
-        if (ctx->dim == 3) ctx->adj_tbar2 = dalloc<float4>(n, e);
+        need(ctx, ctx->adj_tbar, n, e);
+        if (ctx->dim == 3) need(ctx, ctx->adj_tbar2, n, e);
     }
-    for (void* p : {(void*)ctx->adj_abar, (void*)ctx->adj_xpart, (void*)ctx->adj_vpart,
-                    (void*)ctx->adj_xF, (void*)ctx->adj_vhb, (void*)ctx->adj_rhobar,
-                    (void*)ctx->adj_pbar, (void*)ctx->adj_blk, (void*)ctx->adj_pacc,
-                    (void*)ctx->adj_divsb, (void*)ctx->adj_tbar, (void*)ctx->adj_tbar2})
-        ctx->owned.push_back(p);
     if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(adjoint)");
     return ARMANDO_OK;
 }
@@ -1674,32 +1674,25 @@ armando_status alloc_adjoint(armando_ctx* ctx) {
 armando_status alloc_tape(armando_ctx* ctx, int count) {
     cudaError_t e = cudaSuccess;
     const size_t n = (size_t)std::max<int64_t>(ctx->n, 1);
-    while ((int)ctx->tape.size() < count) {
-        TapeSlot T{};
-        T.xh = dalloc<float4>(n, e);
-        T.vm = dalloc<float4>(n, e);
-        T.vmin = dalloc<float4>(n, e);
-        T.rp = dalloc<float4>(n, e);
-        T.p = dalloc<float>(n, e);
-        T.itype = dalloc<int>(n, e);
-        T.nmask = dalloc<unsigned>(n * (ctx->dim == 2 ? mask_words<2>() : mask_words<3>()), e);
-        T.keys = dalloc<unsigned>(n, e);
-        T.perm = dalloc<int>(n, e);
-        T.du = dalloc<float>(n, e);
-        T.start = dalloc<int>((size_t)ctx->cell_cap + 1, e);
-        T.grid = dalloc<DevGrid>(1, e);
-        if (ctx->prm.heat_artificial) T.ulo = dalloc<float>(n, e);
+    if ((int)ctx->tape.size() < count) ctx->tape.resize(count);
+    for (int t = 0; t < count; ++t) {
+        TapeSlot& T = ctx->tape[t];
+        for (float4** q : {&T.xh, &T.vm, &T.vmin, &T.rp}) need(ctx, *q, n, e);
+        need(ctx, T.p, n, e);
+        need(ctx, T.itype, n, e);
+        need(ctx, T.nmask, n * (ctx->dim == 2 ? mask_words<2>() : mask_words<3>()), e);
+        need(ctx, T.keys, n, e);
+        need(ctx, T.perm, n, e);
+        need(ctx, T.du, n, e);
+        need(ctx, T.start, (size_t)ctx->cell_cap + 1, e);
+        need(ctx, T.grid, 1, e);
+        if (ctx->prm.heat_artificial) need(ctx, T.ulo, n, e);
         if (ctx->prm.visc) {
-            T.tau = dalloc<float4>(n, e);
-            if (ctx->dim == 3) T.tau2 = dalloc<float4>(n, e);
+            need(ctx, T.tau, n, e);
+            if (ctx->dim == 3) need(ctx, T.tau2, n, e);
         }
-        for (void* p : {(void*)T.xh, (void*)T.vm, (void*)T.vmin, (void*)T.rp, (void*)T.p,
-                        (void*)T.itype, (void*)T.nmask, (void*)T.keys, (void*)T.perm, (void*)T.du,
-                        (void*)T.start, (void*)T.grid, (void*)T.ulo, (void*)T.tau, (void*)T.tau2})
-            ctx->owned.push_back(p);
         if (e != cudaSuccess)
             return cuda_fail(ctx, e, "cudaMalloc(adjoint tape; a smaller checkpoint_every needs less)");
-        ctx->tape.push_back(T);
     }
     return ARMANDO_OK;
 }
@@ -2108,6 +2101,7 @@ armando_status armando_set_params(armando_ctx* ctx, const armando_params* params
         return fail(ctx, ARMANDO_ERR_UNSUPPORTED, "mirror ghosts (wall_model 3) need a context created with wall_model 3");
     if (sorts_every_step(*params) && ctx->tune.skin != 0)
         return fail(ctx, ARMANDO_ERR_UNSUPPORTED, "mirror ghosts and h evolution sort every iteration: set a tuning with skin 0 first");
+    if (std::memcmp(&ctx->prm, params, sizeof *params) != 0) ctx->adj_ready = false;  // the tape's physics
     ctx->prm = *params;
     ctx->dp = make_dev_params(*params, ctx->tune.reach);
     ctx->dp.n_real = (int)ctx->n;
