@@ -303,7 +303,6 @@ void swap_state(armando_ctx* ctx) {
     std::swap(a.p, b.p);
     std::swap(a.itype, b.itype);
     std::swap(a.id, b.id);
-    ctx->acur ^= 1;
 }
 
 // The shear tensor (physical viscosity).
@@ -732,7 +731,7 @@ armando_status run_step(armando_ctx* ctx, const StepArgs& S, bool first = false)
         free_graphs(ctx);
     }
     const bool fuse = fused(ctx);
-    GraphKey key{S.kdt, S.hdt, S.dt, S.heat_on, fuse ? 1 + ctx->acur : 0, use_lists(ctx) ? 1 : 0,
+    GraphKey key{S.kdt, S.hdt, S.dt, S.heat_on, ctx->A.xh, fuse ? 1 : 0, use_lists(ctx) ? 1 : 0,
                  first && lazy(ctx) && ctx->n_work <= kFirstPlainMax ? 1 : 0};
     auto itg = ctx->graphs.find(key);
     cudaGraphExec_t exec = nullptr;

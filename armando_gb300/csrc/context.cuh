@@ -20,12 +20,13 @@ using namespace ag;
 struct GraphKey {
     float kdt, hdt, dt;
     int heat_on;
-    int par;  // 0: one state buffer; 1, 2: which of the two is current (fused predictor)
-    int lst;  // neighbour lists in use
-    int first;  // a lazily sorting call's first step, which always sorts
+    const void* state;  // which of the context's state buffers is current (they swap roles)
+    int fused;          // the fused predictor
+    int lst;            // neighbour lists in use
+    int first;          // a lazily sorting call's first step, which always sorts
     bool operator<(const GraphKey& o) const {
-        return std::tie(kdt, hdt, dt, heat_on, par, lst, first) <
-               std::tie(o.kdt, o.hdt, o.dt, o.heat_on, o.par, o.lst, o.first);
+        return std::tie(kdt, hdt, dt, heat_on, state, fused, lst, first) <
+               std::tie(o.kdt, o.hdt, o.dt, o.heat_on, o.state, o.fused, o.lst, o.first);
     }
 };
 
@@ -171,9 +172,8 @@ struct armando_ctx {
     OpenSpec open{};
     StateA A2{};
     // Fused predictor (lazily sorting, lean physics, lists): the force pass
-    // writes the next state into A_alt, then the two swap; acur counts swaps.
+    // writes the next state into A_alt, then the two swap.
     StateA A_alt{};
-    int acur = 0;
     bool open_ready = false;
     int *open_keep = nullptr, *d_open_n = nullptr, *h_open_n = nullptr;
     unsigned *open_tc = nullptr, *open_to = nullptr;
