@@ -312,8 +312,8 @@ __device__ __forceinline__ void shear_m(const float4& a, const float4& b, float4
 }
 
 // Forward geometry of two pairs shared by the adjoint gathers: differences, r^2, the
-// gradient factor G and G'(r)/r (0 for a coincident pair), h_i + h_j. An absent entry
-// is the particle itself: d = 0, and every cotangent below vanishes.
+// gradient factor G and G'(r)/r (0 for a coincident pair), h_i + h_j. G < 0 within the
+// support; an absent entry is out of reach (kOutOfReach), where both are zero.
 template <int DIM>
 struct PairGeo2 {
     f2 d[3], dr2, G, dG, hs;
@@ -410,14 +410,17 @@ __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
         const int ml = __reduce_max_sync(0xffffffffu, nl);
         for (int t = 0; t < ml; t += 2) {
             const int ja = t < nl ? s_list[t][tid] : kself, jb = t + 1 < nl ? s_list[t + 1][tid] : kself;
-            const float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            if (t >= nl) xa.x = kOutOfReach;
+            if (t + 1 >= nl) xb.x = kOutOfReach;
             const float4 va = __ldg(B.vm + ja), vb = __ldg(B.vm + jb);
             const float4 ra = __ldg(B.rp + ja), rb = __ldg(B.rp + jb);
             const float4 ca = __ldg(abar + ja), cb = __ldg(abar + jb);
             const f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
             PairGeo2<DIM> pg;
             pair_geo2<DIM>(xi, xa, xb, g, P, pg);
-            const f2 rs = make_float2(rpi.x + ra.x, rpi.x + rb.x);  // 2 rho_bar
+            // 2 rho_bar (a particle without density is its own absent entry: not 0)
+            const f2 rs = make_float2(pg.G.x < 0.f ? rpi.x + ra.x : 1.f, pg.G.y < 0.f ? rpi.x + rb.x : 1.f);
             const f2 w0 = make_float2(va.x - vi.x, vb.x - vi.x), w1 = make_float2(va.y - vi.y, vb.y - vi.y);
             const f2 w2 = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : z2;
             // The rates of s and of j from the pair: with d = x_s - x_j, w = v_j - v_s,
@@ -439,7 +442,7 @@ __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
                     ad = fma2(bc2(abi.z), pg.d[2], ad);
                 }
                 const f2 Sb = neg2(fma2(hb, wd, Ad));
-                f2 T = make_float2(rpi.y + ra.y, rpi.y + rb.y);
+                f2 T = within2(pg.G, make_float2(rpi.y + ra.y, rpi.y + rb.y));
                 f2 Tb = mul2(pg.G, Sb), rv = z2, r2b = z2;
                 if (P.visc_art) {  // Pi = (beta phi - alpha c0) phi / rho_bar, phi = mh vr / den, vr = -w.d < 0
                     const f2 mh = mul2(pg.hs, bc2(0.5f));
@@ -485,7 +488,7 @@ __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
                 const f2 q = mul2(iden, irho);  // 1 / (rho_bar den)
                 const f2 Ah = mul2(mul2(pg.G, pg.dr2), q);
                 const f2 dA = fma2(fma2(mul2(bc2(0.5f), pg.dG), pg.dr2, pg.G), q, neg2(mul2(Ah, iden)));
-                const f2 ps = make_float2(rpi.w + ra.w, rpi.w + rb.w);
+                const f2 ps = within2(pg.G, make_float2(rpi.w + ra.w, rpi.w + rb.w));
                 f2 lo = z2;
                 if (B.ulo) lo = make_float2(uloi - __ldg(B.ulo + ja), uloi - __ldg(B.ulo + jb));
                 const f2 du = add2(make_float2(rpi.z - ra.z, rpi.z - rb.z), lo);
@@ -779,7 +782,9 @@ __global__ void __launch_bounds__(kPassThreads)
         const int ml = __reduce_max_sync(0xffffffffu, nl);
         for (int t = 0; t < ml; t += 2) {
             const int ja = t < nl ? s_list[t][tid] : kself, jb = t + 1 < nl ? s_list[t + 1][tid] : kself;
-            const float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            float4 xa = __ldg(B.xh + ja), xb = __ldg(B.xh + jb);
+            if (t >= nl) xa.x = kOutOfReach;
+            if (t + 1 >= nl) xb.x = kOutOfReach;
             float4 va = make_float4(0.f, 0.f, 0.f, 0.f), vb = va;
             if (DIM == 3 || ah) {
                 va = __ldg(B.vm + ja);
@@ -788,14 +793,15 @@ __global__ void __launch_bounds__(kPassThreads)
             const f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
             PairGeo2<DIM> pg;
             pair_geo2<DIM>(xi, xa, xb, g, P, pg);
-            const f2 c = mul2(fma2(bc2(rbi), mj, mul2(bc2(mi), make_float2(__ldg(rhobar + ja), __ldg(rhobar + jb)))),
-                              pg.G);
+            const f2 wr = fma2(bc2(rbi), mj, mul2(bc2(mi), make_float2(__ldg(rhobar + ja), __ldg(rhobar + jb))));
+            const f2 c = mul2(within2(pg.G, wr), pg.G);
 #pragma unroll
             for (int k = 0; k < DIM; ++k) xb2[k] = fma2(c, pg.d[k], xb2[k]);
             if (ah) {
                 // d/d(vh_s), d/d(x_s) of divs_s (weight dsb_s m_j) and of divs_j
                 // (weight dsb_j m_s, d_js = -d, w_js = -w): the same forms.
-                const f2 cd = fma2(bc2(dsi), mj, mul2(bc2(mi), make_float2(__ldg(divsb + ja), __ldg(divsb + jb))));
+                const f2 cd = within2(
+                    pg.G, fma2(bc2(dsi), mj, mul2(bc2(mi), make_float2(__ldg(divsb + ja), __ldg(divsb + jb)))));
                 const f2 w[3] = {make_float2(va.x - vi.x, vb.x - vi.x), make_float2(va.y - vi.y, vb.y - vi.y),
                                  DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : z2};
                 f2 wd = fma2(w[1], pg.d[1], mul2(w[0], pg.d[0]));

@@ -26,6 +26,12 @@ __device__ __forceinline__ f2 min2(f2 a, float b) { return make_float2(fminf(a.x
 constexpr float kTinyDr2 = 1.0e-37f;
 // a b rounded, also where an addition takes it (for results above 1e-29).
 __device__ __forceinline__ f2 prod2(f2 a, f2 b) { return __ffma2_rn(a, b, make_float2(kTinyDr2, kTinyDr2)); }
+// The x coordinate given to an absent entry (the odd end of a list, a lane whose list is
+// shorter than its neighbours'), which otherwise repeats the particle itself: beyond
+// every support, where the kernel's gradient is zero. At d = 0, where it is largest, the
+// rounding of two products that should cancel, an infinite P or the quotient of a
+// vanishing r^2 would stay.
+constexpr float kOutOfReach = 1.0e18f;
 // v where t < 0, else 0 (also in place of an infinity or NaN).
 __device__ __forceinline__ f2 within2(f2 t, f2 v) {
     return make_float2(t.x < 0.f ? v.x : 0.f, t.y < 0.f ? v.y : 0.f);
