@@ -2495,7 +2495,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
         const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
                          : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);
-        const f2 rc = rcp2(mul2(D, rs));
+        const f2 rc = rcp_prod2(D, rs);
         const f2 A = mul2(max2(vr, 0.0f), rc);
         const f2 ka2 = UNI ? bc2(k_alpha * (2.0f * xi.w)) : mul2(bc2(k_alpha), hs);
         f2 V = DIM == 2 ? mul2(A, ka2) : fma2(A, ka2, T);  // Pi_ij (3D: and T)
@@ -2548,7 +2548,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         if ((PH & 1) && heat_art) {  // art_heat.f:69-97: grad W . d = G r^2
             f2 rh = rc;
             if (P.ah_eta2 != P.av_eta2)
-                rh = rcp2(mul2(fma2(hs2, bc2(0.25f * P.ah_eta2), dr2), rs));
+                rh = rcp_prod2(fma2(hs2, bc2(0.25f * P.ah_eta2), dr2), rs);
             float4 qa = ra, qb = rb;
             if (DIM == 2) {  // u and psi are not in the 2D record
                 qa = __ldg(B.rp + ka);
