@@ -2392,9 +2392,13 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     const int lc = lpk >= 0 ? list_near(lpk) + list_far(lpk) : -1;  // entries (-1: no list)
     if (LST) prefetch_list(B.nlist, B.lstride, s, lc);
     // The place of an absent entry (the odd end of a list, a lane without
-    // entries): the particle itself, whose terms vanish with d = 0 and dv = 0.
+    // entries): the particle itself, whose terms vanish with d = 0 and dv = 0 unless
+    // one of its own values is infinite (a particle without mass that is alone has no
+    // density). So lists put it out of reach, where the kernel is zero, and the cell
+    // walk selects (ina, inb below).
     int kself = valid ? s : 0;
     if (STG) kself = work ? s + SV.shift[DIM == 2 ? g.reach : g.reach * (2 * g.reach + 2)] : 0;
+    const float rho_i = rpi.x != 0.f ? rpi.x : 1.f;  // (no mass near it: all m_j are 0)
     const float k_alpha = P.visc_art ? P.av_alpha * P.c0 : 0.f;        // times h_i + h_j
     const float k_beta = P.visc_art ? 0.5f * P.av_beta : 0.f;          // times (h_i + h_j)^2
     // Push between particles of different type (ArmandoThrust/armando.cu:507-513
@@ -2426,7 +2430,8 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     // {rho, P, u, psi}. No pair test: the kernel's gradient is zero beyond its
     // support, so the entries in the skin margin add nothing. P of a particle
     // without density (no mass near it) is not finite, and a zero gradient times
-    // it no zero: within2 leaves the margin's P out.
+    // it no zero: `taking` leaves out what the margin and absent entries have there.
+    // ina, inb: whether the entries are real (without lists).
     //
     // Pressure, art_visc and their energy rates share one factor per pair: with
     // s = m_j G (grad W = G d), T = P_i + P_j + Pi_ij and dv = v_j - v_i,
@@ -2447,8 +2452,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     // UNI: every particle has the same h (g.huni), whose factors are constants.
     // PH: the physics beyond pressure and art_visc compiled in, bits 1 art_heat,
     // 2 physical viscosity, 4 repulsive walls and the single_step options.
-    auto pair2 = [&](auto uni, auto ph, const int ka, const int kb, const float4& xa, const float4& xb,
-                     const float4& va, const float4& vb, const float4& ra, const float4& rb) {
+    auto pair2 = [&](auto uni, auto ph, const bool ina, const bool inb, const int ka, const int kb,
+                     const float4& xa, const float4& xb, const float4& va, const float4& vb, const float4& ra,
+                     const float4& rb) {
         constexpr bool UNI = decltype(uni)::value;
         constexpr int PH = decltype(ph)::value;
         f2 d0 = make_float2(xi.x - xa.x, xi.x - xb.x), d1 = make_float2(xi.y - xa.y, xi.y - xb.y);
@@ -2471,6 +2477,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         // q - 2, 0 beyond the support
         const f2 t = min2(DIM == 2 ? add2(prod2(r, ih), bc2(-2.0f)) : fma2(r, ih, bc2(-2.0f)), 0.0f);
         const f2 tt = mul2(t, t);
+        auto taking = [&](f2 v) {
+            return LST ? within2(t, v) : make_float2(ina ? v.x : 0.f, inb ? v.y : 0.f);
+        };
         const f2 rhoj = DIM == 2 ? make_float2(va.z, vb.z) : make_float2(ra.x, rb.x);
         if ((PH & 4) && repulsive_walls(P)) {
             push(ka, xa, rhoj.x, d0.x, d1.x, d2.x, dr2.x, tt.x, t.x, ih.x, mj.x, a0, a1, a2);
@@ -2482,16 +2491,16 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         const f2 vz = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : zero2;
         f2 vr = fma2(vy, d1, mul2(vx, d0));
         if (DIM == 3) vr = fma2(vz, d2, vr);
-        const f2 rs = make_float2(rpi.x + rhoj.x, rpi.x + rhoj.y);
+        const f2 rs = make_float2(rho_i + rhoj.x, rho_i + rhoj.y);
         f2 T = DIM == 2 ? make_float2(rpi.y + va.w, rpi.y + vb.w) : make_float2(rpi.y + ra.y, rpi.y + rb.y);
         f2 sv = sm;  // the viscous terms' factor
         if (P.pa_sph != 1) {
             f2 irr = rcp2(mul2(bc2(rpi.x), rhoj));
-            if (LST && (PH & 2)) irr = within2(t, irr);
+            if (PH & 2) irr = taking(irr);
             T = mul2(T, irr);
             sv = mul2(sv, irr);
         }
-        if (LST) T = within2(t, T);
+        T = taking(T);
         const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
         const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
                          : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);
@@ -2516,7 +2525,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         e_sum = dot2(c, vr, e_sum);
         if (cont) drho_s = dot2(neg2(sm), vr, drho_s);  // con_density, density.f:203-216
         if (sle2) {                                   // hsml.f:75-90
-            const f2 dq = within2(t, make_float2(__fdiv_rn(sm.x, rhoj.x), __fdiv_rn(sm.y, rhoj.y)));
+            const f2 dq = taking(make_float2(__fdiv_rn(sm.x, rhoj.x), __fdiv_rn(sm.y, rhoj.y)));
             divh = dot2(dq, vr, divh);
         }
         if (xsph) {  // av_vel.f:47-58: -eps m_j / rho_ij (v_i - v_j) W_ij, eps = 0.3
@@ -2557,8 +2566,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             const f2 ps = make_float2(rpi.w + qa.w, rpi.w + qb.w);
             const f2 lo = make_float2(ulo_i - __ldg(B.ulo + ka), ulo_i - __ldg(B.ulo + kb));
             const f2 du2 = add2(make_float2(rpi.z - qa.z, rpi.z - qb.z), lo);
-            f2 pr = mul2(ps, rh);
-            if (LST) pr = within2(t, pr);
+            const f2 pr = taking(mul2(ps, rh));
             ah_du = dot2(mul2(mul2(mul2(sm, dr2), pr), bc2(2.0f)), du2, ah_du);
         }
     };
@@ -2587,9 +2595,14 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
                     va[u] = __ldg((DIM == 2 ? B.vr : B.vm) + kb[v + u]);
                     rb[u] = DIM == 3 ? __ldg(B.rp + kb[v + u]) : va[u];
                 }
+                if (lc < 4 * b + v + NB) {  // the list ends here
+#pragma unroll
+                    for (int u = 0; u < NB; ++u)
+                        if (4 * b + v + u >= lc) xb[u].x = kOutOfReach;
+                }
 #pragma unroll
                 for (int u = 0; u < NB; u += 2)
-                    pair2(uni, ph, kb[v + u], kb[v + u + 1], xb[u], xb[u + 1], va[u], va[u + 1], rb[u], rb[u + 1]);
+                    pair2(uni, ph, true, true, kb[v + u], kb[v + u + 1], xb[u], xb[u + 1], va[u], va[u + 1], rb[u], rb[u + 1]);
             }
         }
         if (lc >= 0) done = true;
@@ -2699,8 +2712,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
                 xb[u] = STG ? SV.x[k] : __ldg(xsrc + k);
                 va[u] = STG ? SV.v[k] : __ldg((DIM == 2 ? B.vr : B.vm) + k);
                 rb[u] = DIM == 2 ? va[u] : STG ? SV.r[k] : __ldg(B.rp + k);
+                if (LST && t + u >= nl) xb[u].x = kOutOfReach;
             }
-            pair2(uni, ph, kb[0], kb[1], xb[0], xb[1], va[0], va[1], rb[0], rb[1]);
+            pair2(uni, ph, t < nl, t + 1 < nl, kb[0], kb[1], xb[0], xb[1], va[0], va[1], rb[0], rb[1]);
         }
     }
     };
