@@ -24,9 +24,6 @@ __device__ __forceinline__ f2 min2(f2 a, float b) { return make_float2(fminf(a.x
 // distance above 1e-15 times the unit, and a coincident pair (or a particle
 // with itself) gets r = 0 without a comparison.
 constexpr float kTinyDr2 = 1.0e-37f;
-// Added to a product whose reciprocal is taken: 1/(a b) of a product that would flush is
-// finite, and no product above 1e-30 changes.
-constexpr float kTinyDen = 1.2e-38f;
 // a b rounded, also where an addition takes it (for results above 1e-29).
 __device__ __forceinline__ f2 prod2(f2 a, f2 b) { return __ffma2_rn(a, b, make_float2(kTinyDr2, kTinyDr2)); }
 // The x coordinate given to an absent entry (the odd end of a list, a lane whose list is
@@ -55,8 +52,9 @@ __device__ __forceinline__ float rsqrt_fast(float a) {
     return r;
 }
 __device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp_fast(a.x), rcp_fast(a.y)); }
-// 1 / (a b) for a b >= 0.
-__device__ __forceinline__ f2 rcp_prod2(f2 a, f2 b) { return rcp2(__ffma2_rn(a, b, make_float2(kTinyDen, kTinyDen))); }
+// 1 / (a b) for a b >= 0, finite also where the product vanishes (prod2's constant: no
+// register pair of its own).
+__device__ __forceinline__ f2 rcp_prod2(f2 a, f2 b) { return rcp2(prod2(a, b)); }
 __device__ __forceinline__ f2 rsqrt2(f2 a) { return make_float2(rsqrt_fast(a.x), rsqrt_fast(a.y)); }
 
 // ---- float-float on two values at once (hi + lo each; sph_math.cuh's forms) ----
