@@ -2536,10 +2536,10 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
         }
         if (xsph) {  // av_vel.f:47-58: -eps m_j / rho_ij (v_i - v_j) W_ij, eps = 0.3
             const f2 ih2 = mul2(ih, ih);
-            // W = kw ih^dim (q - 2)^4 (2 (q - 2) + 5) / 16; 1 / rho_bar = 2 D rc
+            // W = kw ih^dim (q - 2)^4 (2 (q - 2) + 5) / 16; 0.3 / rho_bar = 0.6 / rs
             f2 wv = mul2(mul2(mul2(tt, tt), fma2(bc2(2.0f), t, bc2(5.0f))), mul2(bc2(0.0625f * P.kw_hi), ih2));
             if (DIM == 3) wv = mul2(wv, ih);
-            const f2 cx = mul2(mul2(mul2(bc2(0.6f), mj), wv), mul2(D, rc));
+            const f2 cx = taking(div2(mul2(mul2(bc2(0.6f), mj), wv), rs));
             x0s = dot2(cx, vx, x0s);
             x1s = dot2(cx, vy, x1s);
             if (DIM == 3) x2s = dot2(cx, vz, x2s);
