@@ -2211,13 +2211,14 @@ __device__ __forceinline__ void shear_body(const StateB& B, const unsigned* __re
             if (g.periodic[2]) d[2] = min_image2(d[2], xi.z, xa.z, xb.z, g, 2);
             dr2 = fma2(d[2], d[2], dr2);
         }
-        const f2 ih = mul2(bc2(2.0f), rcp2(make_float2(xi.w + xa.w, xi.w + xb.w)));
+        const f2 hs = make_float2(xi.w + xa.w, xi.w + xb.w);
+        const f2 ih = mul2(bc2(2.0f), rcp2_rn(hs, rcp2(hs)));
         const f2 ih2 = mul2(ih, ih);
         f2 kg = mul2(bc2(P.kg), mul2(ih2, ih2));
         if (DIM == 3) kg = mul2(kg, ih);
-        const f2 t = min2(fma2(mul2(dr2, rsqrt2(dr2)), ih, bc2(-2.0f)), 0.0f);
-        const f2 rj = within2(t, rcp2(make_float2(__ldg(&B.rp[ka].x), __ldg(&B.rp[kb].x))));
-        const f2 c = mul2(mul2(mul2(mul2(t, t), t), kg), mul2(mj, rj));
+        const f2 t = min2(fma2(sqrt2(dr2, rsqrt2(dr2)), ih, bc2(-2.0f)), 0.0f);
+        const f2 mr = within2(t, div2(mj, make_float2(__ldg(&B.rp[ka].x), __ldg(&B.rp[kb].x))));
+        const f2 c = mul2(mul2(mul2(mul2(t, t), t), kg), mr);
 #pragma unroll
         for (int a = 0; a < DIM; ++a) {
             const f2 u = mul2(c, dv[a]);
