@@ -1826,7 +1826,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                 const f2 f = mul2(mul2(t2, t2), fma2(q, bc2(2.0f), bc2(1.0f)));
                 const f2 m = UNI ? mul2(mj, f) : fma2(cm.hi, f, mul2(cm.lo, f));
                 if ((PH & 4) && nor)
-                    acc_ff2(Wh, Wl, mul2(m, rcp2(rho_in(ka, kb, t))));
+                    acc_ff2(Wh, Wl, div2(m, rho_in(ka, kb, t)));
                 if (UNI && kFarOwn) {
                     const ff2 c = mul_ff2_f(ff2{bc2(al_i.hi), bc2(al_i.lo)}, mj);
                     acc_ff2(Fh, Fl, fma2(c.hi, f, mul2(c.lo, f)));
