@@ -331,14 +331,15 @@ __device__ __forceinline__ void pair_geo2(const float4& xi, const float4& xa, co
     o.dr2 = fma2(o.d[1], o.d[1], fma2(o.d[0], o.d[0], bc2(kTinyDr2)));
     if (DIM == 3) o.dr2 = fma2(o.d[2], o.d[2], o.dr2);
     o.hs = make_float2(xi.w + xa.w, xi.w + xb.w);
-    const f2 ih = mul2(bc2(2.0f), rcp2(o.hs)), ih2 = mul2(ih, ih);
+    const f2 ih = mul2(bc2(2.0f), rcp2_rn(o.hs, rcp2(o.hs))), ih2 = mul2(ih, ih);
     f2 kg = mul2(bc2(P.kg), mul2(ih2, ih2));
     if (DIM == 3) kg = mul2(kg, ih);
     const f2 rs = rsqrt2(o.dr2);
-    const f2 t = min2(fma2(mul2(o.dr2, rs), ih, bc2(-2.0f)), 0.0f);
+    const f2 r = sqrt2(o.dr2, rs);
+    const f2 t = min2(fma2(r, ih, bc2(-2.0f)), 0.0f);
     const f2 kt = mul2(kg, mul2(t, t));
     o.G = mul2(kt, t);
-    o.dG = mul2(mul2(kt, mul2(ih, bc2(3.0f))), rs);
+    o.dG = mul2(mul2(kt, mul2(ih, bc2(3.0f))), rcp2_rn(r, rs));
     if (!(o.dr2.x > 2.0f * kTinyDr2)) o.dG.x = 0.f;
     if (!(o.dr2.y > 2.0f * kTinyDr2)) o.dG.y = 0.f;
 }
@@ -447,18 +448,19 @@ __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
                 if (P.visc_art) {  // Pi = (beta phi - alpha c0) phi / rho_bar, phi = mh vr / den, vr = -w.d < 0
                     const f2 mh = mul2(pg.hs, bc2(0.5f));
                     const f2 den = fma2(mul2(mh, mh), bc2(P.av_eta2), pg.dr2);
-                    const f2 rc = rcp2(mul2(den, rs));
-                    const f2 iden = mul2(rc, rs), irho = mul2(mul2(rc, den), bc2(2.0f));
-                    const f2 phi = mul2(mul2(mh, neg2(max2(wd, 0.0f))), iden);
-                    const f2 pf = mul2(phi, irho);
+                    const f2 rho = mul2(bc2(0.5f), rs), yd = rcp2(den), yr = rcp2(rho);
+                    const f2 phi = div2(mul2(mh, neg2(max2(wd, 0.0f))), den, yd);
+                    const f2 pf = div2(phi, rho, yr);
                     const f2 pv = mul2(fma2(bc2(P.av_beta), phi, bc2(-P.av_alpha * P.c0)), pf);
                     T = add2(T, pv);
-                    rb2 = fma2(mul2(bc2(-0.5f), Tb), mul2(pv, irho), rb2);
-                    f2 phib = mul2(mul2(Tb, irho), fma2(bc2(2.0f * P.av_beta), phi, bc2(-P.av_alpha * P.c0)));
+                    const f2 Tr = div2(Tb, rho, yr);
+                    rb2 = fma2(mul2(bc2(-0.5f), Tr), pv, rb2);
+                    f2 phib = mul2(Tr, fma2(bc2(2.0f * P.av_beta), phi, bc2(-P.av_alpha * P.c0)));
                     if (!(wd.x > 0.f)) phib.x = 0.f;
                     if (!(wd.y > 0.f)) phib.y = 0.f;
-                    rv = mul2(mul2(phib, mh), iden);         // vr_bar
-                    r2b = mul2(mul2(phib, neg2(phi)), iden);  // (r^2)_bar
+                    const f2 pd = div2(phib, den, yd);
+                    rv = mul2(pd, mh);          // vr_bar
+                    r2b = mul2(pd, neg2(phi));  // (r^2)_bar
                     // the parameters: the rates of s alone
                     const f2 Ts = mul2(mul2(mj, pg.G), neg2(fma2(bc2(0.5f * abi.w), wd, ad)));
                     const f2 x = mul2(Ts, pf);
@@ -483,8 +485,8 @@ __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
                 // (e + r^2)): weights du_bar_s m_j - du_bar_j m_s on the pair (s, j).
                 const f2 mh = mul2(pg.hs, bc2(0.5f));
                 const f2 den = fma2(mul2(mh, mh), bc2(P.ah_eta2), pg.dr2);
-                const f2 rc = rcp2(mul2(den, rs));
-                const f2 iden = mul2(rc, rs), irho = mul2(mul2(rc, den), bc2(2.0f));
+                const f2 rho = mul2(bc2(0.5f), rs);
+                const f2 iden = rcp2_rn(den, rcp2(den)), irho = rcp2_rn(rho, rcp2(rho));
                 const f2 q = mul2(iden, irho);  // 1 / (rho_bar den)
                 const f2 Ah = mul2(mul2(pg.G, pg.dr2), q);
                 const f2 dA = fma2(fma2(mul2(bc2(0.5f), pg.dG), pg.dr2, pg.G), q, neg2(mul2(Ah, iden)));
