@@ -2162,15 +2162,18 @@ armando_status apply_tuning(armando_ctx* ctx, const armando_tuning& t) {
     ctx->next_its = 0;  // the device state no longer belongs to the last call
     free_graphs(ctx);
     // Neighbour lists for a lazily sorting step with one lane per particle,
-    // allocated on first use and kept.
+    // allocated on first use and kept. The GPU-C schemes run without where they do not fit.
     if (ctx->lists && lazy(ctx) && t.threads_per_particle == 1 && !ctx->B.nlist && ctx->prm.wall_model != 3) {
         const int lcap = ctx->dim == 2 ? kListCap2 : kListCap3;
         cudaError_t e = cudaSuccess;
         int* nl = dalloc<int>((size_t)list_blocks(lcap) * 4 * (size_t)std::max<int64_t>(ctx->cap, 1), e);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(neighbour lists)");
+        int* nc = e == cudaSuccess ? dalloc<int>((size_t)std::max<int64_t>(ctx->cap, 1), e) : nullptr;
+        if (e != cudaSuccess) {
+            cudaFree(nl);
+            armando_status st = cuda_fail(ctx, e, "cudaMalloc(neighbour lists)");
+            return st == ARMANDO_ERR_OOM && ctx->prm.scheme != 0 ? ARMANDO_OK : st;
+        }
         ctx->owned.push_back(nl);
-        int* nc = dalloc<int>((size_t)std::max<int64_t>(ctx->cap, 1), e);
-        if (e != cudaSuccess) return cuda_fail(ctx, e, "cudaMalloc(neighbour counts)");
         ctx->owned.push_back(nc);
         ctx->B.nlist = nl;
         ctx->B.ncount = nc;
