@@ -651,11 +651,9 @@ armando_status run_ghost_step(armando_ctx* ctx, const StepArgs& S) {
             return fail(ctx, ARMANDO_ERR_CUDA, "mirror ghost count out of range");
     }
     ctx->n_work = (int64_t)n + ng;
-    ctx->num_tiles = blocks_for(ctx->n_work, kSortTile);
     L += launch_grid_and_sort<DIM>(ctx, nullptr, st);
     L += launch_passes<DIM>(ctx, S, nullptr);
     ctx->n_work = n;
-    ctx->num_tiles = blocks_for(n, kSortTile);
     CK(cudaGetLastError());
     ctx->ghosts_last = ng;
     ctx->launches += L;
@@ -813,7 +811,6 @@ armando_status alloc_state(armando_ctx* ctx) {
     ctx->B.mstride = (int)n;
     ctx->B.mtpp = 1;
     ctx->owned.push_back(ctx->B.nmask);
-    ctx->num_tiles = blocks_for(ctx->cap, kSortTile);  // sizes the histogram; set per sort below
     for (int k = 0; k < 2; ++k) {
         ctx->keys[k] = dalloc<unsigned>(n, e);
         ctx->vals[k] = dalloc<int>(n, e);
@@ -824,8 +821,7 @@ armando_status alloc_state(armando_ctx* ctx) {
     ctx->owned.push_back(ctx->placed);
     ctx->ticket = dalloc<unsigned>(1, e);
     ctx->owned.push_back(ctx->ticket);
-    ctx->hist = dalloc<unsigned>((size_t)kRadix * std::max(ctx->num_tiles, 1), e);
-    ctx->num_tiles = blocks_for(ctx->n, kSortTile);
+    ctx->hist = dalloc<unsigned>((size_t)kRadix * std::max(blocks_for(ctx->cap, kSortTile), 1), e);
     ctx->dtotal = dalloc<unsigned>(kRadix, e);
     ctx->bbox_part = dalloc<float>(kBBoxBlocks * 8, e);
     // the status words and the grid, side by side: one copy brings both to the host.
@@ -1525,7 +1521,7 @@ armando_status load_inputs(armando_ctx* ctx, const float* x, const float* vx, co
                                                             rfl, pfl, ctx->flags + 2);
     ctx->launches += 1;
     CK(cudaGetLastError());
-    return nn > 0 ? ARMANDO_OK : force_sort(ctx);
+    return ARMANDO_OK;
 }
 
 // A -> device arrays: below this size each slot writes its particle where the caller
@@ -2496,7 +2492,6 @@ armando_status armando_integrate_open(armando_ctx* ctx, float* x, float* vx, flo
         st = ctx->dim == 2 ? remove_outflow<2>(ctx, n) : remove_outflow<3>(ctx, n);
         if (st != ARMANDO_OK || n == 0) continue;
         ctx->n_work = n;
-        ctx->num_tiles = blocks_for(n, kSortTile);
         const StepArgs S = make_args(ctx, dt, its0 + k);
         const int L = ctx->dim == 2 ? launch_gpuc_step<2>(ctx, S, nullptr)
                                     : launch_gpuc_step<3>(ctx, S, nullptr);  // the count changes: sort
@@ -2504,12 +2499,10 @@ armando_status armando_integrate_open(armando_ctx* ctx, float* x, float* vx, flo
         ctx->steps_done += 1;
         ctx->sorts_host += 1;
         ctx->n_work = ctx->n;
-        ctx->num_tiles = blocks_for(ctx->n, kSortTile);
         cudaError_t e = cudaGetLastError();
         if (e != cudaSuccess) st = cuda_fail(ctx, e, "kernel launch");
     }
     ctx->n_work = ctx->n;
-    ctx->num_tiles = blocks_for(ctx->n, kSortTile);
     if (st != ARMANDO_OK) return st;
     st = ctx->dim == 2 ? store_open<2>(ctx, n, x, vx, mass, rho, p, u, hsml, itype, dvdt, dudt)
                        : store_open<3>(ctx, n, x, vx, mass, rho, p, u, hsml, itype, dvdt, dudt);

@@ -80,7 +80,6 @@ struct armando_ctx {
     unsigned* ticket = nullptr;  // k_bbox_grid
     unsigned* hist = nullptr;
     unsigned* dtotal = nullptr;
-    int num_tiles = 0;
     int* start = nullptr;
     long long cell_cap = 0;
     float* bbox_part = nullptr;

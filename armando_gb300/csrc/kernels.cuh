@@ -2008,7 +2008,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
         }
     } else {
         Cursor cu = cursor_begin<DIM>(g);
-        int shift = 0;  // staged index - slot in the cursor's row
+        static_assert(!STG, "staged passes: one lane per particle");
         while (__any_sync(0xffffffffu, !done)) {
             int nn = 0, nf = 0;
             // Test phase: fill the near / far lists, kTestBatch candidate loads in flight.
@@ -2021,11 +2021,8 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                         done = true;
                         break;
                     }
-                    if (STG) shift = SV.shift[cursor_row<DIM>(cu, g.reach)];
-                    if (TPP > 1) {
-                        cu.k += sub;
-                        continue;
-                    }
+                    cu.k += sub;
+                    continue;
                 }
                 if (nn > cap_density<LST>() - kTestBatch || nf > cap_density<LST>() - kTestBatch) break;
                 const int k0 = cu.k;
@@ -2034,7 +2031,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                 for (int u = 0; u < kTestBatch; ++u) {
                     const int ku = min(k0 + u * TPP, cu.ke - 1);
                     kb[u] = k0 + u * TPP;
-                    xb[u] = STG ? SV.x[ku + shift] : __ldg(xsrc + ku);
+                    xb[u] = __ldg(xsrc + ku);
                 }
                 cu.k += cnt * TPP;
                 unsigned pb = 0u;  // pass bits of this batch
@@ -2045,11 +2042,10 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
                     if (u >= cnt || k == s || !pair_delta<DIM>(xi, xb[u], g, d, dr2)) continue;
                     pb |= 1u << u;
                     const float hs = xi.w + xb[u].w;  // near: q < near_q() with h = hs/2
-                    const LT e = (LT)(STG ? k + shift : k);
                     if (DIM == 3 || dr2 < (0.25f * near_q<DIM>() * near_q<DIM>()) * hs * hs)
-                        s_near[nn++][tid] = e;
+                        s_near[nn++][tid] = (LT)k;
                     else
-                        s_far[nf++][tid] = e;
+                        s_far[nf++][tid] = (LT)k;
                 }
                 if (ord - 32 * wb >= 32) {  // word wb is complete
                     if (mask_on && wb < W) B.nmask[mask_word_index<W>(wb, B.mstride, mlane)] = (unsigned)cur;

@@ -51,12 +51,6 @@ SPH_HD ff two_diff(float a, float b) {
     float e = __fsub_rn(__fsub_rn(a, __fsub_rn(s, bb)), __fadd_rn(b, bb));
     return {s, e};
 }
-// Dekker Fast2Sum, requires |a| >= |b|.
-SPH_HD ff fast_two_sum(float a, float b) {
-    float s = __fadd_rn(a, b);
-    float e = __fsub_rn(b, __fsub_rn(s, a));
-    return {s, e};
-}
 // a * b == p + e exactly (fused multiply-add residual).
 SPH_HD ff two_prod(float a, float b) {
     float p = __fmul_rn(a, b);
