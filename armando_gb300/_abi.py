@@ -269,6 +269,7 @@ EXPORTED = [
 ]
 N_TUNINGS = 27
 N_PHASES = 6
+# ("radix_sort": the sort phase, a counting sort; callers index by the name)
 PHASE_NAMES = ["grid_hash", "radix_sort", "cells_reorder", "density", "shear", "force"]
 
 _lib = None

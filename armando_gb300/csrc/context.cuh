@@ -53,7 +53,9 @@ struct armando_ctx {
     // memory through L1; both give the same bits).
     bool staging = false;
     // Neighbour lists between sorts (ARMANDO_NEIGHBOUR_LISTS=0 at creation:
-    // walk the cells every iteration; 2D results are the same bits).
+    // walk the cells every iteration; the GPU-C schemes' results are the same bits, the
+    // CERN step's differ by the rounding of its sums: in 2D the split of near and far
+    // pairs is another one and a far pair's weight is rounded by itself).
     bool lists = true;
     // Fused predictor on the iterations between sorts (ARMANDO_FUSED_PREDICTOR=0
     // at creation: a reorder copy every iteration; the same bits).
