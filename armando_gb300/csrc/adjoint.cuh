@@ -346,9 +346,9 @@ __device__ __forceinline__ void pair_geo2(const float4& xi, const float4& xa, co
 
 // EXT: artificial heat or physical viscosity is on; without them their operands are
 // compiled out. The pair's two directions share one set of terms, on two neighbours
-// at a time, with two reciprocals a pair; formed apart, with nine divisions each, they
-// took 152 us at 260,904 particles (2D), now 71; EXT's operands are what
-// held it to three blocks an SM.
+// at a time, with two estimated reciprocals a pair that every quotient corrects (div2);
+// formed apart, with nine divisions each, they took 152 us at 260,904 particles (2D), now
+// 62; EXT's operands are what held it to three blocks an SM.
 template <int DIM, bool EXT>
 __global__ void __launch_bounds__(kPassThreads, EXT ? 3 : 5)
     k_adj_force(StateB B, const unsigned* __restrict__ keys, const int* __restrict__ start,
