@@ -2506,6 +2506,8 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             sv = mul2(sv, irr);
         }
         T = taking(T);
+        if ((PH & 4) && P.wall_model == 1)  // push only: the other's P is not part of it
+            T = make_float2(mj.x != 0.f ? T.x : 0.f, mj.y != 0.f ? T.y : 0.f);
         const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
         const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
                          : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);

@@ -1,0 +1,49 @@
+"""wall_model 1, where the push is the only interaction of particles of different type:
+the pressure that a wall carries plays no part. Walls whose pressure is infinite or not
+a number: the fluid's results are those of walls with none, to the bit, on the cells and
+on lists.
+"""
+import numpy as np
+import pytest
+
+import armando_gb300 as ag
+from armando_gb300 import cases
+from helpers import FIELDS
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module", autouse=True)
+def _lib():
+    from armando_gb300 import build
+
+    build.build_library()
+    ag.load_library()
+
+
+def _case(dim, p):
+    if dim == 2:
+        c = cases.perturbed(cases.dam_break(dx=0.04, jitter=0.1), seed=181, dv=0.1)
+    else:
+        c = cases.perturbed(cases.channel(n_x=16, n_yz=8, length=16 * 7.9e-4, width=8 * 7.9e-4, layers=2,
+                                          jitter=0.1), seed=182, dv=0.05, du=50.0)
+    c.params.wall_model = 1
+    c.p[c.itype <= 0] = p
+    return c
+
+
+@pytest.mark.parametrize("p", [np.nan, np.inf])
+@pytest.mark.parametrize("tuning", [(1, 1, 128, 0), (2, 1, 128, 20), (1, 2, 128, 0)])
+@pytest.mark.parametrize("dim", [2, 3])
+def test_wall_pressure_plays_no_part(dim, tuning, p):
+    out = []
+    for q in (0.0, p):
+        c = _case(dim, q)
+        with ag.Context(c.params, c.n_fluid, c.n_wall) as ctx:
+            ctx.set_tuning(*tuning)
+            ctx.step(c, c.dt, 1)
+        out.append(c)
+    fl = out[0].itype > 0
+    for f in FIELDS:
+        a, b = (getattr(c, f).reshape(c.n, -1)[fl] for c in out)
+        assert np.isfinite(b).all() and np.array_equal(a, b), f
