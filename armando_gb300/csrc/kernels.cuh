@@ -1848,6 +1848,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
             f2 vd = fma2(make_float2(va.y - vi.y, vb.y - vi.y), d1,
                          mul2(make_float2(va.x - vi.x, vb.x - vi.x), d0));
             if (DIM == 3) vd = fma2(make_float2(va.z - vi.z, vb.z - vi.z), d2, vd);
+            if ((PH & 4) && P.wall_model == 1) vd = make_float2(ina ? vd.x : 0.f, inb ? vd.y : 0.f);
             divs = dot2(gm, vd, divs);
         }
     };
@@ -2191,9 +2192,12 @@ __device__ __forceinline__ void shear_body(const StateB& B, const unsigned* __re
         const float4 xa = __ldg(B.xh + ka), xb = __ldg(B.xh + kb);
         const float4 va = __ldg(B.vm + ka), vb = __ldg(B.vm + kb);
         f2 mj = DIM == 2 ? make_float2(xa.z, xb.z) : make_float2(va.w, vb.w);
-        if (P.wall_model == 1) {  // push only
-            if (__ldg(B.itype + ka) != it_i) mj.x = 0.f;
-            if (__ldg(B.itype + kb) != it_i) mj.y = 0.f;
+        bool pa = false, pb = false;  // push only: nothing else of the other is read
+        if (P.wall_model == 1) {
+            pa = __ldg(B.itype + ka) != it_i;
+            pb = __ldg(B.itype + kb) != it_i;
+            if (pa) mj.x = 0.f;
+            if (pb) mj.y = 0.f;
         }
         f2 d[3], dv[3];
         d[0] = make_float2(xi.x - xa.x, xi.x - xb.x);
@@ -2209,6 +2213,8 @@ __device__ __forceinline__ void shear_body(const StateB& B, const unsigned* __re
             if (g.periodic[2]) d[2] = min_image2(d[2], xi.z, xa.z, xb.z, g, 2);
             dr2 = fma2(d[2], d[2], dr2);
         }
+#pragma unroll
+        for (int a = 0; a < DIM; ++a) dv[a] = make_float2(pa ? 0.f : dv[a].x, pb ? 0.f : dv[a].y);
         const f2 hs = make_float2(xi.w + xa.w, xi.w + xb.w);
         const f2 ih = mul2(bc2(2.0f), rcp2_rn(hs, rcp2(hs)));
         const f2 ih2 = mul2(ih, ih);
@@ -2408,10 +2414,10 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
     const float k_beta = P.visc_art ? 0.5f * P.av_beta : 0.f;          // times (h_i + h_j)^2
     // Push between particles of different type (ArmandoThrust/armando.cu:507-513
     // for wall_model 1, acpu.c:424-429 for 2) along (x_i - x_j)/r, c = c0; with
-    // wall_model 1 the pair's only interaction (its mass is zeroed).
+    // wall_model 1 the pair's only interaction: true, its mass zeroed.
     auto push = [&](const int k, const float4& xj, float rhoj, float e0, float e1, float e2, float dr2,
                     float tt, float t, float ih, float& mj, float& p0, float& p1, float& p2) {
-        if (__ldg(B.itype + k) == it) return;
+        if (__ldg(B.itype + k) == it) return false;
         const float r = fast_sqrt_pos(dr2);
         if (dr2 > 2.0f * kTinyDr2 && t < 0.f) {
             const float w = 0.0625f * tt * tt * fmaf(2.0f, t, 5.0f);  // W / W(0)
@@ -2428,7 +2434,9 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             p1 = fmaf(f, e1, p1);
             if (DIM == 3) p2 = fmaf(f, e2, p2);
         }
-        if (P.wall_model == 1) mj = 0.f;
+        if (P.wall_model != 1) return false;
+        mj = 0.f;
+        return true;
     };
     // Terms of two entries (pressure, viscosity, art_visc, art_heat, options).
     // va, vb: the neighbours' 2D {vx, vy, rho, P} (ra, rb unused) or 3D v and
@@ -2486,14 +2494,16 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             return LST ? within2(t, v) : make_float2(ina ? v.x : 0.f, inb ? v.y : 0.f);
         };
         const f2 rhoj = DIM == 2 ? make_float2(va.z, vb.z) : make_float2(ra.x, rb.x);
+        bool pa = false, pb = false;  // push only: nothing else of the other is read
         if ((PH & 4) && repulsive_walls(P)) {
-            push(ka, xa, rhoj.x, d0.x, d1.x, d2.x, dr2.x, tt.x, t.x, ih.x, mj.x, a0, a1, a2);
-            push(kb, xb, rhoj.y, d0.y, d1.y, d2.y, dr2.y, tt.y, t.y, ih.y, mj.y, a0, a1, a2);
+            pa = push(ka, xa, rhoj.x, d0.x, d1.x, d2.x, dr2.x, tt.x, t.x, ih.x, mj.x, a0, a1, a2);
+            pb = push(kb, xb, rhoj.y, d0.y, d1.y, d2.y, dr2.y, tt.y, t.y, ih.y, mj.y, a0, a1, a2);
         }
+        auto others = [&](f2 v) { return make_float2(pa ? 0.f : v.x, pb ? 0.f : v.y); };
         const f2 gw = mul2(mul2(mul2(kg, t), t), t);  // G (2D)
         const f2 sm = DIM == 2 ? mul2(mj, gw) : mul2(mul2(tt, t), mul2(mj, kg));
-        const f2 vx = make_float2(va.x - vi.x, vb.x - vi.x), vy = make_float2(va.y - vi.y, vb.y - vi.y);
-        const f2 vz = DIM == 3 ? make_float2(va.z - vi.z, vb.z - vi.z) : zero2;
+        const f2 vx = others(make_float2(va.x - vi.x, vb.x - vi.x)), vy = others(make_float2(va.y - vi.y, vb.y - vi.y));
+        const f2 vz = DIM == 3 ? others(make_float2(va.z - vi.z, vb.z - vi.z)) : zero2;
         f2 vr = fma2(vy, d1, mul2(vx, d0));
         if (DIM == 3) vr = fma2(vz, d2, vr);
         const f2 rs = make_float2(rpi.x + rhoj.x, rpi.x + rhoj.y);
@@ -2505,9 +2515,7 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             T = mul2(T, irr);
             sv = mul2(sv, irr);
         }
-        T = taking(T);
-        if ((PH & 4) && P.wall_model == 1)  // push only: the other's P is not part of it
-            T = make_float2(mj.x != 0.f ? T.x : 0.f, mj.y != 0.f ? T.y : 0.f);
+        T = others(taking(T));
         const f2 hs2 = UNI ? bc2(4.0f * xi.w * xi.w) : mul2(hs, hs);
         const f2 D = UNI ? add2(dr2, bc2(P.av_eta2 * (xi.w * xi.w)))
                          : fma2(hs2, bc2(0.25f * P.av_eta2), dr2);
@@ -2546,12 +2554,13 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             if (DIM == 3) x2s = dot2(cx, vz, x2s);
         }
         if ((PH & 2) && visc) {
-            const float4 qa = __ldg(B.tau + ka), qb = __ldg(B.tau + kb);
+            const int ia = pa ? s : ka, ib = pb ? s : kb;  // (sv is 0 there)
+            const float4 qa = __ldg(B.tau + ia), qb = __ldg(B.tau + ib);
             const f2 sxx = make_float2(ti.x + qa.x, ti.x + qb.x), syy = make_float2(ti.y + qa.y, ti.y + qb.y);
             const f2 sxy = make_float2(ti.z + qa.z, ti.z + qb.z);
             f2 h0 = fma2(sxy, d1, mul2(sxx, d0)), h1 = fma2(syy, d1, mul2(sxy, d0));
             if (DIM == 3) {
-                const float4 ua = __ldg(B.tau2 + ka), ub = __ldg(B.tau2 + kb);
+                const float4 ua = __ldg(B.tau2 + ia), ub = __ldg(B.tau2 + ib);
                 const f2 szz = make_float2(ti.w + qa.w, ti.w + qb.w);
                 const f2 sxz = make_float2(ti2.x + ua.x, ti2.x + ub.x), syz = make_float2(ti2.y + ua.y, ti2.y + ub.y);
                 h0 = fma2(sxz, d2, h0);
@@ -2572,8 +2581,8 @@ __device__ __forceinline__ void force_body(const StateB& B, const StateA& A,
             }
             const f2 ps = make_float2(rpi.w + qa.w, rpi.w + qb.w);
             const f2 lo = make_float2(ulo_i - __ldg(B.ulo + ka), ulo_i - __ldg(B.ulo + kb));
-            const f2 du2 = add2(make_float2(rpi.z - qa.z, rpi.z - qb.z), lo);
-            const f2 pr = taking(mul2(ps, rh));
+            const f2 du2 = others(add2(make_float2(rpi.z - qa.z, rpi.z - qb.z), lo));
+            const f2 pr = others(taking(mul2(ps, rh)));
             ah_du = dot2(mul2(mul2(mul2(sm, dr2), pr), bc2(2.0f)), du2, ah_du);
         }
     };
