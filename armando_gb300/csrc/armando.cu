@@ -153,7 +153,8 @@ DevParams make_dev_params(const armando_params& p, int reach = 1) {
     d.eta = p.eta;
     d.av_alpha = p.av_alpha;
     d.av_beta = p.av_beta;
-    d.av_eta2 = p.av_eta * p.av_eta;
+    // (the force pass forms art_visc's quotient either way: off, av_eta may be anything)
+    d.av_eta2 = p.visc_artificial ? p.av_eta * p.av_eta : 0.1f * 0.1f;
     d.ah_g1 = p.ah_g1;
     d.ah_g2 = p.ah_g2;
     d.ah_eta2 = p.ah_eta * p.ah_eta;
