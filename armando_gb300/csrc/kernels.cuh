@@ -1848,7 +1848,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
             f2 vd = fma2(make_float2(va.y - vi.y, vb.y - vi.y), d1,
                          mul2(make_float2(va.x - vi.x, vb.x - vi.x), d0));
             if (DIM == 3) vd = fma2(make_float2(va.z - vi.z, vb.z - vi.z), d2, vd);
-            if ((PH & 4) && P.wall_model == 1) vd = make_float2(ina ? vd.x : 0.f, inb ? vd.y : 0.f);
+            if (PH & 4) vd = make_float2(mj.x != 0.f ? vd.x : 0.f, mj.y != 0.f ? vd.y : 0.f);
             divs = dot2(gm, vd, divs);
         }
     };
