@@ -2146,7 +2146,7 @@ __device__ __forceinline__ void density_body(const StateB& B, const unsigned* __
         const float divv = __fdiv_rn(divs, rho);
         rp.w = fmaf(P.ah_g2 * xi.w * xi.w, fabsf(divv) - divv, __fmul_rn(P.ah_g1 * xi.w, P.c0));
     }
-    if (LST && fluid && !(fabsf(rp.y) < 1.0e20f && rho > 1.0e-15f)) {  // the force pass walks its cells
+    if (LST && fluid && !(fabsf(rp.y) < 1.0e34f && rho > 1.0e-18f)) {  // the force pass walks its cells
         B.ncount[s] = -1;
         B.nmask[mask_word_index<W>(0, B.mstride, mlane)] = ~0u;
         if (W > 1) B.nmask[mask_word_index<W>(1, B.mstride, mlane)] = ~0u;
