@@ -201,8 +201,9 @@ armando_status armando_batch_create(armando_ctx** ctx, int32_t n_instances,
                                     const int64_t* n_fluid, const int64_t* n_wall,
                                     int32_t mem_kind);
 
-/* Replaces the context's parameters (same dim). Takes effect at the next call.
- * Batch contexts: ARMANDO_ERR_UNSUPPORTED. */
+/* Replaces the context's parameters (same dim). Takes effect at the next call;
+ * other values end a pending armando_backward (INVALID_ARG there: it needs a new
+ * armando_forward_checkpointed). Batch contexts: ARMANDO_ERR_UNSUPPORTED. */
 armando_status armando_set_params(armando_ctx* ctx, const armando_params* params);
 
 /*
@@ -360,7 +361,8 @@ typedef struct armando_tuning {
 
 armando_status armando_get_tuning(armando_ctx* ctx, armando_tuning* out);
 /* INVALID_ARG for a value outside the lists above; UNSUPPORTED for
- * threads_per_particle > 1 or skin > 0 on a batch context. */
+ * threads_per_particle > 1 or skin > 0 on a batch context; OOM where a CERN-scheme
+ * context's neighbour lists (skin > 0) do not fit (a GPU-C context runs without). */
 armando_status armando_set_tuning(armando_ctx* ctx, const armando_tuning* t);
 
 /* The autotuner's candidate tunings, k = 0 .. ARMANDO_N_TUNINGS - 1: k < 18
